@@ -150,19 +150,28 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* sw, const uint3
 }
 
 // raw query records [n][16] -> encoded bf16 rows [n][128] (the training path;
-// inference encodes inside k_nrc_infer_tc).  The row is built in 64 registers
-// and stored as 16-byte chunks.
+// inference encodes inside k_nrc_infer_tc): a pair of lanes per row, each
+// storing its half of the row in 16-byte chunks.
 __global__ void __launch_bounds__(128) k_nrc_encode(NrcDev C, const float* __restrict__ feat, const int* n_dev, int64_t n_static,
                                                     int offset, int limit, __nv_bfloat16* __restrict__ X) {
     int64_t n = n_dev ? int64_t(*n_dev) : n_static;
     n = n - offset;
     if (limit > 0 && n > limit) n = limit;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        uint32_t w[kNrcIn / 2];
-        encode_row(C, feat + (size_t(offset) + size_t(i)) * kNrcFeatFloats, w);
+    const int lane = threadIdx.x & 31, h = lane & 1;
+    const int64_t warps = int64_t(gridDim.x) * (blockDim.x / 32);
+    for (int64_t w = blockIdx.x * int64_t(blockDim.x / 32) + (threadIdx.x >> 5); w * 16 < n; w += warps) {
+        const int64_t i = w * 16 + (lane >> 1);
+        uint32_t wg[8], wb[16], wt[4];   // a warp stays converged: rows past n repeat the last one
+        encode_pair(C, feat + (size_t(offset) + size_t(i < n ? i : n - 1)) * kNrcFeatFloats, h, wg, wb, wt);
+        if (i >= n) continue;
         uint4* dst = reinterpret_cast<uint4*>(X + size_t(i) * kNrcIn);
 #pragma unroll
-        for (int k = 0; k < kNrcIn / 8; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+        for (int k = 0; k < 2; ++k) dst[2 * h + k] = make_uint4(wg[4 * k], wg[4 * k + 1], wg[4 * k + 2], wg[4 * k + 3]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            dst[4 + 4 * h + k] = make_uint4(wb[4 * k], wb[4 * k + 1], wb[4 * k + 2], wb[4 * k + 3]);
+        dst[12 + h] = h ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(wt[0], wt[1], wt[2], wt[3]);
+        dst[14 + h] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -515,11 +524,7 @@ int nrc_encode(bg_cache* c, const float* feat, const int* n_dev, int64_t n_stati
 }
 
 int nrc_infer(bg_cache* c, const int* n_dev, int64_t n_static, float4* out, cudaStream_t st) {
-    if (c->desc.mlp_kernel == 0)
-        k_nrc_infer_tc<<<c->sms * kTiCtasPerSm, kTiThreads, kTiSmem, st>>>(c->dev, c->X.as<__nv_bfloat16>(), n_dev, n_static, out,
-                                                          c->scene->dev.errflags, nullptr);
-    else
-        k_nrc_infer<<<c->sms * 4, 128, kInferSmem, st>>>(c->dev, c->X.as<__nv_bfloat16>(), n_dev, n_static, out);
+    k_nrc_infer<<<c->sms * 4, 128, kInferSmem, st>>>(c->dev, c->X.as<__nv_bfloat16>(), n_dev, n_static, out);
     BG_CUDA(cudaGetLastError());
     return BG_OK;
 }
@@ -528,8 +533,8 @@ int nrc_infer(bg_cache* c, const int* n_dev, int64_t n_static, float4* out, cuda
 // into the inference kernel; the mma.sync path encodes into X first.
 int nrc_query(bg_cache* c, const float* feat, const int* n_dev, int64_t n_static, float4* out, cudaStream_t st) {
     if (c->desc.mlp_kernel == 0) {
-        k_nrc_infer_tc<<<c->sms * kTiCtasPerSm, kTiThreads, kTiSmem, st>>>(c->dev, nullptr, n_dev, n_static, out, c->scene->dev.errflags,
-                                                          feat);
+        k_nrc_infer_tc<<<c->sms * kTiCtasPerSm, kTiThreads, kTiSmem, st>>>(c->dev, n_dev, n_static, out,
+                                                                           c->scene->dev.errflags, feat);
         BG_CUDA(cudaGetLastError());
         return BG_OK;
     }
@@ -612,11 +617,10 @@ int nrc_graph_node(bg_cache* c, cudaGraphExec_t exec, cudaGraphNode_t node, bool
     NrcDev C = c->dev;
     const __nv_bfloat16* Xc = c->X.as<__nv_bfloat16>();
     if (kp.func == reinterpret_cast<void*>(k_nrc_infer_tc)) {
-        // (NrcDev, X, n_dev, n_static, out, errflags, feat); X is null when the kernel encodes
+        // (NrcDev, n_dev, n_static, out, errflags, feat)
         *is_cache = true;
         if (!exec) return BG_OK;
-        const __nv_bfloat16* X = *static_cast<const __nv_bfloat16* const*>(a[1]) ? Xc : nullptr;
-        void* args[] = {&C, &X, a[2], a[3], a[4], a[5], a[6]};
+        void* args[] = {&C, a[1], a[2], a[3], a[4], a[5]};
         kp.kernelParams = args;
         kp.extra = nullptr;
         BG_CUDA(cudaGraphExecKernelNodeSetParams(exec, node, &kp));

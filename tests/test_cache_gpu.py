@@ -104,6 +104,31 @@ def test_forward_matches_oracle(ctx, mlp_kernel):
     assert err < 2e-2, err
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 127, 128, 129, 38_017])
+def test_query_row_counts_match_oracle(ctx, n):
+    """Rows around a warp's 16 and a tile's 128, and more tiles than the grid has
+    groups; a hashed table and dense levels.  bf16 activations: 2e-2 of the largest
+    output, as for the other forward tests; rows past n stay untouched."""
+    import torch
+    from oracle import nrc_oracle as O
+    gs, cache = _cache(ctx, log2t=10)
+    rng = np.random.default_rng(n)
+    mlp0, grid0, _, _ = cache.params()
+    cache.set_params(mlp0, (rng.random(grid0.shape).astype(np.float32) - 0.5) * 0.5)
+    feat = _features(n, rng)
+    out = torch.full((n + 3, 4), 7.0, dtype=torch.float32, device="cuda")
+    fd = torch.from_numpy(feat).cuda()
+    cache.query(fd.data_ptr(), out.data_ptr(), n)
+    torch.cuda.synchronize()
+    mlp, g, _, _ = cache.params()
+    res, log2t, bmin, bscale = _oracle_args(cache)
+    X, _ = O.encode(feat.astype(np.float64), g, res, log2t, bmin, bscale)
+    ref, _, _ = O.forward(X, mlp)
+    got = out.cpu().numpy()
+    assert np.abs(got[:n, :3] - ref[:, :3]).max() < 2e-2 * np.abs(ref[:, :3]).max()
+    assert (got[:n, 3] == 0).all() and (got[n:] == 7).all()
+
+
 @pytest.mark.parametrize("mlp_kernel", [0, 1], ids=["tcgen05", "mma_sync"])
 def test_adam_training_reduces_loss(ctx, mlp_kernel):
     import torch
