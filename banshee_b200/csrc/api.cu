@@ -279,8 +279,8 @@ static void launch_layout(bg_scene* s, bool any_hit, const float4* rays, int64_t
 int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                  bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
                  unsigned long long* work, const int* roots, const ShadowResolve* resolve) {
-    unsigned long long* w = work ? work : next_work_counter(s);
-    BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
+    unsigned long long* w = work ? work : next_work_counter(s);   // the caller's is cleared
+    if (!work) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
     ShadowResolve res{nullptr, nullptr, nullptr, 0};
     if (resolve && !counters) {
         if (any_hit) res = *resolve;
@@ -859,6 +859,7 @@ static int host_cast(bg_scene* s, const bg_ray* rays, void* out, int64_t n, bool
     char* hp = static_cast<char*>(c->pinned);
     char* dp = c->dev.as<char>();
     memcpy(hp, rays, rb);
+    BG_CUDA(cudaMemsetAsync(dp, 0, sizeof(unsigned long long), c->st));
     BG_CUDA(cudaMemcpyAsync(dp + 256, hp, rb, cudaMemcpyHostToDevice, c->st));
     rc = launch_trace(s, any, reinterpret_cast<const float4*>(dp + 256), n, nullptr,
                       any ? nullptr : reinterpret_cast<bg_hit*>(dp + 256 + rb), any ? reinterpret_cast<uint8_t*>(dp + 256 + rb) : nullptr,

@@ -186,6 +186,7 @@ struct ShadowResolve {
     float4* slots;
     int hit_class;
 };
+// work: the launch's work counter, cleared by the caller (null: one of the scene's).
 int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                  bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters = nullptr,
                  int stride = 1, unsigned long long* work = nullptr, const int* roots = nullptr,

@@ -50,7 +50,17 @@ __global__ void k_clamp_count(int* n, int cap) {
 }
 
 constexpr int kShadeThreads = 128;
-constexpr int kMaxBounceCounters = 6 * 1024;   // 6 work counters per bounce, maxdepth <= 1024
+// Counters of one bounce: queue lengths, material-class list lengths and the
+// work counters of its traces (extension, shadow, MIS, and the three counting
+// replays).  A pass has one record per bounce (and one past the last, whose
+// extension queue stays empty), all cleared by one memset at its start.
+struct BounceRec {
+    int n_ext, n_sh, n_mis, n_end, n_query, n_cls[3];
+    unsigned long long work[6];
+    int pad[12];
+};
+static_assert(sizeof(BounceRec) == 128, "bounce counters are 128 bytes");
+constexpr int kMaxBounces = 1024;              // maxdepth <= 1024
 constexpr int kGraphKey = 15;                    // int64 fields identifying a captured pass
 
 
@@ -76,11 +86,11 @@ struct RenderState {
     DevBuf mis_rays, mis_a, mis_b, mis_c, mis_hits;
     DevBuf end_path;
     DevBuf cls;        // material-class lists of the extension queue: 3 x cap queue indices
-    DevBuf counts;     // int: ext[0], ext[1], sh, mis, end ; u64 totals at +64 bytes
+    DevBuf counts;     // int: training-row counts of the two sets ; u64 totals at +64 bytes
     DevBuf st_key, st_cnt, st_rng, st_bs, st_thr, st_rad, st_dithr, st_flags;
     DevBuf slots, sample_rad;
     DevBuf cnt_out;    // outputs of the instrumented 1/64 replays
-    DevBuf work;       // persistent-kernel work counters of the pass (6 per bounce)
+    DevBuf bounce;     // BounceRec[kMaxBounces + 1]: counters of the pass in flight
     // radiance-cache mode: cache queries, training-path vertex records, training samples
     DevBuf q_feat, q_path, q_thr, q_out, rec, tr_feat, tr_target;
     int64_t q_cap = 0, tr_cap = 0;       // tr_cap: rows per training set
@@ -151,23 +161,18 @@ void render_state_free(RenderState* rs) {
                       &rs->sh_rays, &rs->sh_contrib, &rs->sh_slot, &rs->mis_rays, &rs->mis_a, &rs->mis_b,
                       &rs->mis_c, &rs->mis_hits, &rs->end_path, &rs->counts, &rs->st_key, &rs->st_cnt, &rs->st_rng,
                       &rs->st_bs, &rs->st_thr, &rs->st_rad, &rs->st_dithr, &rs->st_flags, &rs->slots,
-                      &rs->sample_rad, &rs->cnt_out, &rs->work, &rs->q_feat, &rs->q_path, &rs->q_thr,
+                      &rs->sample_rad, &rs->cnt_out, &rs->bounce, &rs->q_feat, &rs->q_path, &rs->q_thr,
                       &rs->q_out, &rs->rec, &rs->tr_feat, &rs->tr_target, &rs->segs, &rs->jobs,
                       &rs->ext_root[0], &rs->ext_root[1], &rs->sh_root, &rs->mis_root, &rs->cls})
         b->release();
     delete rs;
 }
 
-enum : int { kCntExt0 = 0, kCntExt1 = 1, kCntSh = 2, kCntMis = 3, kCntEnd = 4, kCntQuery = 5, kCntTrain = 6 };
-constexpr int kCntCls = 12;   // three material-class counters (k_classify)
-// extension traces write the material class of each hit into its primid
-static const ShadowResolve kExtTrace{nullptr, nullptr, nullptr, 1};
-// shadow / MIS / ended-path counters of the odd bounces when direct light is
-// resolved one bounce late (the even bounces use kCntSh..kCntEnd)
-constexpr int kCntSh1 = 8;
 // training rows alternate between two halves of tr_feat / tr_target (counters
 // kCntTrain + set): a frame writes one while the previous frame's are trained on
-constexpr int kCntTrainSets = 2;
+constexpr int kCntTrain = 0, kCntTrainSets = 2;
+// extension traces write the material class of each hit into its primid
+static const ShadowResolve kExtTrace{nullptr, nullptr, nullptr, 1};
 enum : unsigned { kFlagNoClamp = 1u, kFlagTrain = 2u };   // bits 8..15: recorded vertices of a training path
 
 struct PathState {
@@ -581,9 +586,11 @@ __device__ __forceinline__ void shade_path(const DevScene& S, const ShadeArgs& A
     }
 }
 
-// Every hit of the extension queue, material read per hit.
+// Every hit of the extension queue, material read per hit.  AoTracer: 8 blocks per
+// SM (64 registers; measured: 8 > 7 > 10 > 6).  Small passes of the others: a few
+// blocks at most run, so registers instead of spills.
 template <int KIND, bool CACHE, bool AREA>
-__global__ void __launch_bounds__(kShadeThreads, 8)   // 64 registers (measured: 8 > 7 > 10 > 6 blocks / SM)
+__global__ void __launch_bounds__(kShadeThreads, KIND == BG_TRACER_AO ? 8 : 4)
 k_shade(DevScene S, ShadeArgs A, PathState P, Queues Q) {
     const int n = *Q.n_ext_in;
     if (blockIdx.x == 0 && threadIdx.x == 0) Q.totals[0] += (unsigned long long)n;
@@ -673,7 +680,6 @@ k_shade_class(DevScene S, ShadeArgs A, PathState P, Queues Q) {
 template <int KIND, bool CACHE, bool AREA>
 static int launch_shade_split(const DevScene& d, int nb, int nbc, cudaStream_t st, const ShadeArgs& A,
                               const PathState& P, const Queues& Q) {
-    BG_CUDA(cudaMemsetAsync(Q.n_cls, 0, 3 * sizeof(int), st));
     k_classify<<<nb, kClassifyThreads, 0, st>>>(Q, A.cap);
     k_shade_class<KIND, CACHE, AREA, kMatOther><<<nbc, kShadeThreads, 0, st>>>(d, A, P, Q);
     k_shade_class<KIND, CACHE, AREA, BG_MAT_LAMBERT><<<nbc, kShadeThreads, 0, st>>>(d, A, P, Q);
@@ -681,9 +687,23 @@ static int launch_shade_split(const DevScene& d, int nb, int nbc, cudaStream_t s
     return BG_OK;
 }
 
+// Passes of at most this many paths are shaded by one kernel: each of the four
+// launches of the class split takes 2-3 us however little it has to do.
+constexpr int64_t kOneShadePaths = 32768;
+
 // The shading kernels for a tracer kind, cache mode and the scene's lights.
 // Returns the number of kernels launched (< 0: an error code).  AoTracer has no
 // BSDF: its paths are shaded by one kernel.
+template <int KIND, bool CACHE, bool AREA>
+static int launch_shade_kind(const DevScene& d, int nb, int nbc, cudaStream_t st, const ShadeArgs& A, const PathState& P,
+                             const Queues& Q) {
+    if (A.cap <= kOneShadePaths) {
+        k_shade<KIND, CACHE, AREA><<<nb, kShadeThreads, 0, st>>>(d, A, P, Q);
+        return 1;
+    }
+    const int rc = launch_shade_split<KIND, CACHE, AREA>(d, nb, nbc, st, A, P, Q);
+    return rc ? rc : 4;
+}
 static int launch_shade(const DevScene& d, int kind, bool cache, int nb, int nbc, cudaStream_t st,
                         const ShadeArgs& A, const PathState& P, const Queues& Q) {
     const bool area = d.has_area != 0;
@@ -691,17 +711,14 @@ static int launch_shade(const DevScene& d, int kind, bool cache, int nb, int nbc
         k_shade<BG_TRACER_AO, false, false><<<nb, kShadeThreads, 0, st>>>(d, A, P, Q);
         return 1;
     }
-    int rc;
     if (kind == BG_TRACER_DI)
-        rc = area ? launch_shade_split<BG_TRACER_DI, false, true>(d, nb, nbc, st, A, P, Q)
-                  : launch_shade_split<BG_TRACER_DI, false, false>(d, nb, nbc, st, A, P, Q);
-    else if (cache)
-        rc = area ? launch_shade_split<BG_TRACER_GI, true, true>(d, nb, nbc, st, A, P, Q)
-                  : launch_shade_split<BG_TRACER_GI, true, false>(d, nb, nbc, st, A, P, Q);
-    else
-        rc = area ? launch_shade_split<BG_TRACER_GI, false, true>(d, nb, nbc, st, A, P, Q)
-                  : launch_shade_split<BG_TRACER_GI, false, false>(d, nb, nbc, st, A, P, Q);
-    return rc ? rc : 4;
+        return area ? launch_shade_kind<BG_TRACER_DI, false, true>(d, nb, nbc, st, A, P, Q)
+                    : launch_shade_kind<BG_TRACER_DI, false, false>(d, nb, nbc, st, A, P, Q);
+    if (cache)
+        return area ? launch_shade_kind<BG_TRACER_GI, true, true>(d, nb, nbc, st, A, P, Q)
+                    : launch_shade_kind<BG_TRACER_GI, true, false>(d, nb, nbc, st, A, P, Q);
+    return area ? launch_shade_kind<BG_TRACER_GI, false, true>(d, nb, nbc, st, A, P, Q)
+                : launch_shade_kind<BG_TRACER_GI, false, false>(d, nb, nbc, st, A, P, Q);
 }
 
 // BSDF-sampled rays towards area lights: the closest hit must be on a bundle
@@ -877,7 +894,7 @@ static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L) {
         (rc = rs->st_dithr.ensure(2 * C * 16)) || (rc = rs->st_flags.ensure(C * 4)) ||
         (rc = rs->slots.ensure(2 * C * rs->kmax * 16)) || (rc = rs->sample_rad.ensure(C * 16)) ||
         (rc = rs->cnt_out.ensure((C * 2 * L / 64 + 64) * 16)) ||
-        (rc = rs->work.ensure(size_t(kMaxBounceCounters) * 8)))
+        (rc = rs->bounce.ensure(size_t(kMaxBounces + 1) * sizeof(BounceRec))))
         return rc;
     int nb = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade<BG_TRACER_AO, false, false>, kShadeThreads, 0);
@@ -944,10 +961,12 @@ struct PassCfg {
     float ao_radius;
 };
 
-// Queue pointers of a bounce: extension queue `c` in, 1 - c out; shadow, MIS
-// and ended-path queues and their counters of parity `par`.
-static void pass_queues(RenderState* rs, int c, bool batched, Queues& Q, int par = 0) {
+// Queue pointers and counters of bounce b: extension queue b & 1 in, the other
+// out; shadow, MIS and ended-path queues of parity `par`.
+static void pass_queues(RenderState* rs, int b, bool batched, Queues& Q, int par = 0) {
     int* cnt = rs->counts.as<int>();
+    BounceRec* rec = rs->bounce.as<BounceRec>() + b;
+    const int c = b & 1;
     const size_t C = size_t(rs->cap), L = size_t(rs->nlights);
     const size_t sh = par ? C * 2 * L : 0, mi = par ? C * L : 0;   // entries before this parity's half
     Q.ext_hits = rs->ext_hits.as<bg_hit>();
@@ -957,15 +976,14 @@ static void pass_queues(RenderState* rs, int c, bool batched, Queues& Q, int par
     Q.mis_b = rs->mis_b.as<float4>() + mi;
     Q.mis_c = rs->mis_c.as<int4>() + mi; Q.mis_hits = rs->mis_hits.as<bg_hit>() + mi;
     Q.end_path = rs->end_path.as<int>() + (par ? C : 0);
-    const int c0 = par ? kCntSh1 : kCntSh;
-    Q.n_sh = cnt + c0; Q.n_mis = cnt + c0 + 1; Q.n_end = cnt + c0 + 2;
+    Q.n_sh = &rec->n_sh; Q.n_mis = &rec->n_mis; Q.n_end = &rec->n_end;
     Q.totals = reinterpret_cast<unsigned long long*>(rs->counts.as<char>() + 64);
     Q.ext_rays_in = rs->ext_rays[c].as<float4>(); Q.ext_path_in = rs->ext_path[c].as<int>();
     Q.ext_rays_out = rs->ext_rays[1 - c].as<float4>(); Q.ext_path_out = rs->ext_path[1 - c].as<int>();
-    Q.n_ext_in = cnt + (c ? kCntExt1 : kCntExt0);
-    Q.n_ext_out = cnt + (c ? kCntExt0 : kCntExt1);
+    Q.n_ext_in = &rec->n_ext;
+    Q.n_ext_out = &rec[1].n_ext;
     Q.q_feat = rs->q_feat.as<float4>(); Q.q_path = rs->q_path.as<int>(); Q.q_thr = rs->q_thr.as<float4>();
-    Q.n_query = cnt + kCntQuery;
+    Q.n_query = &rec->n_query;
     Q.tr_feat = rs->tr_feat.as<float4>() + size_t(rs->tr_set) * rs->tr_cap * 4;
     Q.tr_target = rs->tr_target.as<float4>() + size_t(rs->tr_set) * rs->tr_cap;
     Q.n_train = cnt + kCntTrain + rs->tr_set;
@@ -975,7 +993,7 @@ static void pass_queues(RenderState* rs, int c, bool batched, Queues& Q, int par
     Q.sh_root = batched ? rs->sh_root.as<int>() + sh : nullptr;
     Q.mis_root = batched ? rs->mis_root.as<int>() + mi : nullptr;
     Q.jobs = rs->jobs.as<JobRec>();
-    Q.n_cls = cnt + kCntCls;
+    Q.n_cls = rec->n_cls;
     Q.cls = rs->cls.as<int>();
 }
 
@@ -1001,10 +1019,10 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
     const int nb = rs->blocks;
     PathState P = path_state(rs);
     Queues Q;
-    int cur = 0;
-    pass_queues(rs, cur, c.batched, Q);
-    int* cnt = rs->counts.as<int>();
+    pass_queues(rs, 0, c.batched, Q);
     int rc;
+    const int depth = std::max(1, c.maxdepth);
+    BG_CUDA(cudaMemsetAsync(rs->bounce.ptr, 0, size_t(depth + 1) * sizeof(BounceRec), st));
     k_generate<<<nb, kShadeThreads, 0, st>>>(c.segs, c.nseg, c.total, P, Q, c.cache ? c.train_stride : 0, c.train_phase);
     if (ins) ++ins->launches;
     bg_hit* cnt_hits = rs->cnt_out.as<bg_hit>();
@@ -1018,7 +1036,6 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
     // running two chains side by side shortens the pass.
     const bool fork = (ins == nullptr || (!ins->time_phases && !ins->count_trav)) && rs->fstream != nullptr &&
                       rs->mstream != nullptr;
-    const int depth = std::max(1, c.maxdepth);
     if (fork && !c.cache) {
         // Direct light resolved one bounce late.  Shade(b) gathers the DI of
         // bounce b - 2 and writes its own into the slot half of parity b, so the
@@ -1031,11 +1048,9 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
         cudaEvent_t evd[2] = {rs->ev_join, rs->ev_mjoin};
         for (int b = 0; b < depth; ++b) {
             const int par = b & 1;
-            unsigned long long* wk = rs->work.as<unsigned long long>() + 6 * b;
-            pass_queues(rs, cur, c.batched, Q, par);
+            unsigned long long* wk = rs->bounce.as<BounceRec>()[b].work;
+            pass_queues(rs, b, c.batched, Q, par);
             if (b >= 2) BG_CUDA(cudaStreamWaitEvent(st, evd[par], 0));   // bounce b - 2's side work is done
-            BG_CUDA(cudaMemsetAsync(Q.n_ext_out, 0, sizeof(int), st));
-            BG_CUDA(cudaMemsetAsync(cnt + (par ? kCntSh1 : kCntSh), 0, 3 * sizeof(int), st));
             if (b == 0) {
                 if ((rc = launch_trace(s, false, Q.ext_rays_in, 0, Q.n_ext_in, Q.ext_hits, nullptr, st, nullptr, 1, wk,
                                        Q.ext_root_in, &kExtTrace)))
@@ -1063,11 +1078,10 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
             BG_CUDA(cudaEventRecord(evd[par], ds));
             if (ins) ins->launches += 3;
             if (b + 1 < depth) {
-                cur = 1 - cur;
                 Queues Qn;
-                pass_queues(rs, cur, c.batched, Qn, par ^ 1);
+                pass_queues(rs, b + 1, c.batched, Qn, par ^ 1);
                 if ((rc = launch_trace(s, false, Qn.ext_rays_in, 0, Qn.n_ext_in, Qn.ext_hits, nullptr, st, nullptr, 1,
-                                       wk + 6, Qn.ext_root_in, &kExtTrace)))
+                                       rs->bounce.as<BounceRec>()[b + 1].work, Qn.ext_root_in, &kExtTrace)))
                     return rc;
                 if (ins) { ++ins->launches; ++ins->launches_extend; }
             }
@@ -1075,9 +1089,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
         BG_CUDA(cudaStreamWaitEvent(st, evd[(depth - 1) & 1], 0));   // the side stream is in bounce order
     }
     for (int b = 0; b < depth && !(fork && !c.cache); ++b) {
-        unsigned long long* wk = rs->work.as<unsigned long long>() + 6 * b;
-        BG_CUDA(cudaMemsetAsync(Q.n_ext_out, 0, sizeof(int), st));
-        BG_CUDA(cudaMemsetAsync(cnt + kCntSh, 0, 3 * sizeof(int), st));
+        unsigned long long* wk = rs->bounce.as<BounceRec>()[b].work;
         if (!fork || b == 0) {
             if (ins) ins->mark(0);
             if ((rc = launch_trace(s, false, Q.ext_rays_in, 0, Q.n_ext_in, Q.ext_hits, nullptr, st, nullptr, 1, wk, Q.ext_root_in, &kExtTrace))) return rc;
@@ -1090,7 +1102,6 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
         ShadeArgs A{b, c.maxdepth, c.kind, rs->kmax, c.batched ? 1 : 0, c.cache ? c.cache_depth : -1,
                     c.cache ? c.train_end : -1, c.cache ? c.train_stride : 0, c.ao_radius, 0, int(rs->cap)};
         const bool query_here = c.cache && (b == c.cache_depth || b == c.train_end);
-        if (query_here) BG_CUDA(cudaMemsetAsync(Q.n_query, 0, sizeof(int), st));
         // the network the queries read is the one the previous frame's rows trained
         // (with side streams the wait sits on the query's own stream, below)
         const bool wait_here = c.cache && (c.wait_train || !ins) && b == c.cache_depth;
@@ -1102,11 +1113,11 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
         const bool forked = fork && b + 1 < depth;
         if (forked) {
             Queues Qn;
-            pass_queues(rs, 1 - cur, c.batched, Qn);
+            pass_queues(rs, b + 1, c.batched, Qn);
             BG_CUDA(cudaEventRecord(rs->ev_fork, st));
             BG_CUDA(cudaStreamWaitEvent(rs->fstream, rs->ev_fork, 0));
             if ((rc = launch_trace(s, false, Qn.ext_rays_in, 0, Qn.n_ext_in, Qn.ext_hits, nullptr, rs->fstream, nullptr, 1,
-                                   wk + 6, Qn.ext_root_in, &kExtTrace)))
+                                   rs->bounce.as<BounceRec>()[b + 1].work, Qn.ext_root_in, &kExtTrace)))
                 return rc;
             BG_CUDA(cudaEventRecord(rs->ev_join, rs->fstream));
             if (ins) { ++ins->launches; ++ins->launches_extend; }
@@ -1157,8 +1168,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
                                                  c.cache ? c.cache_depth : 0, b, 0, int(rs->cap));
         if (ins) ins->launches += s->dev.has_area ? 2 : 1;
         if (forked) BG_CUDA(cudaStreamWaitEvent(st, rs->ev_join, 0));
-        cur = 1 - cur;
-        pass_queues(rs, cur, c.batched, Q);
+        if (b + 1 < depth) pass_queues(rs, b + 1, c.batched, Q);
     }
     // the accumulation buffer may still be arriving from the host (bg_render_host)
     // (captured into the pass graph as an event-wait node; a plain wait otherwise)
