@@ -115,72 +115,87 @@ void ScratchBuf::release() {
     bytes = 0;
 }
 
+// Result of ray i: prim with its material class in bits 28-29, -1 = none (t = tmax).
+// Any hit with res.slots: a visible ray stores its contribution in its slot.
+template <bool ANY>
+__device__ __forceinline__ void trace_emit(const ShadowResolve& res, bg_hit* hits, uint8_t* occ, int i, int prim, float t,
+                                           float u, float v) {
+    if (ANY) {
+        if (!res.slots) occ[i] = prim >= 0 ? 1 : 0;
+        else if (prim < 0) res.slots[__ldg(res.slot_of + i)] = __ldg(res.contrib + i);
+    } else {
+        const int id = (prim >= 0 && !res.hit_class) ? prim & kPrimMask : prim;
+        reinterpret_cast<float4*>(hits)[i] = make_float4(t, __int_as_float(id), u, v);
+    }
+}
+
 // ------------------------------------------------------------ trace kernel
 // Persistent threads with per-lane dynamic fetch: lanes whose ray finished
 // take new ray indices from one global counter with a single warp-aggregated
-// atomicAdd, every kRefillStepsClosest / kRefillStepsAny traversal steps.
+// atomicAdd, every refill_steps() traversal steps.
 // Termination: the counter is monotone and every ray finishes after at most
 // one visit per node.
-template <bool ANY, bool COUNT, int THREADS = kTraceThreads, int WIDTH = 4, bool WT = false>
+template <bool ANY, bool COUNT, int THREADS, int WIDTH, bool WT, int WALK>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
-k_trace(DevScene S, const float4* __restrict__ rays, int64_t n_static, const int* __restrict__ n_dev,
+k_trace(DevScene scene, const float4* __restrict__ rays, int64_t n_static, const int* __restrict__ n_dev,
         bg_hit* __restrict__ hits, uint8_t* __restrict__ occ, unsigned long long* __restrict__ work,
         unsigned long long* __restrict__ counters, int stride, const int* __restrict__ roots, ShadowResolve res) {
     // roots (optional): per-ray root node, for rays of several scenes merged into one
     // res.slots (any hit, optional): visible rays store their contribution in their slot
     // COUNT: instrumented replay of rays 0, stride, 2*stride, ... (outputs compacted)
-    const int64_t n_all = n_dev ? int64_t(*n_dev) : n_static;
-    const int64_t n = COUNT ? (n_all + stride - 1) / stride : n_all;
+    TraceScene S;
+    static_cast<DevScene&>(S) = scene;
+    S.rays = rays;
+    constexpr bool kOwn = WALK == kWalkPacked || WALK == kWalkFused;
+    __shared__ float4 own[kOwn ? 2 : 1][kOwn ? THREADS : 1];
+    S.own = &own[0][kOwn ? threadIdx.x : 0];
+    S.ownstep = THREADS;
+    const int n_all = n_dev ? *n_dev : int(n_static);   // (at most 2^30: launch_trace)
+    const int n = COUNT ? (n_all + stride - 1) / stride : n_all;
     const unsigned lane = threadIdx.x & 31u;
-    constexpr int kSm = smem_stack_entries<WIDTH>();
+    constexpr int kSm = smem_stack_entries<WIDTH, WALK>();
     int2 lstack[stack_entries<WIDTH>() - kSm];
     __shared__ int2 sstack[kSm > 0 ? kSm : 1][THREADS];
     const RayStack<kSm> stack{&sstack[0][threadIdx.x], lstack, THREADS};
-    TravState<WT> s;
+    TravState<WT, WALK> s;
     Counters cnt{0ull, 0ull, 0ull};
-    int64_t ridx = -1;
-    bool active = false, exhausted = false;
+    bool active = false, again = false;   // again: the lane's ray is walked again on the plain nodes
+    bool exhausted = false;
     for (;;) {
-        if (!exhausted) {
-            unsigned need = __ballot_sync(0xffffffffu, !active);
-            if (need) {
-                int c = __popc(need);
-                int leader = __ffs(need) - 1;
-                unsigned long long base = 0;
-                if (lane == unsigned(leader)) base = atomicAdd(work, (unsigned long long)c);
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (base + c >= (unsigned long long)n) exhausted = true;
-                if (!active) {
-                    int64_t my = int64_t(base) + __popc(need & ((1u << lane) - 1u));
-                    if (my < n) {
-                        ridx = my;
-                        const int64_t src = COUNT ? my * stride : my;
-                        float4 a = __ldg(rays + 2 * src), b = __ldg(rays + 2 * src + 1);
-                        trav_init(s, a, b);
-                        if (roots) s.item = __ldg(roots + src);
-                        if (COUNT) ++cnt.rays;
-                        active = true;
-                    }
-                }
-            }
+        const unsigned need = __ballot_sync(0xffffffffu, !active && !again);
+        int my = n;
+        if (need && !exhausted) {
+            const int c = __popc(need), leader = __ffs(need) - 1;
+            int first = 0;
+            if (lane == unsigned(leader)) first = int(min(atomicAdd(work, (unsigned long long)c), (unsigned long long)n));
+            first = __shfl_sync(0xffffffffu, first, leader);
+            exhausted = first + c >= n;
+            my = first + __popc(need & ((1u << lane) - 1u));
         }
-        if (!__any_sync(0xffffffffu, active)) break;
-        if (active) {
-            if (trav_steps<ANY, COUNT, WIDTH>(S, s, stack, ANY ? kRefillStepsAny : kRefillStepsClosest, cnt)) {
-                if (ANY) {
-                    if (!res.slots) occ[ridx] = s.prim >= 0 ? 1 : 0;
-                    else if (s.prim < 0) res.slots[__ldg(res.slot_of + ridx)] = __ldg(res.contrib + ridx);
-                } else {
-                    bg_hit h;
-                    h.t = s.prim >= 0 ? s.best : s.r.tmax;
-                    h.primid = s.prim;
-                    h.u = s.u;
-                    h.v = s.v;
-                    if (res.hit_class && s.prim >= 0) h.primid = s.prim | (s.cls << kClassShift);
-                    reinterpret_cast<float4*>(hits)[ridx] = *reinterpret_cast<float4*>(&h);
-                }
-                active = false;
-            }
+        // (Measured and rejected: rays reserved 32 at a time per warp and prefetched, one
+        // atomic per 32: the reserve unbalances the end of every launch, C3 36.0 -> 38.4 ms.)
+        if (again || (!active && my < n)) {
+            const int src = again ? s.r.idx : COUNT ? my * stride : my;
+            trav_init(s, S, again ? kPlainWalk : 0u, __ldg(rays + 2 * int64_t(src)), __ldg(rays + 2 * int64_t(src) + 1), src,
+                      roots ? __ldg(roots + src) : 0);
+            if (COUNT) ++cnt.rays;
+            active = true;
+            again = false;
+        }
+        const unsigned live = __ballot_sync(0xffffffffu, active);
+        if (!live) break;
+        // rays of one octant (a camera's, mostly) share nodes: their warp is bound by
+        // issue slots, not by the L1's data pipe, and reads the 128-byte nodes
+        bool fused = false;
+        if constexpr (WALK == kWalkPacked && WIDTH == 4) {
+            const uint32_t oct = s.r.flags & kOctMask;
+            const uint32_t lead = __shfl_sync(0xffffffffu, oct, __ffs(live) - 1);
+            fused = __all_sync(0xffffffffu, !active || oct == lead);
+        }
+        if (active && trav_steps<ANY, COUNT, WIDTH>(S, s, stack, refill_steps<ANY, WALK>(), fused, cnt)) {
+            active = false;
+            if (WALK != kWalkPlain && (s.r.flags & kNearTie)) again = true;   // the plain walk decides
+            else trace_emit<ANY>(res, hits, occ, COUNT ? s.r.idx / stride : s.r.idx, s.prim, s.best, s.u, s.v);   // (best = tmax on a miss)
         }
     }
     if (COUNT) {
@@ -197,34 +212,62 @@ k_trace(DevScene S, const float4* __restrict__ rays, int64_t n_static, const int
     }
 }
 
-template <bool ANY, bool COUNT, int THREADS, int WIDTH, bool WT>
+// The walk of a large launch.
+//   casts       packed: L1-bound incoherent rays gain most (coherent / incoherent
+//               closest, incoherent any in Mrays/s, plain before -> packed: soups of
+//               1,000 triangles 17751 / 5971 / 8134 -> 17453 / 7210 / 9789, 16,000
+//               6048 / 2050 / 2844 -> 6224 / 3149 / 4292, 64,000 3188 / 1267 / 1720 ->
+//               3643 / 1998 / 2715, 1M 1784 / 1041 / 1282 -> 1961 / 1442 / 1895).  A
+//               smaller scene's nodes lie in the L1, which then is no bound (100
+//               triangles, any hits: plain 18034, packed 16483).
+//   renders     fused: their rays are issue-bound (16 K to 800 K triangles: 1.83,
+//               2.14, 2.48, 2.75 ms -> 1.70, 2.02, 2.25, 2.65; packed bytes alone 5 %
+//               slower than plain).
+//   8-wide      packed: half the instructions of its decode (1000 -> 1090 incoherent
+//               closest, 1360 -> 1448 any, 2447 -> 2904 coherent any).
+constexpr int64_t kPackTriangles = 1000;
+template <int WIDTH>
+static int choose_walk(const DevScene& d, bool render) {
+    if (!packed_walk<WIDTH>(d)) return kWalkPlain;
+    if (WIDTH == 8) return kWalkPacked;
+    if (render) return kWalkFused;
+    return d.ntris < kPackTriangles ? kWalkPlain : kWalkPacked;
+}
+
+template <bool ANY, bool COUNT, int THREADS, int WIDTH, bool WT, int WALK>
 static int trace_blocks(bg_scene* s) {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace<ANY, COUNT, THREADS, WIDTH, WT>, THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace<ANY, COUNT, THREADS, WIDTH, WT, WALK>, THREADS, 0);
     if (nb < 1) nb = 1;
     return nb * s->ctx->num_sms;
 }
 
 // Grid sizes of every traversal variant of the scene's intersection test:
-// [width 4/8][any][count][128/256 threads].
-template <int WIDTH, bool WT>
-static void setup_width(bg_scene* s, int w) {
-    s->trace_blocks[w][0][0][0] = trace_blocks<false, false, 128, WIDTH, WT>(s);
-    s->trace_blocks[w][1][0][0] = trace_blocks<true, false, 128, WIDTH, WT>(s);
-    s->trace_blocks[w][0][1][0] = trace_blocks<false, true, 128, WIDTH, WT>(s);
-    s->trace_blocks[w][1][1][0] = trace_blocks<true, true, 128, WIDTH, WT>(s);
-    s->trace_blocks[w][0][0][1] = trace_blocks<false, false, 256, WIDTH, WT>(s);
-    s->trace_blocks[w][1][0][1] = trace_blocks<true, false, 256, WIDTH, WT>(s);
+// [walk][width 4/8][any][count][128/256 threads].
+template <int WIDTH, bool WT, int WALK>
+static void setup_width(bg_scene* s) {
+    auto& b = s->trace_blocks[WALK][WIDTH == 8];
+    b[0][0][0] = trace_blocks<false, false, 128, WIDTH, WT, WALK>(s);
+    b[1][0][0] = trace_blocks<true, false, 128, WIDTH, WT, WALK>(s);
+    b[0][0][1] = trace_blocks<false, false, 256, WIDTH, WT, WALK>(s);
+    b[1][0][1] = trace_blocks<true, false, 256, WIDTH, WT, WALK>(s);
+    if (WALK == kWalkPlain) {
+        b[0][1][0] = trace_blocks<false, true, 128, WIDTH, WT, kWalkPlain>(s);
+        b[1][1][0] = trace_blocks<true, true, 128, WIDTH, WT, kWalkPlain>(s);
+    }
+}
+template <bool WT>
+static void setup_walks(bg_scene* s) {
+    setup_width<4, WT, kWalkPlain>(s);
+    setup_width<4, WT, kWalkPacked>(s);
+    setup_width<4, WT, kWalkFused>(s);
+    setup_width<8, WT, kWalkPlain>(s);
+    setup_width<8, WT, kWalkPacked>(s);
 }
 
 void scene_launch_setup(bg_scene* s) {
-    if (s->dev.watertight) {
-        setup_width<4, true>(s, 0);
-        setup_width<8, true>(s, 1);
-    } else {
-        setup_width<4, false>(s, 0);
-        setup_width<8, false>(s, 1);
-    }
+    if (s->dev.watertight) setup_walks<true>(s);
+    else setup_walks<false>(s);
 }
 
 unsigned long long* next_work_counter(bg_scene* s) {
@@ -232,61 +275,77 @@ unsigned long long* next_work_counter(bg_scene* s) {
     return s->work.as<unsigned long long>() + slot;
 }
 
-template <int WIDTH, bool WT>
-static void launch_width(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
-                         bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
-                         unsigned long long* w, const int* roots,
-                         ShadowResolve res = ShadowResolve{nullptr, nullptr, nullptr, 0}) {
-    const int wi = WIDTH == 8 ? 1 : 0;
-    const DevScene& d = s->dev;
-    // a static count smaller than the persistent grid (a few rays of a *_host
-    // call) gets only the blocks it can use
-    auto grid = [&](int blocks, int threads) {
-        if (n_dev || n_static <= 0) return blocks;
-        const int64_t rays_n = counters ? (n_static + stride - 1) / stride : n_static;
-        return int(std::max<int64_t>(1, std::min<int64_t>(blocks, (rays_n + threads - 1) / threads)));
+template <int WIDTH, bool WT, int WALK>
+static void launch_walk(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev, bg_hit* hits,
+                        uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride, unsigned long long* w,
+                        const int* roots, const ShadowResolve& res) {
+    const auto& b = s->trace_blocks[WALK][WIDTH == 8];
+    auto go = [&](auto kernel, int blocks, int threads) {
+        // a static count smaller than the persistent grid (a few rays of a *_host
+        // call) gets only the blocks it can use
+        if (!n_dev && n_static > 0) {
+            const int64_t rays_n = counters ? (n_static + stride - 1) / stride : n_static;
+            blocks = int(std::max<int64_t>(1, std::min<int64_t>(blocks, (rays_n + threads - 1) / threads)));
+        }
+        kernel<<<blocks, threads, 0, st>>>(s->dev, rays, n_static, n_dev, hits, occ, w, counters, counters ? stride : 1, roots, res);
     };
     if (counters) {
-        if (any_hit)
-            k_trace<true, true, 128, WIDTH, WT><<<grid(s->trace_blocks[wi][1][1][0], 128), 128, 0, st>>>(d, rays, n_static, n_dev, hits, occ, w, counters, stride, roots, res);
-        else
-            k_trace<false, true, 128, WIDTH, WT><<<grid(s->trace_blocks[wi][0][1][0], 128), 128, 0, st>>>(d, rays, n_static, n_dev, hits, occ, w, counters, stride, roots, res);
+        if (any_hit) go(k_trace<true, true, 128, WIDTH, WT, kWalkPlain>, b[1][1][0], 128);
+        else go(k_trace<false, true, 128, WIDTH, WT, kWalkPlain>, b[0][1][0], 128);
     } else if (s->tune_threads == 256) {
-        if (any_hit)
-            k_trace<true, false, 256, WIDTH, WT><<<grid(s->trace_blocks[wi][1][0][1], 256), 256, 0, st>>>(d, rays, n_static, n_dev, hits, occ, w, nullptr, 1, roots, res);
-        else
-            k_trace<false, false, 256, WIDTH, WT><<<grid(s->trace_blocks[wi][0][0][1], 256), 256, 0, st>>>(d, rays, n_static, n_dev, hits, occ, w, nullptr, 1, roots, res);
+        if (any_hit) go(k_trace<true, false, 256, WIDTH, WT, WALK>, b[1][0][1], 256);
+        else go(k_trace<false, false, 256, WIDTH, WT, WALK>, b[0][0][1], 256);
     } else if (any_hit) {
-        k_trace<true, false, 128, WIDTH, WT><<<grid(s->trace_blocks[wi][1][0][0], 128), 128, 0, st>>>(d, rays, n_static, n_dev, hits, occ, w, nullptr, 1, roots, res);
+        go(k_trace<true, false, 128, WIDTH, WT, WALK>, b[1][0][0], 128);
     } else {
-        k_trace<false, false, 128, WIDTH, WT><<<grid(s->trace_blocks[wi][0][0][0], 128), 128, 0, st>>>(d, rays, n_static, n_dev, hits, occ, w, nullptr, 1, roots, res);
+        go(k_trace<false, false, 128, WIDTH, WT, WALK>, b[0][0][0], 128);
     }
 }
 
+template <int WIDTH, bool WT>
+static void launch_width(bg_scene* s, bool render, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
+                         bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
+                         unsigned long long* w, const int* roots, const ShadowResolve& res) {
+    const int walk = counters ? kWalkPlain : choose_walk<WIDTH>(s->dev, render);   // (counting replays: the plain walk)
+    if (walk == kWalkPacked)
+        launch_walk<WIDTH, WT, kWalkPacked>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else if (walk == kWalkFused)
+        launch_walk<4, WT, kWalkFused>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else
+        launch_walk<WIDTH, WT, kWalkPlain>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+}
+
 // The traversal kernel of the scene's node layout and intersection test.
-static void launch_layout(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
+static void launch_layout(bg_scene* s, bool render, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                           bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
-                          unsigned long long* w, const int* roots, ShadowResolve res) {
+                          unsigned long long* w, const int* roots, const ShadowResolve& res) {
     // (Measured and rejected: any-hit rays on the 8-wide nodes while closest-hit
     // rays use the 4-wide ones: the C3 shadow traversal took 16.6 instead of 13.6 ms.)
     const bool w8 = s->dev.width == 8, wt = s->dev.watertight != 0;
-    if (w8 && wt) launch_width<8, true>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
-    else if (w8) launch_width<8, false>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
-    else if (wt) launch_width<4, true>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
-    else launch_width<4, false>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    if (w8 && wt) launch_width<8, true>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else if (w8) launch_width<8, false>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else if (wt) launch_width<4, true>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else launch_width<4, false>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
 }
 
 int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                  bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
                  unsigned long long* work, const int* roots, const ShadowResolve* resolve) {
     unsigned long long* w = work ? work : next_work_counter(s);   // the caller's is cleared
-    if (!work) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
     ShadowResolve res{nullptr, nullptr, nullptr, 0};
     if (resolve && !counters) {
         if (any_hit) res = *resolve;
         else res.hit_class = resolve->hit_class;
     }
-    launch_layout(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    if (!work) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
+    // ray indices are 32-bit in the kernel: a larger array goes in pieces
+    // (counting replays keep one output per ray replayed: pieces are whole strides)
+    const int64_t piece = (int64_t(1) << 30) / stride * stride;
+    for (int64_t at = 0; at == 0 || at < n_static; at += piece) {
+        if (at > 0) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
+        launch_layout(s, n_dev != nullptr, any_hit, rays + 2 * at, std::min(n_static - at, piece), n_dev, hits ? hits + at / stride : nullptr,
+                      occ ? occ + at / stride : nullptr, st, counters, stride, w, roots, res);
+    }
     BG_CUDA(cudaGetLastError());
     return BG_OK;
 }
@@ -455,6 +514,8 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
             return set_error(BG_ERR_UNSUPPORTED, "8-wide BVH needs a %d-entry traversal stack (> %d)", ms8, kStackSize8);
         nn8 = 0;
     }
+    bool packed = false;
+    if (nn4 && (rc = device_pack_nodes(s->nodes.as<WideNode4>(), nn4, s->qnodes, &packed))) return rc;
     const auto tb1 = std::chrono::steady_clock::now();
     // traversal records in leaf order, shading records in primitive order
     if ((rc = s->tris.ensure(size_t(ntris) * sizeof(TriRec))) || (rc = s->shade.ensure(size_t(ntris) * sizeof(ShadeRec))))
@@ -483,6 +544,7 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
     BG_CUDA(cudaMemset(s->work.ptr, 0, kWorkSlots * sizeof(unsigned long long)));
     DevScene& d = s->dev;
     d.nodes = nn4 ? s->nodes.as<WideNode4>() : nullptr;
+    d.qnodes = packed ? s->qnodes.as<QNode4>() : nullptr;
     d.nodes8 = nn8 ? s->nodes8.as<QNode8>() : nullptr;
     s->nnodes4 = nn4;
     s->nnodes8 = nn8;
@@ -502,6 +564,8 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
     d.has_area = 0;
     for (const LightRec& L : lights) d.has_area |= L.type == BG_LIGHT_AREA ? 1 : 0;
     d.watertight = watertight ? 1 : 0;
+    d.extent = 0.f;
+    for (int k = 0; k < 3; ++k) d.extent = std::max(d.extent, std::max(std::fabs(s->bbox_lo[k]), std::fabs(s->bbox_hi[k])));
     d.bg[0] = s->bg[0]; d.bg[1] = s->bg[1]; d.bg[2] = s->bg[2];
     scene_launch_setup(s);
     auto t1 = std::chrono::steady_clock::now();
@@ -618,8 +682,8 @@ int bg_scene_destroy(bg_scene* s) {
     {
         DeviceGuard dg(ctx->device);
         cudaDeviceSynchronize();
-        for (DevBuf* b : {&s->nodes, &s->nodes8, &s->tris, &s->shade, &s->bundles, &s->mats_d, &s->lights_d, &s->err,
-                          &s->work, &s->host_rays, &s->host_out})
+        for (DevBuf* b : {&s->nodes, &s->qnodes, &s->nodes8, &s->tris, &s->shade, &s->bundles, &s->mats_d,
+                          &s->lights_d, &s->err, &s->work, &s->host_rays, &s->host_out})
             b->release();
         if (s->render) render_state_free(s->render);
         if (s->ev_accum) cudaEventDestroy(s->ev_accum);
@@ -731,8 +795,8 @@ int bg_scene_commit(bg_scene* s, const bg_build_opts* opts) {
     if (rc != BG_OK) {
         // a failed commit keeps nothing on the device: the scene stays
         // uncommitted and may be committed again (e.g. after memory is freed)
-        for (DevBuf* b : {&s->nodes, &s->nodes8, &s->tris, &s->shade, &s->bundles, &s->mats_d, &s->lights_d, &s->err,
-                          &s->work})
+        for (DevBuf* b : {&s->nodes, &s->qnodes, &s->nodes8, &s->tris, &s->shade, &s->bundles, &s->mats_d,
+                          &s->lights_d, &s->err, &s->work})
             b->release();
         s->dev = DevScene{};
         s->nnodes4 = s->nnodes8 = 0;
@@ -916,7 +980,7 @@ int bg_traversal_counts(bg_scene* s, const bg_ray* rays, int64_t n, int32_t any_
         rc = launch_trace(s, any_hit != 0, reinterpret_cast<const float4*>(rays), n, nullptr, hits, occ, st, cnt, 1);
         if (rc) { tmp.release(); return rc; }
     }
-    unsigned long long h[3] = {0, 0, 0};
+    unsigned long long h[3] = {0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     tmp.release();
@@ -1002,11 +1066,11 @@ extern "C" int bg_traversal_counts_noalloc(bg_scene* s, const bg_ray* rays, int6
     cudaError_t e = cudaMemsetAsync(base, 0, kNoAllocHeader, st);   // counters and work counter start at zero
     if (e == cudaSuccess && n > 0) {
         const float4* r4 = reinterpret_cast<const float4*>(rays);
-        launch_layout(s, any_hit != 0, r4, n, nullptr, any_hit ? nullptr : hits, any_hit ? occ : nullptr, st, cnt, 1,
+        launch_layout(s, false, any_hit != 0, r4, n, nullptr, any_hit ? nullptr : hits, any_hit ? occ : nullptr, st, cnt, 1,
                       work, nullptr, ShadowResolve{nullptr, nullptr, nullptr, 0});
         e = cudaGetLastError();
     }
-    unsigned long long h[3] = {0, 0, 0};
+    unsigned long long h[3] = {0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return set_error(BG_ERR_CUDA, "bg_traversal_counts_noalloc: %s", cudaGetErrorString(e));

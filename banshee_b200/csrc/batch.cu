@@ -190,6 +190,9 @@ int bg_batch_commit(bg_batch* b) {
     BG_CUDA(cudaDeviceSynchronize());
     DevScene& d = M.dev;
     d.nodes = all4 ? M.nodes.as<WideNode4>() : nullptr;
+    bool packed = false;
+    if (all4 && (rc = device_pack_nodes(M.nodes.as<WideNode4>(), nn, M.qnodes, &packed))) return rc;
+    d.qnodes = packed ? M.qnodes.as<QNode4>() : nullptr;
     d.nodes8 = all8 ? M.nodes8.as<QNode8>() : nullptr;
     d.width = all4 ? (all8 ? kDefaultNodeWidth : 4) : 8;
     M.nnodes4 = nn; M.nnodes8 = nn8;
@@ -206,6 +209,8 @@ int bg_batch_commit(bg_batch* b) {
     d.has_area = 0;
     for (bg_scene* s : b->scenes) d.has_area |= s->dev.has_area;
     d.watertight = b->scenes[0]->dev.watertight;
+    d.extent = 0.f;
+    for (bg_scene* s : b->scenes) d.extent = std::max(d.extent, s->dev.extent);
     scene_launch_setup(&M);
     bg_scene_info& info = M.info;
     info.ntriangles = nt;
@@ -349,7 +354,7 @@ int bg_batch_destroy(bg_batch* b) {
         bg_scene& M = b->merged;
         DeviceGuard dg(ctx->device);
         cudaDeviceSynchronize();
-        for (DevBuf* d : {&M.nodes, &M.nodes8, &M.tris, &M.shade, &M.bundles, &M.mats_d, &M.lights_d, &M.err, &M.work,
+        for (DevBuf* d : {&M.nodes, &M.qnodes, &M.nodes8, &M.tris, &M.shade, &M.bundles, &M.mats_d, &M.lights_d, &M.err, &M.work,
                           &M.host_rays, &M.host_out})
             d->release();
         if (M.render) { render_state_free(M.render); M.render = nullptr; }

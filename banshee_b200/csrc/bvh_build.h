@@ -19,7 +19,7 @@ constexpr int32_t kEmptyChild = 0x7fffffff;
 constexpr int kLeafStartBits = 27;
 constexpr int32_t kMaxLeafStart = (1 << kLeafStartBits) - 1;
 
-inline int32_t encode_leaf(int32_t start, int32_t count) {
+constexpr int32_t encode_leaf(int32_t start, int32_t count) {
     return int32_t(0x80000000u | (uint32_t(count - 1) << kLeafStartBits) | uint32_t(start));
 }
 
@@ -51,6 +51,23 @@ struct alignas(32) QNode8 {
     uint32_t qx[4], qy[4], qz[4];
 };
 static_assert(sizeof(QNode8) == 96, "compressed node must be three 32-byte sectors");
+
+// 64-byte form of a WideNode4 (same index, same child codes): what the
+// traversal walks.  Per axis a plane byte q lies at o_a + (2^15 + q) * s_a
+// (o_a: the grid origin less 2^15 s_a), which the traversal evaluates as
+// fmaf(2^15 + q, s_a / d_a, (o_a - ray origin_a) / d_a): the byte is placed in
+// the mantissa of the float 2^15 + q.  lo bytes are rounded down and hi bytes
+// up with 1/64 of a step to spare, four times the rounding of that expression
+// (2^-9 of a step for each of its two roundings at 2^15 steps), so every plane
+// is conservative as evaluated.  Byte k of a word belongs to child k.
+struct alignas(32) QNode4 {
+    float ox, oy, oz, sx;
+    float sy, sz;
+    uint32_t lox, hix;
+    uint32_t loy, hiy, loz, hiz;
+    int32_t child[4];
+};
+static_assert(sizeof(QNode4) == 64, "packed node must be two 32-byte sectors");
 
 struct BuildParams {
     int max_leaf = 4;       // triangles per leaf

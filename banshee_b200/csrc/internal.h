@@ -111,7 +111,7 @@ struct bg_scene {
     float bbox_lo[3] = {0.f, 0.f, 0.f}, bbox_hi[3] = {0.f, 0.f, 0.f};   // world bounds of all triangles
     bool committed = false;
 
-    bg::DevBuf nodes, tris, shade, bundles, mats_d, lights_d, err;
+    bg::DevBuf nodes, qnodes, tris, shade, bundles, mats_d, lights_d, err;
     bg::DevBuf work;          // persistent-kernel work counters (scratch)
     std::atomic<unsigned> work_slot{0};
     bg::DevBuf host_rays, host_out;   // staging of bg_render_host
@@ -119,7 +119,7 @@ struct bg_scene {
     bg::DevScene dev{};
     bg_scene_info info{};
     bg::RenderState* render = nullptr;
-    int trace_blocks[2][2][2][2] = {};   // [width 4/8][any][count][128/256 threads]: persistent grid sizes
+    int trace_blocks[4][2][2][2][2] = {};   // [walk][width 4/8][any][count][128/256 threads]: persistent grid sizes
     int64_t tune_paths = 0;   // autotuned paths per pass (0 = default)
     int tune_threads = 0;     // autotuned traversal block size (0 = default 128)
     bg::DevBuf nodes8;        // 8-wide compressed tree (empty if not built)
@@ -159,11 +159,6 @@ int sah_binary_tree(const float* lo, const float* hi, int64_t n, int32_t* sorted
 struct MeshArrays {
     ScratchBuf verts, normals, uvs, vi, ni, ti, mat, offs, bundle, lo, hi, bbox;
 };
-// material class of a hit (bits 28-29 of a packed primid): 0 misses / emissive,
-// 1 Lambert, 2 GGX; primids stay below 2^27
-constexpr int kPrimMask = (1 << 28) - 1;
-constexpr int kClassShift = 28;
-
 int upload_mesh_arrays(const std::vector<MeshHost>& meshes, int64_t ntris, MeshArrays& A);
 // world boxes into A.lo / A.hi (Mesh::GetShapeWorldBounds) and the scene bounds of their finite values
 int device_world_boxes(MeshArrays& A, const BundleRec* bundles, int64_t ntris, float bbox_lo[3], float bbox_hi[3]);
@@ -172,6 +167,9 @@ int device_world_boxes(MeshArrays& A, const BundleRec* bundles, int64_t ntris, f
 // mat_class: class per material index (0 other, 1 Lambert, 2 GGX), stored in TriRec e2.w
 int device_records(const MeshArrays& A, const BundleRec* bundles, const int32_t* order, int64_t ntris,
                    TriRec* tris, ShadeRec* shade, bool vertices, const int32_t* mat_class, int nmat);
+// nodes packed for traversal (QNode4) into `out`; *packed = false when some
+// node's planes are outside the packed range (the traversal then walks `nodes`)
+int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* packed);
 constexpr int kWorkSlots = 256;
 unsigned long long* next_work_counter(bg_scene* s);
 void scene_launch_setup(bg_scene* s);

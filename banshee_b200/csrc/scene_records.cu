@@ -203,6 +203,66 @@ int device_world_boxes(MeshArrays& A, const BundleRec* bundles, int64_t ntris, f
     return BG_OK;
 }
 
+// WideNode4 -> QNode4, in double precision: the step of an axis is 1/250 of the
+// children's extent, but at least 2^-22 of the largest coordinate, so that the
+// float rounding of the grid origin stays below half a step.
+__global__ void k_pack_nodes(const WideNode4* __restrict__ nodes, int64_t n, QNode4* __restrict__ out,
+                             unsigned int* __restrict__ bad) {
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        const float* f = reinterpret_cast<const float*>(nodes + i);   // lo x 4, hi x 4, lo y ...
+        QNode4 q;
+        float org[3], step[3];
+        uint32_t lo[3], hi[3];
+        bool ok = true;
+        for (int k = 0; k < 4; ++k) q.child[k] = nodes[i].child[k];
+        for (int a = 0; a < 3; ++a) {
+            double L = 0.0, H = 0.0;
+            bool any = false;
+            for (int k = 0; k < 4; ++k) {
+                if (q.child[k] == kEmptyChild) continue;
+                const float l = f[8 * a + k], h = f[8 * a + 4 + k];
+                ok = ok && fabsf(l) <= 1e15f && fabsf(h) <= 1e15f;   // (false for NaN)
+                L = any ? fmin(L, double(l)) : double(l);
+                H = any ? fmax(H, double(h)) : double(h);
+                any = true;
+            }
+            const double big = fmax(fabs(L), fabs(H));
+            const double sd = fmax(fmax((H - L) * (1.0 / 250.0), big * (1.0 / 4194304.0)), 1e-18);
+            step[a] = __double2float_ru(sd);
+            org[a] = __double2float_rn(L - 32770.0 * double(step[a]));
+            const double base = double(org[a]) + 32768.0 * double(step[a]);
+            lo[a] = hi[a] = 0u;
+            for (int k = 0; k < 4; ++k) {
+                if (q.child[k] == kEmptyChild) { lo[a] |= 255u << (8 * k); continue; }
+                const double ql = floor((double(f[8 * a + k]) - base) / double(step[a]) - 1.0 / 64.0);
+                const double qh = ceil((double(f[8 * a + 4 + k]) - base) / double(step[a]) + 1.0 / 64.0);
+                ok = ok && ql >= 0.0 && qh <= 255.0;
+                lo[a] |= (uint32_t(int(ql)) & 255u) << (8 * k);
+                hi[a] |= (uint32_t(int(qh)) & 255u) << (8 * k);
+            }
+        }
+        q.ox = org[0]; q.oy = org[1]; q.oz = org[2];
+        q.sx = step[0]; q.sy = step[1]; q.sz = step[2];
+        q.lox = lo[0]; q.hix = hi[0]; q.loy = lo[1]; q.hiy = hi[1]; q.loz = lo[2]; q.hiz = hi[2];
+        out[i] = q;
+        if (!ok) atomicOr(bad, 1u);
+    }
+}
+
+int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* packed) {
+    *packed = false;
+    ScratchBuf bad;
+    int rc;
+    if ((rc = out.ensure(size_t(n) * sizeof(QNode4))) || (rc = bad.ensure(sizeof(unsigned)))) return rc;
+    BG_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned), 0));
+    k_pack_nodes<<<grid_for(n), kRT>>>(nodes, n, out.as<QNode4>(), bad.as<unsigned>());
+    BG_CUDA(cudaGetLastError());
+    unsigned h = 0;
+    BG_CUDA(cudaMemcpy(&h, bad.ptr, sizeof(h), cudaMemcpyDeviceToHost));
+    *packed = h == 0;
+    return BG_OK;
+}
+
 int device_records(const MeshArrays& A, const BundleRec* bundles, const int32_t* order, int64_t ntris, TriRec* tris,
                    ShadeRec* shade, bool vertices, const int32_t* mat_class, int nmat) {
     k_tri_records<<<grid_for(ntris), kRT>>>(ntris, order, A.bundle.as<int32_t>(), A.offs.as<MeshOff>(),

@@ -1,6 +1,7 @@
 // Device-resident scene layout (HBM), shared by host upload code and kernels.
 //
 //   nodes    WideNode4[nnodes]   128 B, one L2 line per 4-wide node
+//   qnodes   QNode4[nnodes]       64 B, the 4-wide nodes packed for traversal
 //   nodes8   QNode8[nnodes8]      96 B, three 32-byte sectors per 8-wide compressed node
 //   tris     TriRec[ntris]        48 B, leaf order; what traversal streams
 //   shade    ShadeRec[ntris]     112 B, global primitive order; read once per hit
@@ -65,8 +66,14 @@ struct LightRec {
     float pad;
 };
 
+// material class of a hit (bits 28-29 of a packed primid): 0 misses / emissive,
+// 1 Lambert, 2 GGX; primids stay below 2^27
+constexpr int kPrimMask = (1 << 28) - 1;
+constexpr int kClassShift = 28;
+
 struct DevScene {
     const WideNode4* nodes;
+    const QNode4* qnodes;   // nodes packed for traversal (null: planes out of the packed range)
     const QNode8* nodes8;
     const TriRec* tris;
     const ShadeRec* shade;
@@ -80,7 +87,7 @@ struct DevScene {
     float bg[3];
     int32_t has_area;       // some light is an AreaLight (selects the shading variant)
     int32_t watertight;     // tris hold (p1, p2, p3) for the watertight test, not (p1, e1, e2)
-    int32_t pad3;
+    float extent;           // largest |coordinate| of the world bounds
 };
 
 }  // namespace bg

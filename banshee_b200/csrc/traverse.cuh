@@ -8,12 +8,26 @@
 //     computed with the reference's exact operation order in the bundle's
 //     object space (ray transformed by minv as transform_ray does,
 //     math/mathutils.h:154-157; skipped for identity bundles, where it is exact);
-//   * the box test is this project's own: a slab test with a relative slack of
-//     4e-7 on the exit distance (more than the 2*gamma(3) rounding bound of
-//     (lo - o) * (1/d)), so no box that holds an accepted triangle is culled.
+//   * the box test is this project's own: a slab test with a relative slack on
+//     the exit distance, so no box that holds an accepted triangle is culled.
 // Children are visited nearest-first; stack entries keep their entry distance
 // and are culled against the current closest hit, widened by the same slack,
 // when popped.
+//
+// Two kinds of walk share the code:
+//   plain  slabs as (plane - o) * (1/d), slack 4e-7 (more than the 2*gamma(3)
+//          rounding bound).  Among triangles whose t are equal to the last bit the
+//          one visited last wins, so its visiting order is part of the result.
+//   packed one fused multiply-add per plane with a per-ray bound of the roundings,
+//          on the 64-byte QNode4 nodes, on the 128-byte nodes (fused) or on the
+//          8-wide nodes, slack 1e-5.  Its boxes contain the plain ones, its order
+//          differs in detail.  A closest-hit ray that ends with a second triangle
+//          within 1e-5 (relative) of its closest t is walked again on the plain
+//          nodes, so ids, t, u and v are those of the plain walk, ties included;
+//          an any-hit answer does not depend on the order.
+// Rays the packed arithmetic does not cover (a direction component of 0 or out
+// of range, not finite) take the plain walk from the start, as does the
+// instrumented replay (COUNT).
 #pragma once
 
 #include <type_traits>
@@ -26,21 +40,30 @@ namespace bg {
 
 constexpr int kStackSize = 64;     // entries per ray, 4-wide; the builder checks max_stack against it
 constexpr int kStackSize8 = 96;    // entries per ray, 8-wide (up to 7 pushes per level)
-// stack entries per ray kept in shared memory: 8 for the 4-wide traversal
-// (measured: +6 % incoherent / +3 % coherent ray casts), none for the 8-wide one
-template <int WIDTH>
-__host__ __device__ constexpr int smem_stack_entries() { return WIDTH == 4 ? 8 : 0; }
+// Walks (template parameter WALK): kWalkPlain the plain walk alone; kWalkPacked
+// and kWalkFused the packed arithmetic on QNode4 / QNode8 nodes and on the
+// 128-byte nodes.
+constexpr int kWalkPlain = 0, kWalkPacked = 1, kWalkFused = 3;
+
+// stack entries per ray kept in shared memory: 8 for the 4-wide walks, 12 for the
+// packed one (1M-triangle soup, closest / any incoherent: 4 entries 1241 / 1646
+// Mrays/s, 8 1360 / 1779, 12 1436 / 1835), none for the 8-wide ones
+template <int WIDTH, int WALK>
+__host__ __device__ constexpr int smem_stack_entries() { return WIDTH == 8 ? 0 : WALK == kWalkPacked ? 12 : 8; }
 template <int WIDTH>
 __host__ __device__ constexpr int stack_entries() { return WIDTH == 8 ? kStackSize8 : kStackSize; }
-// traversal steps between warp refill points (measured on passes of 2^24 paths:
-// closest hit 24 > 16 > 12 by about 1 % of the frame; any hit 16 > 8, 32).
+// Traversal steps between warp refill points.  Renders (fused and plain walk):
+// closest hit 24 > 16 > 12 by about 1 % of the frame, any hit 16 > 8, 32; 12 / 8
+// cost the C3 frame 3 %.  Casts on packed nodes: 12 / 8 (coherent closest 1953
+// against 1878 Mrays/s at 24 / 16, incoherent any 1865 against 1798), 8-wide nodes
+// the same (incoherent any 1615 against 1530).
 // (Measured and rejected: each lane's next ray prefetched into shared memory by
 // cp.async from a per-warp pool of 32 indices, refilling every 24 / 12 / 8 / 4
 // steps: C3 567 -> 528 / 519 / 511 / 280 Msamples/s with 4-wide nodes; and
 // registers capped at 48 or 40 for 40 or 48 resident warps per SM: spills,
 // 559 -> 544 / 495 Msamples/s.)
-constexpr int kRefillStepsClosest = 24;
-constexpr int kRefillStepsAny = 16;
+template <bool ANY, int WALK>
+__host__ __device__ constexpr int refill_steps() { return WALK == kWalkPacked ? (ANY ? 8 : 12) : (ANY ? 16 : 24); }
 constexpr float kBoxSlack = 4e-7f;
 // The slack is applied as one fused multiply-add, t1 + |t1| * kBoxSlack rounded
 // once: the same half-ulp guarantee as a multiply and an add (whose product
@@ -52,20 +75,104 @@ constexpr float kBoxSlack = 4e-7f;
 // is huge for rays nearly parallel to an axis, so such rays visited most of the
 // tree: C3 ran at 8 instead of 500 Msamples/s.)
 
-struct Ray {
+// Slack of the packed walk: its box tests, its culling of popped entries and
+// the distance within which a second hit sends the ray to the plain walk.
+constexpr float kFastSlack = 1e-5f;
+
+// Ray::flags: bits 0-2 sign of 1/d per axis
+constexpr uint32_t kOctMask = 7u;
+constexpr uint32_t kPlainWalk = 8u;   // walk the plain nodes
+constexpr uint32_t kNearTie = 16u;    // packed walk: a second triangle near the closest one
+
+// kWalkPacked and kWalkFused keep the ray's origin and direction, which they need
+// only for a new bundle's object-space ray and for a plain visit, in shared memory:
+// six registers less during the walk (from global memory, C3 was 3 % slower).
+struct RayFast {
+    v3 inv;          // 1 / d
+    v3 cn, cf;       // -o / d less / plus a bound of the roundings: near / far planes
+    float tmin;
+    uint32_t flags;
+    int32_t idx;     // index in the ray array
+};
+template <int WALK>
+struct Ray : RayFast {};
+template <>
+struct Ray<kWalkPlain> {
     v3 o, d, inv;
-    float tmin, tmax;
-    uint32_t oct;    // bit k set: direction component k is negative (sign of 1/d)
+    float tmin;
+    uint32_t flags;
+    int32_t idx;
 };
 
-__device__ __forceinline__ Ray make_ray(float4 a, float4 b) {
-    Ray r;
-    r.o = mk(a.x, a.y, a.z); r.tmin = a.w;
-    r.d = mk(b.x, b.y, b.z); r.tmax = b.w;
-    r.inv = mk(1.f / r.d.x, 1.f / r.d.y, 1.f / r.d.z);
-    r.oct = (signbit(r.inv.x) ? 1u : 0u) | (signbit(r.inv.y) ? 2u : 0u) | (signbit(r.inv.z) ? 4u : 0u);
+// the scene and the ray array of one launch
+struct TraceScene : DevScene {
+    const float4* rays;
+    float4* own;      // this lane's ray in shared memory (kWalkPacked, kWalkFused): o at own[0], d at own[ownstep]
+    int ownstep;
+};
+
+// Whether the packed arithmetic covers the scene.
+template <int WIDTH>
+__host__ __device__ __forceinline__ bool packed_walk(const DevScene& S) {
+    return S.extent <= 1e15f && (WIDTH == 8 || S.qnodes != nullptr);
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+__device__ __forceinline__ uint32_t octant(v3 inv) {
+    return (__float_as_uint(inv.x) >> 31) | ((__float_as_uint(inv.y) >> 30) & 2u) | ((__float_as_uint(inv.z) >> 29) & 4u);
+}
+
+// walk: kPlainWalk to walk the plain nodes whatever the ray, 0 otherwise
+__device__ __forceinline__ void make_ray(RayFast& r, float extent, uint32_t walk, float4 a, float4 b, int32_t idx) {
+    r.idx = idx;
+    r.tmin = a.w;
+    r.inv = mk(1.f / b.x, 1.f / b.y, 1.f / b.z);
+    const v3 ai = mk(fabsf(r.inv.x), fabsf(r.inv.y), fabsf(r.inv.z));
+    const float far = max3(fabsf(a.x), fabsf(a.y), fabsf(a.z));
+    // the packed arithmetic's range (comparisons false for NaN: plain walk)
+    const bool ok = ai.x <= 1e15f && ai.y <= 1e15f && ai.z <= 1e15f && min3(ai.x, ai.y, ai.z) >= 1e-15f && far <= 1e15f;
+    r.flags = octant(r.inv) | (ok ? walk : kPlainWalk);
+    // every rounding of a plane's distance (of 1/d, of the intercepts, of the final
+    // multiply-add) is at most 2^-24 of (|plane| + |o|) / |d|; five of them add up
+    const float e = (extent + far) * 4.8e-7f;
+    const float ex = fmaf(e, ai.x, 1e-36f), ey = fmaf(e, ai.y, 1e-36f), ez = fmaf(e, ai.z, 1e-36f);
+    const float ox = a.x * r.inv.x, oy = a.y * r.inv.y, oz = a.z * r.inv.z;
+    r.cn = mk(-ox - ex, -oy - ey, -oz - ez);
+    r.cf = mk(ex - ox, ey - oy, ez - oz);
+}
+__device__ __forceinline__ void make_ray(Ray<kWalkPlain>& r, float, uint32_t, float4 a, float4 b, int32_t idx) {
+    r.idx = idx;
+    r.tmin = a.w;
+    r.inv = mk(1.f / b.x, 1.f / b.y, 1.f / b.z);
+    r.flags = octant(r.inv) | kPlainWalk;
+}
+// keeping and giving back the ray's origin and direction
+__device__ __forceinline__ void keep_ray(const TraceScene& S, RayFast&, float4 a, float4 b) {
+    S.own[0] = a;
+    S.own[S.ownstep] = b;
+}
+__device__ __forceinline__ void world_ray(const TraceScene& S, const RayFast&, v3& o, v3& d) {
+    const float4 a = S.own[0], b = S.own[S.ownstep];
+    o = mk(a.x, a.y, a.z);
+    d = mk(b.x, b.y, b.z);
+}
+template <class RAY>
+__device__ __forceinline__ void keep_regs(RAY& r, float4 a, float4 b) {
+    r.o = mk(a.x, a.y, a.z);
+    r.d = mk(b.x, b.y, b.z);
+}
+__device__ __forceinline__ void keep_ray(const TraceScene&, Ray<kWalkPlain>& r, float4 a, float4 b) { keep_regs(r, a, b); }
+__device__ __forceinline__ void world_ray(const TraceScene&, const Ray<kWalkPlain>& r, v3& o, v3& d) { o = r.o; d = r.d; }
 
 // Mesh::IntersectFace (primitive/mesh.cpp:7-45), bit-exact.
 __device__ __forceinline__ bool mt_test(v3 o, v3 d, v3 p1, v3 e1, v3 e2, float tmin, float tmax,
@@ -115,19 +222,17 @@ __device__ __forceinline__ void shear(ObjRayWT& c) {
     c.sz = 1.f / dz;
 }
 
-template <class OR>
-__device__ __forceinline__ void obj_ray(const DevScene& S, const Ray& r, int b, OR& c) {
+template <class RAY, class OR>
+__device__ __forceinline__ void obj_ray(const TraceScene& S, const RAY& r, int b, OR& c) {
     if (b == c.bundle) return;
     c.bundle = b;
-    if (b < 0) {
-        c.o = r.o; c.d = r.d;
-    } else {
-        const float* mi = S.bundles[b].minv;
-        float m[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) m[k] = __ldg(mi + k);
-        c.o = xf_point(m, r.o);
-        c.d = xf_vector(m, r.d);
+    world_ray(S, r, c.o, c.d);
+    if (b >= 0) {
+        const float4* mi = reinterpret_cast<const float4*>(S.bundles[b].minv);   // three 16-byte rows
+        const float4 m0 = __ldg(mi), m1 = __ldg(mi + 1), m2 = __ldg(mi + 2);
+        const float m[12] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w, m2.x, m2.y, m2.z, m2.w};
+        c.o = xf_point(m, c.o);
+        c.d = xf_vector(m, c.d);
     }
     shear(c);
 }
@@ -167,90 +272,238 @@ __device__ __forceinline__ bool wt_test(const ObjRayWT& c, v3 p1, v3 p2, v3 p3, 
     return true;
 }
 
-// Test the 4 children of node `ni`; returns a hit mask and entry distances.
-__device__ __forceinline__ uint32_t box4(const WideNode4* __restrict__ nodes, int ni, const Ray& r, float best,
-                                         float tn[4], int32_t ch[4]) {
-    // the near / far planes of each axis are picked by load address (the node
-    // stores lo and hi of an axis in adjacent float4s), not by per-plane selects
-    const float4* p = reinterpret_cast<const float4*>(nodes + ni);
-    const int fx = int(r.oct & 1u), fy = int((r.oct >> 1) & 1u), fz = int((r.oct >> 2) & 1u);
+// entry distance of a child that is not hit: +inf
+#define kMiss __int_as_float(0x7f800000)
+
+// Orders four children by entry distance with a sorting network on registers
+// (a missed child's +inf sorts last).
+// ALL = false: only the nearest comes first (an any-hit ray: the order of the
+// others does not pay for its two comparators).
+template <bool ALL = true>
+__device__ __forceinline__ void sort4(float (&t)[4], int32_t (&c)[4]) {
+    auto cex = [&](int a, int b) {
+        const bool sw = t[a] > t[b];
+        const float ta = t[a], tb = t[b];
+        const int ca = c[a], cb = c[b];
+        t[a] = sw ? tb : ta; t[b] = sw ? ta : tb;
+        c[a] = sw ? cb : ca; c[b] = sw ? ca : cb;
+    };
+    cex(0, 1); cex(2, 3); cex(0, 2);
+    if (ALL) { cex(1, 3); cex(1, 2); }
+}
+
+// Plain visit of 4-wide node p: its children in order of entry distance, +inf for
+// one that is not hit.  A ray with infinite direction components can enter an empty
+// slot (all its slabs are 0 or NaN); such a child is dropped when it is popped, or
+// here (DROP) where the walk's pops do not test for it: that test in every pop cost
+// the fused any-hit walk 5 %.  (The near / far planes of each axis are picked by load
+// address: the node stores lo and hi of an axis in adjacent float4s.)
+struct Children4 {
+    float t[4];
+    int32_t c[4];
+    int nh;      // the first nh were hit
+};
+template <bool DROP>
+__device__ __forceinline__ Children4 box4_plain(const float4* __restrict__ p, v3 o, v3 inv, uint32_t flags, float tmin,
+                                                float best) {
+    const int fx = int(flags & 1u), fy = int((flags >> 1) & 1u), fz = int((flags >> 2) & 1u);
     const float4 nx4 = __ldg(p + fx), fx4 = __ldg(p + (1 - fx));
     const float4 ny4 = __ldg(p + 2 + fy), fy4 = __ldg(p + 3 - fy);
     const float4 nz4 = __ldg(p + 4 + fz), fz4 = __ldg(p + 5 - fz);
-    int4 c = __ldg(reinterpret_cast<const int4*>(p + 6));
+    const int4 c = __ldg(reinterpret_cast<const int4*>(p + 6));
     const float nxa[4] = {nx4.x, nx4.y, nx4.z, nx4.w}, fxa[4] = {fx4.x, fx4.y, fx4.z, fx4.w};
     const float nya[4] = {ny4.x, ny4.y, ny4.z, ny4.w}, fya[4] = {fy4.x, fy4.y, fy4.z, fy4.w};
     const float nza[4] = {nz4.x, nz4.y, nz4.z, nz4.w}, fza[4] = {fz4.x, fz4.y, fz4.z, fz4.w};
-    ch[0] = c.x; ch[1] = c.y; ch[2] = c.z; ch[3] = c.w;
-    uint32_t mask = 0;
+    Children4 r;
+    r.c[0] = c.x; r.c[1] = c.y; r.c[2] = c.z; r.c[3] = c.w;
+    r.nh = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        float ax = (nxa[i] - r.o.x) * r.inv.x;
-        float bx = (fxa[i] - r.o.x) * r.inv.x;
-        float ay = (nya[i] - r.o.y) * r.inv.y;
-        float by = (fya[i] - r.o.y) * r.inv.y;
-        float az = (nza[i] - r.o.z) * r.inv.z;
-        float bz = (fza[i] - r.o.z) * r.inv.z;
-        float t0 = fmaxf(fmaxf(ax, ay), fmaxf(az, r.tmin));
+        float ax = (nxa[i] - o.x) * inv.x;
+        float bx = (fxa[i] - o.x) * inv.x;
+        float ay = (nya[i] - o.y) * inv.y;
+        float by = (fya[i] - o.y) * inv.y;
+        float az = (nza[i] - o.z) * inv.z;
+        float bz = (fza[i] - o.z) * inv.z;
+        float t0 = fmaxf(fmaxf(ax, ay), fmaxf(az, tmin));
         float t1 = fminf(fminf(bx, by), fminf(bz, best));
         t1 = fmaf(fabsf(t1), kBoxSlack, t1);
-        tn[i] = t0;
-        if (t0 <= t1) mask |= 1u << i;
+        const bool hit = t0 <= t1 && !(DROP && r.c[i] == kEmptyChild);
+        r.t[i] = hit ? t0 : kMiss;
+        r.nh += hit ? 1 : 0;
     }
-    return mask;
+    sort4(r.t, r.c);
+    return r;
 }
 
-// Test the 8 children of compressed node `ni`.  Each plane is dequantised
-// exactly (P = fmaf(2^23 + q, s, o2), see QNode8) and then tested exactly as in
-// box4, so the same slack argument holds.  Returns the hit mask over slots.
-__device__ __forceinline__ uint32_t box8(const QNode8* __restrict__ nodes, int ni, const Ray& r, float best,
-                                         float tn[8], int32_t ch[8]) {
+// 32 bytes in one load (32-byte aligned)
+struct Words8 {
+    uint32_t w[8];
+};
+__device__ __forceinline__ Words8 ldg256(const void* p) {
+    Words8 r;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7])
+        : "l"(p));
+    return r;
+}
+
+// Two multiply-adds in one instruction: {a0, a1} * {m, m} + {c0, c1}
+__device__ __forceinline__ float2 fma2(float a0, float a1, float m, float c0, float c1) {
+    float2 r;
+    asm("{\n\t.reg .b64 a, m, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 m, {%4, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+        "fma.rn.f32x2 d, a, m, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a0), "f"(a1), "f"(m), "f"(c0), "f"(c1));
+    return r;
+}
+// Near and far distance of the slab whose plane bytes are byte `i` of words n
+// and f: the bytes as the floats 2^15 + q, slope m, intercepts cn, cf.
+__device__ __forceinline__ float2 slab(uint32_t n, uint32_t f, int i, float m, float cn, float cf) {
+    const uint32_t sel = 0x7604u | (uint32_t(i) << 4);
+    return fma2(__uint_as_float(__byte_perm(n, 0x47000000u, sel)), __uint_as_float(__byte_perm(f, 0x47000000u, sel)), m, cn, cf);
+}
+
+// Test the 4 children of packed node `ni` (packed walk): entry distances, +inf
+// for a child that is not hit.  `cull`: the distance beyond which nothing
+// matters.  (An empty slot's byte box is inverted, but the slack can be longer
+// than a very small box: an empty child may come back as hit, and is dropped
+// where it is visited.)
+// What bounds the walk on incoherent rays is the L1's data pipe: 91-95 % of its
+// peak with the 128-byte nodes (seven 16-byte loads per visit, each lane on a
+// line of its own), issue slots 50 %.  Two 32-byte loads per visit bring it to
+// 54-62 %; the instructions of the byte decode (one PRMT per plane) are paid for
+// by the slabs' multiply-adds, two planes at a time.
+__device__ __forceinline__ void box4_packed(const QNode4* __restrict__ nodes, int ni, const RayFast& r, float cull,
+                                            float (&tn)[4], int32_t (&ch)[4]) {
+    const Words8 A = ldg256(nodes + ni), B = ldg256(reinterpret_cast<const char*>(nodes + ni) + 32);
+    auto F = [](uint32_t v) { return __uint_as_float(v); };
+    const float ix = F(A.w[3]) * r.inv.x, iy = F(A.w[4]) * r.inv.y, iz = F(A.w[5]) * r.inv.z;
+    const float2 cx = fma2(F(A.w[0]), F(A.w[0]), r.inv.x, r.cn.x, r.cf.x);
+    const float2 cy = fma2(F(A.w[1]), F(A.w[1]), r.inv.y, r.cn.y, r.cf.y);
+    const float2 cz = fma2(F(A.w[2]), F(A.w[2]), r.inv.z, r.cn.z, r.cf.z);
+    const bool gx = r.flags & 1u, gy = r.flags & 2u, gz = r.flags & 4u;
+    const uint32_t nx = gx ? A.w[7] : A.w[6], fx = gx ? A.w[6] : A.w[7];
+    const uint32_t ny = gy ? B.w[1] : B.w[0], fy = gy ? B.w[0] : B.w[1];
+    const uint32_t nz = gz ? B.w[3] : B.w[2], fz = gz ? B.w[2] : B.w[3];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 x = slab(nx, fx, i, ix, cx.x, cx.y), y = slab(ny, fy, i, iy, cy.x, cy.y), z = slab(nz, fz, i, iz, cz.x, cz.y);
+        const float t0 = fmaxf(max3(x.x, y.x, z.x), r.tmin), t1 = fminf(min3(x.y, y.y, z.y), cull);
+        tn[i] = t0 <= t1 ? t0 : kMiss;
+        ch[i] = int32_t(B.w[4 + i]);
+    }
+}
+
+// Fused visit of 4-wide node `ni`: the plain node's planes with the packed walk's
+// arithmetic, two children's planes in one instruction (12 multiply-adds instead
+// of 48 operations, and no slack per child).
+__device__ __forceinline__ void box4_fused(const WideNode4* __restrict__ nodes, int ni, const RayFast& r, float cull,
+                                           float (&tn)[4], int32_t (&ch)[4]) {
     const float4* p = reinterpret_cast<const float4*>(nodes + ni);
-    const float4 hd = __ldg(p);
-    const int4 c0 = __ldg(reinterpret_cast<const int4*>(p + 1));
-    const int4 c1 = __ldg(reinterpret_cast<const int4*>(p + 2));
-    const uint4 qx = __ldg(reinterpret_cast<const uint4*>(p + 3));
-    const uint4 qy = __ldg(reinterpret_cast<const uint4*>(p + 4));
-    const uint4 qz = __ldg(reinterpret_cast<const uint4*>(p + 5));
-    const uint32_t meta = __float_as_uint(hd.w);
-    const float sx = __uint_as_float((meta & 0xffu) << 23);
-    const float sy = __uint_as_float(((meta >> 8) & 0xffu) << 23);
-    const float sz = __uint_as_float(((meta >> 16) & 0xffu) << 23);
-    const uint32_t valid = meta >> 24;
-    // near / far plane bytes of slots 0-3 (.x) and 4-7 (.y) for this ray's octant
-    const bool nx = r.oct & 1u, ny = r.oct & 2u, nz = r.oct & 4u;
-    const uint2 qnx = nx ? make_uint2(qx.z, qx.w) : make_uint2(qx.x, qx.y);
-    const uint2 qfx = nx ? make_uint2(qx.x, qx.y) : make_uint2(qx.z, qx.w);
-    const uint2 qny = ny ? make_uint2(qy.z, qy.w) : make_uint2(qy.x, qy.y);
-    const uint2 qfy = ny ? make_uint2(qy.x, qy.y) : make_uint2(qy.z, qy.w);
-    const uint2 qnz = nz ? make_uint2(qz.z, qz.w) : make_uint2(qz.x, qz.y);
-    const uint2 qfz = nz ? make_uint2(qz.x, qz.y) : make_uint2(qz.z, qz.w);
-    ch[0] = c0.x; ch[1] = c0.y; ch[2] = c0.z; ch[3] = c0.w;
-    ch[4] = c1.x; ch[5] = c1.y; ch[6] = c1.z; ch[7] = c1.w;
-    uint32_t mask = 0;
+    const int fx = int(r.flags & 1u), fy = int((r.flags >> 1) & 1u), fz = int((r.flags >> 2) & 1u);
+    const float4 nx = __ldg(p + fx), gx = __ldg(p + (1 - fx));
+    const float4 ny = __ldg(p + 2 + fy), gy = __ldg(p + 3 - fy);
+    const float4 nz = __ldg(p + 4 + fz), gz = __ldg(p + 5 - fz);
+    const int4 c = __ldg(reinterpret_cast<const int4*>(p + 6));
+    ch[0] = c.x; ch[1] = c.y; ch[2] = c.z; ch[3] = c.w;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float2 ax = h ? fma2(nx.z, nx.w, r.inv.x, r.cn.x, r.cn.x) : fma2(nx.x, nx.y, r.inv.x, r.cn.x, r.cn.x);
+        const float2 ay = h ? fma2(ny.z, ny.w, r.inv.y, r.cn.y, r.cn.y) : fma2(ny.x, ny.y, r.inv.y, r.cn.y, r.cn.y);
+        const float2 az = h ? fma2(nz.z, nz.w, r.inv.z, r.cn.z, r.cn.z) : fma2(nz.x, nz.y, r.inv.z, r.cn.z, r.cn.z);
+        const float2 bx = h ? fma2(gx.z, gx.w, r.inv.x, r.cf.x, r.cf.x) : fma2(gx.x, gx.y, r.inv.x, r.cf.x, r.cf.x);
+        const float2 by = h ? fma2(gy.z, gy.w, r.inv.y, r.cf.y, r.cf.y) : fma2(gy.x, gy.y, r.inv.y, r.cf.y, r.cf.y);
+        const float2 bz = h ? fma2(gz.z, gz.w, r.inv.z, r.cf.z, r.cf.z) : fma2(gz.x, gz.y, r.inv.z, r.cf.z, r.cf.z);
+        const float t0 = fmaxf(max3(ax.x, ay.x, az.x), r.tmin), t1 = fmaxf(max3(ax.y, ay.y, az.y), r.tmin);
+        tn[2 * h] = t0 <= fminf(min3(bx.x, by.x, bz.x), cull) ? t0 : kMiss;
+        tn[2 * h + 1] = t1 <= fminf(min3(bx.y, by.y, bz.y), cull) ? t1 : kMiss;
+    }
+}
+
+// The operands of an 8-wide node: header, child codes, and the near / far plane
+// bytes of slots 0-3 (.x) and 4-7 (.y) for the ray's octant.
+struct Node8 {
+    v3 o2, s;
+    uint32_t valid;
+    int32_t ch[8];
+    uint2 nx, fx, ny, fy, nz, fz;
+};
+__device__ __forceinline__ Node8 load8(const QNode8* __restrict__ node, uint32_t flags) {
+    const char* p = reinterpret_cast<const char*>(node);
+    const Words8 A = ldg256(p), B = ldg256(p + 32), C = ldg256(p + 64);
+    Node8 n;
+    n.o2 = mk(__uint_as_float(A.w[0]), __uint_as_float(A.w[1]), __uint_as_float(A.w[2]));
+    const uint32_t meta = A.w[3];
+    n.s = mk(__uint_as_float((meta & 0xffu) << 23), __uint_as_float(((meta >> 8) & 0xffu) << 23),
+             __uint_as_float(((meta >> 16) & 0xffu) << 23));
+    n.valid = meta >> 24;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { n.ch[i] = int32_t(A.w[4 + i]); n.ch[4 + i] = int32_t(B.w[i]); }
+    const bool gx = flags & 1u, gy = flags & 2u, gz = flags & 4u;
+    const uint2 lx = make_uint2(B.w[4], B.w[5]), hx = make_uint2(B.w[6], B.w[7]);
+    const uint2 ly = make_uint2(C.w[0], C.w[1]), hy = make_uint2(C.w[2], C.w[3]);
+    const uint2 lz = make_uint2(C.w[4], C.w[5]), hz = make_uint2(C.w[6], C.w[7]);
+    n.nx = gx ? hx : lx; n.fx = gx ? lx : hx;
+    n.ny = gy ? hy : ly; n.fy = gy ? ly : hy;
+    n.nz = gz ? hz : lz; n.fz = gz ? lz : hz;
+    return n;
+}
+
+// Plain visit of an 8-wide node: each plane is dequantised exactly (P = fmaf(2^23
+// + q, s, o2), see QNode8) and then tested exactly as in box4_plain, so the same
+// slack argument holds.  Entry distances of all slots and the mask of the hit ones.
+struct Children8 {
+    float t[8];
+    uint32_t mask;
+};
+__device__ __forceinline__ Children8 box8_plain(const Node8& n, v3 o, v3 inv, float tmin, float best) {
+    Children8 r;
+    r.mask = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         // byte (i & 3) of the word as the float 2^23 + q
         const uint32_t sel = 0x7540u | uint32_t(i & 3);
-        const float nqx = __uint_as_float(__byte_perm(i < 4 ? qnx.x : qnx.y, 0x4B000000u, sel));
-        const float fqx = __uint_as_float(__byte_perm(i < 4 ? qfx.x : qfx.y, 0x4B000000u, sel));
-        const float nqy = __uint_as_float(__byte_perm(i < 4 ? qny.x : qny.y, 0x4B000000u, sel));
-        const float fqy = __uint_as_float(__byte_perm(i < 4 ? qfy.x : qfy.y, 0x4B000000u, sel));
-        const float nqz = __uint_as_float(__byte_perm(i < 4 ? qnz.x : qnz.y, 0x4B000000u, sel));
-        const float fqz = __uint_as_float(__byte_perm(i < 4 ? qfz.x : qfz.y, 0x4B000000u, sel));
-        const float ax = (fmaf(nqx, sx, hd.x) - r.o.x) * r.inv.x;
-        const float bx = (fmaf(fqx, sx, hd.x) - r.o.x) * r.inv.x;
-        const float ay = (fmaf(nqy, sy, hd.y) - r.o.y) * r.inv.y;
-        const float by = (fmaf(fqy, sy, hd.y) - r.o.y) * r.inv.y;
-        const float az = (fmaf(nqz, sz, hd.z) - r.o.z) * r.inv.z;
-        const float bz = (fmaf(fqz, sz, hd.z) - r.o.z) * r.inv.z;
-        float t0 = fmaxf(fmaxf(ax, ay), fmaxf(az, r.tmin));
+        const float nqx = __uint_as_float(__byte_perm(i < 4 ? n.nx.x : n.nx.y, 0x4B000000u, sel));
+        const float fqx = __uint_as_float(__byte_perm(i < 4 ? n.fx.x : n.fx.y, 0x4B000000u, sel));
+        const float nqy = __uint_as_float(__byte_perm(i < 4 ? n.ny.x : n.ny.y, 0x4B000000u, sel));
+        const float fqy = __uint_as_float(__byte_perm(i < 4 ? n.fy.x : n.fy.y, 0x4B000000u, sel));
+        const float nqz = __uint_as_float(__byte_perm(i < 4 ? n.nz.x : n.nz.y, 0x4B000000u, sel));
+        const float fqz = __uint_as_float(__byte_perm(i < 4 ? n.fz.x : n.fz.y, 0x4B000000u, sel));
+        const float ax = (fmaf(nqx, n.s.x, n.o2.x) - o.x) * inv.x, bx = (fmaf(fqx, n.s.x, n.o2.x) - o.x) * inv.x;
+        const float ay = (fmaf(nqy, n.s.y, n.o2.y) - o.y) * inv.y, by = (fmaf(fqy, n.s.y, n.o2.y) - o.y) * inv.y;
+        const float az = (fmaf(nqz, n.s.z, n.o2.z) - o.z) * inv.z, bz = (fmaf(fqz, n.s.z, n.o2.z) - o.z) * inv.z;
+        const float t0 = fmaxf(fmaxf(ax, ay), fmaxf(az, tmin));
         float t1 = fminf(fminf(bx, by), fminf(bz, best));
         t1 = fmaf(fabsf(t1), kBoxSlack, t1);
-        tn[i] = t0;
-        if (t0 <= t1) mask |= 1u << i;
+        r.t[i] = t0;
+        if (t0 <= t1) r.mask |= 1u << i;
     }
-    return mask & valid;
+    r.mask &= n.valid;
+    return r;
+}
+
+// Packed visit of an 8-wide node: as box4_packed, the byte read as 2^15 + q against
+// the origin moved by (2^23 - 2^15) steps (exact), the intercepts widened by 1/128
+// of a step for the roundings at 2^15 steps.
+__device__ __forceinline__ float2 cut8(float o2, float step, float inv, float slope, float cn, float cf) {
+    const float o = fmaf(8355840.f, step, o2);   // 2^23 - 2^15
+    const float2 c = fma2(o, o, inv, cn, cf);
+    return make_float2(fmaf(fabsf(slope), -0.0078125f, c.x), fmaf(fabsf(slope), 0.0078125f, c.y));
+}
+__device__ __forceinline__ uint32_t box8_packed(const Node8& n, const RayFast& r, float cull, float (&tn)[8]) {
+    const float ix = n.s.x * r.inv.x, iy = n.s.y * r.inv.y, iz = n.s.z * r.inv.z;
+    const float2 cx = cut8(n.o2.x, n.s.x, r.inv.x, ix, r.cn.x, r.cf.x), cy = cut8(n.o2.y, n.s.y, r.inv.y, iy, r.cn.y, r.cf.y);
+    const float2 cz = cut8(n.o2.z, n.s.z, r.inv.z, iz, r.cn.z, r.cf.z);
+    uint32_t mask = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float2 x = slab(i < 4 ? n.nx.x : n.nx.y, i < 4 ? n.fx.x : n.fx.y, i & 3, ix, cx.x, cx.y);
+        const float2 y = slab(i < 4 ? n.ny.x : n.ny.y, i < 4 ? n.fy.x : n.fy.y, i & 3, iy, cy.x, cy.y);
+        const float2 z = slab(i < 4 ? n.nz.x : n.nz.y, i < 4 ? n.fz.x : n.fz.y, i & 3, iz, cz.x, cz.y);
+        tn[i] = fmaxf(max3(x.x, y.x, z.x), r.tmin);
+        if (tn[i] <= fminf(min3(x.y, y.y, z.y), cull)) mask |= 1u << i;
+    }
+    return mask & n.valid;
 }
 
 // Slot permutation s -> s ^ oct applied to an 8-bit mask.
@@ -283,39 +536,53 @@ struct Counters {
 };
 
 // Per-lane traversal state kept across refill points.
-template <bool WT>
+template <bool WT, int WALK>
 struct TravState {
-    Ray r;
+    Ray<WALK> r;
     typename std::conditional<WT, ObjRayWT, ObjRay>::type cache;
     float best, u, v;
-    int prim;
-    int cls;        // material class of the closest hit so far (TriRec e2.w)
+    float cull;     // best with the walk's slack: nothing beyond it matters
+    int prim;       // closest hit so far, its material class (TriRec e2.w) in bits 28-29; -1 = none
     int item;       // current node / leaf code; kNone when the stack must be popped
     int sp;
 };
 constexpr int kNone = 0x7fffffff;   // == kEmptyChild
 
 template <class TS>
-__device__ __forceinline__ void trav_init(TS& s, float4 a, float4 b) {
-    s.r = make_ray(a, b);
-    s.cache.bundle = -2;
-    s.best = s.r.tmax;
+__device__ __forceinline__ float trav_cull(const TS& s, float t) {
+    return fmaf(fabsf(t), (s.r.flags & kPlainWalk) ? kBoxSlack : kFastSlack, t);   // (a constant in the plain walk)
+}
+
+// walk: kPlainWalk to start on the plain nodes, 0 otherwise
+template <class TS>
+__device__ __forceinline__ void trav_init(TS& s, const TraceScene& S, uint32_t walk, float4 a, float4 b, int32_t idx, int root) {
+    make_ray(s.r, S.extent, walk, a, b, idx);
+    keep_ray(S, s.r, a, b);
+    s.cache.bundle = -1;   // world space: the object-space ray of an identity bundle
+    s.cache.o = mk(a.x, a.y, a.z);
+    s.cache.d = mk(b.x, b.y, b.z);
+    shear(s.cache);
+    s.best = b.w;
+    s.cull = trav_cull(s, b.w);
     s.prim = -1;
-    s.cls = 0;
     s.u = s.v = 0.f;
-    s.item = 0;      // root
+    s.item = root;
     s.sp = 0;
+    // A NaN in the origin or direction makes every triangle's t NaN, a miss, and
+    // with all slabs NaN nothing would be culled.
+    if ((s.r.flags & kPlainWalk) && (isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(b.x) || isnan(b.y) || isnan(b.z))) s.item = kNone;
 }
 
 // Runs at most `steps` node / leaf visits.  Returns true when the ray is done.
 // Pops the next stack entry, skipping entries that start beyond the closest
 // hit; false when the stack is empty.
-template <bool ANY, class STACK, class TS>
-__device__ __forceinline__ bool trav_pop(TS& s, const STACK& stack, int& item) {
+template <bool ANY, class STACK, bool WT, int WALK>
+__device__ __forceinline__ bool trav_pop(TravState<WT, WALK>& s, const STACK& stack, int& item) {
     while (s.sp > 0) {
         const int2 e = stack.get(--s.sp);
         // the entry distance carries the box test's rounding: cull with its slack
-        if (!ANY && __int_as_float(e.y) > fmaf(fabsf(s.best), kBoxSlack, s.best)) continue;
+        if (!ANY && __int_as_float(e.y) > s.cull) continue;
+        if (WALK != kWalkFused && e.x == kNone) continue;   // an empty slot (box4_packed, box4_plain)
         item = e.x;
         return true;
     }
@@ -324,18 +591,30 @@ __device__ __forceinline__ bool trav_pop(TS& s, const STACK& stack, int& item) {
 
 // Visits internal node `item`: continues with the nearest hit child (s.item),
 // pushes the others.  False on stack overflow (error flag raised).
-template <bool COUNT, int WIDTH, class STACK, class TS>
-__device__ __forceinline__ bool trav_node(const DevScene& S, TS& s, const STACK& stack, int item,
-                                          Counters& cnt) {
+template <bool ANY, bool COUNT, int WIDTH, class STACK, bool WT, int WALK>
+__device__ __forceinline__ bool trav_node(const TraceScene& S, TravState<WT, WALK>& s, const STACK& stack, int item,
+                                          bool fused, Counters& cnt) {
     if (COUNT) ++cnt.nodes;
+    const bool plain = WALK == kWalkPlain || (s.r.flags & kPlainWalk) != 0;
+    v3 o, d;
     if (WIDTH == 8) {
         float tn[8];
-        int32_t ch[8];
-        const uint32_t mask = box8(S.nodes8, item, s.r, s.best, tn, ch);
+        uint32_t mask;
+        const Node8 n = load8(S.nodes8 + item, s.r.flags);
+        if (plain) {
+            world_ray(S, s.r, o, d);
+            const Children8 c = box8_plain(n, o, s.r.inv, s.r.tmin, s.best);
+            mask = c.mask;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tn[i] = c.t[i];
+        } else if constexpr (WALK != kWalkPlain) {
+            mask = box8_packed(n, s.r, s.cull, tn);
+        }
         if (mask == 0) { s.item = kNone; return true; }
         // visit order i = slot ^ octant: continue with the first hit, push the
         // others so that they pop in visit order
-        const uint32_t om = octant_order(mask, s.r.oct);
+        const uint32_t oct = s.r.flags & kOctMask;
+        const uint32_t om = octant_order(mask, oct);
         const uint32_t rest = om & (om - 1u);
         const int first = __ffs(om) - 1;
         const int nrest = __popc(rest);
@@ -346,45 +625,44 @@ __device__ __forceinline__ bool trav_node(const DevScene& S, TS& s, const STACK&
         int next = kNone;
 #pragma unroll
         for (int sl = 0; sl < 8; ++sl) {
-            const int i = sl ^ int(s.r.oct);
-            if ((rest >> i) & 1u) stack.put(s.sp + __popc(rest >> (i + 1)), make_int2(ch[sl], __float_as_int(tn[sl])));
-            if (i == first) next = ch[sl];
+            const int i = sl ^ int(oct);
+            if ((rest >> i) & 1u) stack.put(s.sp + __popc(rest >> (i + 1)), make_int2(n.ch[sl], __float_as_int(tn[sl])));
+            if (i == first) next = n.ch[sl];
         }
         s.sp += nrest;
         s.item = next;
         return true;
     }
-    float tn[4];
-    int32_t ch[4];
-    const uint32_t mask = box4(S.nodes, item, s.r, s.best, tn, ch);
-    // order the children by entry distance with a 4-input sorting network on
-    // registers (missed children get +inf and sort last)
-    const int nh = __popc(mask);
-    if (nh == 0) { s.item = kNone; return true; }
-    float ht[4];
-    int hc[4];
+    if (plain) {
+        world_ray(S, s.r, o, d);
+        const Children4 h = box4_plain<WALK == kWalkFused>(reinterpret_cast<const float4*>(S.nodes + item), o, s.r.inv, s.r.flags, s.r.tmin, s.best);
+        if (h.nh == 0) { s.item = kNone; return true; }
+        // push the farther ones (farthest first), continue with the nearest
+        if (s.sp + h.nh - 1 > kStackSize) {
+            atomicOr(S.errflags, BG_FLAG_STACK_OVERFLOW);
+            return false;
+        }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        ht[i] = (mask & (1u << i)) ? tn[i] : __int_as_float(0x7f800000);
-        hc[i] = ch[i];
-    }
-    auto cex = [&](int a, int b) {
-        const bool sw = ht[a] > ht[b];
-        const float ta = ht[a], tb = ht[b];
-        const int ca = hc[a], cb = hc[b];
-        ht[a] = sw ? tb : ta; ht[b] = sw ? ta : tb;
-        hc[a] = sw ? cb : ca; hc[b] = sw ? ca : cb;
-    };
-    cex(0, 1); cex(2, 3); cex(0, 2); cex(1, 3); cex(1, 2);
-    // push the farther ones (farthest first), continue with the nearest
-    if (s.sp + nh - 1 > kStackSize) {
-        atomicOr(S.errflags, BG_FLAG_STACK_OVERFLOW);
-        return false;
-    }
+        for (int i = 3; i >= 1; --i)
+            if (i < h.nh) stack.put(s.sp++, make_int2(h.c[i], __float_as_int(h.t[i])));
+        s.item = h.c[0];
+    } else if constexpr (WALK != kWalkPlain) {
+        float tn[4];
+        int32_t ch[4];
+        if (WALK == kWalkFused || fused) box4_fused(S.nodes, item, s.r, s.cull, tn, ch);
+        else box4_packed(S.qnodes, item, s.r, s.cull, tn, ch);
+        sort4<!ANY>(tn, ch);
+        // (the commit has checked that no walk needs more than kStackSize entries; the packed
+        // boxes can only let in an empty slot besides)
+        if (s.sp + 3 > kStackSize) {
+            s.r.flags |= kNearTie;   // no room to spare: the plain walk decides
+            return false;
+        }
 #pragma unroll
-    for (int i = 3; i >= 1; --i)
-        if (i < nh) stack.put(s.sp++, make_int2(hc[i], __float_as_int(ht[i])));
-    s.item = hc[0];
+        for (int i = 3; i >= 1; --i)
+            if (tn[i] < kMiss) stack.put(s.sp++, make_int2(ch[i], __float_as_int(tn[i])));
+        s.item = tn[0] < kMiss ? ch[0] : kNone;
+    }
     return true;
 }
 
@@ -396,8 +674,8 @@ __device__ __forceinline__ bool trav_node(const DevScene& S, TS& s, const STACK&
 // incoherent closest hits +4 %, any hits +3.5 %, C3 frame +1-2 %).
 // WT: the scene's records hold the vertices (p1, p2, p3) and the test is the
 // watertight one; otherwise they hold (p1, e1, e2) for Moller-Trumbore.
-template <bool ANY, bool COUNT, bool WT>
-__device__ __forceinline__ bool trav_leaf(const DevScene& S, TravState<WT>& s, int item, Counters& cnt) {
+template <bool ANY, bool COUNT, bool WT, int WALK>
+__device__ __forceinline__ bool trav_leaf(const TraceScene& S, TravState<WT, WALK>& s, int item, Counters& cnt) {
     const uint32_t code = uint32_t(item);
     const int count = int((code >> kLeafStartBits) & 15u) + 1;
     const int start = int(code & uint32_t(kMaxLeafStart));
@@ -407,35 +685,45 @@ __device__ __forceinline__ bool trav_leaf(const DevScene& S, TravState<WT>& s, i
     float4 v0 = __ldg(tp), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
     if (COUNT) ++cnt.tris;
     obj_ray(S, s.r, __float_as_int(v0.w), s.cache);
+    // packed walk: a hit just beyond the closest one is found too (near tie)
+    const bool margin = WALK != kWalkPlain && !ANY && s.prim >= 0 && !(s.r.flags & kPlainWalk);
+    const float tmax = margin ? s.cull : s.best;
     float t, a, b;
     bool hit;
     if constexpr (WT)
-        hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin,
-                      ANY ? s.r.tmax : s.best, t, a, b);
+        hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin, tmax, t, a, b);
     else
         hit = mt_test(s.cache.o, s.cache.d, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z),
-                      s.r.tmin, ANY ? s.r.tmax : s.best, t, a, b);
+                      s.r.tmin, tmax, t, a, b);
     if (hit) {
-        s.prim = __float_as_int(e1.w);
+        if (margin) {
+            // near the hit it replaces (or is replaced by): a tie; clearly closer: none any more
+            if (t < fmaf(fabsf(s.best), -kFastSlack, s.best)) s.r.flags &= ~kNearTie;
+            else s.r.flags |= kNearTie;
+            if (t > s.best) return false;
+        }
+        s.prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
         if (ANY) return true;
         s.best = t; s.u = a; s.v = b;
-        s.cls = __float_as_int(e2.w);
+        s.cull = trav_cull(s, t);
     }
     return false;
 }
 
 // Runs at most `steps` node / leaf visits.  Returns true when the ray is done.
+// fused (kWalkPacked on 4-wide nodes, the same in all lanes of the warp): visit the
+// 128-byte nodes instead of the packed ones.
 // (Measured and rejected: node and leaf visits in two warp-wide phases,
 // with or without postponing a lane's leaf while others still descend: the
 // votes and the longer loops cost 2.5-4x on C2 and C3.)
-template <bool ANY, bool COUNT, int WIDTH, class STACK, bool WT>
-__device__ __forceinline__ bool trav_steps(const DevScene& S, TravState<WT>& s, const STACK& stack, int steps,
-                                           Counters& cnt) {
+template <bool ANY, bool COUNT, int WIDTH, class STACK, bool WT, int WALK>
+__device__ __forceinline__ bool trav_steps(const TraceScene& S, TravState<WT, WALK>& s, const STACK& stack, int steps,
+                                           bool fused, Counters& cnt) {
     for (int it = 0; it < steps; ++it) {
         int item = s.item;
         if (item == kNone && !trav_pop<ANY>(s, stack, item)) return true;
         if (item >= 0) {
-            if (!trav_node<COUNT, WIDTH>(S, s, stack, item, cnt)) return true;
+            if (!trav_node<ANY, COUNT, WIDTH>(S, s, stack, item, fused, cnt)) return true;
         } else {
             if (trav_leaf<ANY, COUNT>(S, s, item, cnt)) return true;
         }
