@@ -212,6 +212,47 @@ k_trace(DevScene scene, const float4* __restrict__ rays, int64_t n_static, const
     }
 }
 
+// Few rays: a group of lanes walks each (coop_walk), rays dealt out in order.
+// A kernel of its own: the walk needs more registers than k_trace has at 32
+// warps per SM, and the groups that matter are too few to need that many.
+constexpr int kCoopThreads = 128, kCoopBlocks = 5;   // blocks per SM
+template <bool ANY, bool WT>
+__global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
+k_trace_coop(DevScene scene, const float4* __restrict__ rays, int n_static, const int* __restrict__ n_dev,
+             bg_hit* __restrict__ hits, uint8_t* __restrict__ occ, const int* __restrict__ roots, ShadowResolve res,
+             int warps, volatile unsigned* err_out) {
+    // err_out (optional, host memory): receives the scene's error word
+    __shared__ int2 sstack[8][kCoopThreads];
+    int2 lstack[kStackSize - 8];
+    TraceScene S;
+    static_cast<DevScene&>(S) = scene;
+    S.rays = rays;
+    const int n = n_dev ? *n_dev : n_static;
+    const int G = max(8, coop_group(n, warps));
+    const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5), per = 32 / G, base = lane & ~(G - 1);
+    const int step = int(gridDim.x) * (kCoopThreads / 32) * per;
+    for (int first = (int(blockIdx.x) * (kCoopThreads / 32) + warp) * per; first < n; first += step) {
+        const int idx = first + lane / G;
+        const bool live = idx < n;
+        const int root = live && roots ? __ldg(roots + idx) : 0;
+        const CoopHit r = coop_walk<ANY, WT>(S, live, idx, root, G, lane & (G - 1), base, &sstack[0][warp * 32], kCoopThreads);
+        if (r.writer) trace_emit<ANY>(res, hits, occ, idx, r.prim, r.t, r.u, r.v);
+        if (r.redo) {
+            const RayStack<8> stack{&sstack[0][threadIdx.x], lstack, kCoopThreads};
+            TravState<WT, kWalkPlain> s;
+            Counters none{0ull, 0ull, 0ull};
+            trav_init(s, S, kPlainWalk, __ldg(rays + 2 * int64_t(idx)), __ldg(rays + 2 * int64_t(idx) + 1), idx, root);
+            while (!trav_steps<ANY, false, 4>(S, s, stack, 64, false, none)) {}
+            trace_emit<ANY>(res, hits, occ, idx, s.prim, s.best, s.u, s.v);
+        }
+        if (err_out && (idx == 0 || r.redo) && (r.writer || r.redo)) {
+            const unsigned f = *static_cast<volatile unsigned*>(S.errflags);
+            if (f) *err_out = f;
+        }
+        __syncwarp();
+    }
+}
+
 // The walk of a large launch.
 //   casts       packed: L1-bound incoherent rays gain most (coherent / incoherent
 //               closest, incoherent any in Mrays/s, plain before -> packed: soups of
@@ -328,14 +369,31 @@ static void launch_layout(bg_scene* s, bool render, bool any_hit, const float4* 
     else launch_width<4, false>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
 }
 
+// Whether a launch of at most n rays goes to groups of lanes (k_trace_coop).
+static bool groups_walk(const bg_scene* s, int64_t n) {
+    return s->dev.width == 4 && packed_walk<4>(s->dev) && coop_group(n, s->ctx->num_sms * kCoopBlocks * (kCoopThreads / 32)) != 0;
+}
+
 int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                  bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
-                 unsigned long long* work, const int* roots, const ShadowResolve* resolve) {
+                 unsigned long long* work, const int* roots, const ShadowResolve* resolve, int64_t n_most, unsigned* err_out) {
     unsigned long long* w = work ? work : next_work_counter(s);   // the caller's is cleared
     ShadowResolve res{nullptr, nullptr, nullptr, 0};
     if (resolve && !counters) {
         if (any_hit) res = *resolve;
         else res.hit_class = resolve->hit_class;
+    }
+    // at most `n_most` rays, few enough for groups of lanes
+    const int64_t most = n_dev ? n_most : n_static;
+    const int warps = s->ctx->num_sms * kCoopBlocks * (kCoopThreads / 32);
+    if (!counters && most > 0 && groups_walk(s, most)) {
+        const int grid = int(std::min<int64_t>(s->ctx->num_sms * kCoopBlocks, (most * coop_group(most, warps) + kCoopThreads - 1) / kCoopThreads));
+        auto go = [&](auto kernel) { kernel<<<grid, kCoopThreads, 0, st>>>(s->dev, rays, int(n_static), n_dev, hits, occ, roots, res, warps, err_out); };
+        const bool wt = s->dev.watertight != 0;
+        if (any_hit) wt ? go(k_trace_coop<true, true>) : go(k_trace_coop<true, false>);
+        else wt ? go(k_trace_coop<false, true>) : go(k_trace_coop<false, false>);
+        BG_CUDA(cudaGetLastError());
+        return BG_OK;
     }
     if (!work) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
     // ray indices are 32-bit in the kernel: a larger array goes in pieces
@@ -880,6 +938,7 @@ struct CastStage {
     ~CastStage() { release(); }
 };
 constexpr int kStages = 4;
+constexpr int64_t kHostInPlace = 1024;   // rays of a call that the kernel reads from and answers into pinned host memory
 thread_local CastStage t_stage[kStages];
 thread_local uint64_t t_stage_clock = 0;
 }  // namespace
@@ -909,7 +968,6 @@ static int host_cast(bg_scene* s, const bg_ray* rays, void* out, int64_t n, bool
     if (!c->st) BG_CUDA(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
     const size_t rb = size_t(n) * sizeof(bg_ray), ob = size_t(n) * (any ? 1 : sizeof(bg_hit));
     const size_t ob16 = (ob + 15) & ~size_t(15);
-    if ((rc = c->dev.ensure(256 + rb + ob16))) return rc;
     if (c->pinned_bytes < rb + ob16 + 16) {
         if (c->pinned) cudaFreeHost(c->pinned);
         c->pinned = nullptr;
@@ -921,16 +979,27 @@ static int host_cast(bg_scene* s, const bg_ray* rays, void* out, int64_t n, bool
         c->pinned_bytes = want;
     }
     char* hp = static_cast<char*>(c->pinned);
-    char* dp = c->dev.as<char>();
     memcpy(hp, rays, rb);
-    BG_CUDA(cudaMemsetAsync(dp, 0, sizeof(unsigned long long), c->st));
-    BG_CUDA(cudaMemcpyAsync(dp + 256, hp, rb, cudaMemcpyHostToDevice, c->st));
-    rc = launch_trace(s, any, reinterpret_cast<const float4*>(dp + 256), n, nullptr,
-                      any ? nullptr : reinterpret_cast<bg_hit*>(dp + 256 + rb), any ? reinterpret_cast<uint8_t*>(dp + 256 + rb) : nullptr,
-                      c->st, nullptr, 1, reinterpret_cast<unsigned long long*>(dp));
-    if (rc) return rc;
-    BG_CUDA(cudaMemcpyAsync(hp + rb, dp + 256 + rb, ob, cudaMemcpyDeviceToHost, c->st));
-    BG_CUDA(cudaMemcpyAsync(hp + rb + ob16, s->err.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
+    memset(hp + rb + ob16, 0, sizeof(unsigned));
+    if (n <= kHostInPlace && groups_walk(s, n)) {
+        // the kernel reads the rays from the pinned staging and writes the results and
+        // the error word there: one launch and no copies
+        rc = launch_trace(s, any, reinterpret_cast<const float4*>(hp), n, nullptr, any ? nullptr : reinterpret_cast<bg_hit*>(hp + rb),
+                          any ? reinterpret_cast<uint8_t*>(hp + rb) : nullptr, c->st, nullptr, 1, nullptr, nullptr, nullptr, 0,
+                          reinterpret_cast<unsigned*>(hp + rb + ob16));
+        if (rc) return rc;
+    } else {
+        if ((rc = c->dev.ensure(256 + rb + ob16))) return rc;
+        char* dp = c->dev.as<char>();
+        BG_CUDA(cudaMemsetAsync(dp, 0, sizeof(unsigned long long), c->st));
+        BG_CUDA(cudaMemcpyAsync(dp + 256, hp, rb, cudaMemcpyHostToDevice, c->st));
+        rc = launch_trace(s, any, reinterpret_cast<const float4*>(dp + 256), n, nullptr,
+                          any ? nullptr : reinterpret_cast<bg_hit*>(dp + 256 + rb), any ? reinterpret_cast<uint8_t*>(dp + 256 + rb) : nullptr,
+                          c->st, nullptr, 1, reinterpret_cast<unsigned long long*>(dp));
+        if (rc) return rc;
+        BG_CUDA(cudaMemcpyAsync(hp + rb, dp + 256 + rb, ob, cudaMemcpyDeviceToHost, c->st));
+        BG_CUDA(cudaMemcpyAsync(hp + rb + ob16, s->err.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
+    }
     BG_CUDA(cudaStreamSynchronize(c->st));
     memcpy(out, hp + rb, ob);
     unsigned flags = 0;

@@ -185,8 +185,10 @@ struct ShadowResolve {
     int hit_class;
 };
 // work: the launch's work counter, cleared by the caller (null: one of the scene's).
+// n_most: a bound of *n_dev where the caller has one (0 = none).  err_out (launches
+// by groups of lanes only): receives the scene's error word where it is not 0.
 int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                  bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters = nullptr,
                  int stride = 1, unsigned long long* work = nullptr, const int* roots = nullptr,
-                 const ShadowResolve* resolve = nullptr);
+                 const ShadowResolve* resolve = nullptr, int64_t n_most = 0, unsigned* err_out = nullptr);
 }  // namespace bg

@@ -1020,6 +1020,8 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
     PathState P = path_state(rs);
     Queues Q;
     pass_queues(rs, 0, c.batched, Q);
+    // bounds of the queues' lengths (a captured pass serves any number of paths up to cap)
+    const int64_t most = rs->cap, most_sh = most * rs->kmax, most_mis = most * rs->nlights;
     int rc;
     const int depth = std::max(1, c.maxdepth);
     BG_CUDA(cudaMemsetAsync(rs->bounce.ptr, 0, size_t(depth + 1) * sizeof(BounceRec), st));
@@ -1053,7 +1055,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
             if (b >= 2) BG_CUDA(cudaStreamWaitEvent(st, evd[par], 0));   // bounce b - 2's side work is done
             if (b == 0) {
                 if ((rc = launch_trace(s, false, Q.ext_rays_in, 0, Q.n_ext_in, Q.ext_hits, nullptr, st, nullptr, 1, wk,
-                                       Q.ext_root_in, &kExtTrace)))
+                                       Q.ext_root_in, &kExtTrace, most)))
                     return rc;
                 if (ins) { ++ins->launches; ++ins->launches_extend; }
             }
@@ -1065,11 +1067,11 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
             BG_CUDA(cudaStreamWaitEvent(ds, rs->ev_fork, 0));
             const ShadowResolve sr{Q.sh_contrib, Q.sh_slot, P.slots};
             if ((rc = launch_trace(s, true, Q.sh_rays, 0, Q.n_sh, nullptr, nullptr, ds, nullptr, 1, wk + 2, Q.sh_root,
-                                   &sr)))
+                                   &sr, most_sh)))
                 return rc;
             if (s->dev.has_area) {   // MIS rays go to area lights only (the queue is empty otherwise)
                 if ((rc = launch_trace(s, false, Q.mis_rays, 0, Q.n_mis, Q.mis_hits, nullptr, ds, nullptr, 1, wk + 3,
-                                       Q.mis_root)))
+                                       Q.mis_root, nullptr, most_mis)))
                     return rc;
                 k_resolve_mis<<<nb, kShadeThreads, 0, ds>>>(s->dev, P, Q);
                 if (ins) ins->launches += 2;
@@ -1081,7 +1083,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
                 Queues Qn;
                 pass_queues(rs, b + 1, c.batched, Qn, par ^ 1);
                 if ((rc = launch_trace(s, false, Qn.ext_rays_in, 0, Qn.n_ext_in, Qn.ext_hits, nullptr, st, nullptr, 1,
-                                       rs->bounce.as<BounceRec>()[b + 1].work, Qn.ext_root_in, &kExtTrace)))
+                                       rs->bounce.as<BounceRec>()[b + 1].work, Qn.ext_root_in, &kExtTrace, most)))
                     return rc;
                 if (ins) { ++ins->launches; ++ins->launches_extend; }
             }
@@ -1092,7 +1094,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
         unsigned long long* wk = rs->bounce.as<BounceRec>()[b].work;
         if (!fork || b == 0) {
             if (ins) ins->mark(0);
-            if ((rc = launch_trace(s, false, Q.ext_rays_in, 0, Q.n_ext_in, Q.ext_hits, nullptr, st, nullptr, 1, wk, Q.ext_root_in, &kExtTrace))) return rc;
+            if ((rc = launch_trace(s, false, Q.ext_rays_in, 0, Q.n_ext_in, Q.ext_hits, nullptr, st, nullptr, 1, wk, Q.ext_root_in, &kExtTrace, most))) return rc;
             if (ins) { ins->mark(0); ++ins->launches; ++ins->launches_extend; }
         }
         if (ins && ins->count_trav) {
@@ -1117,7 +1119,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
             BG_CUDA(cudaEventRecord(rs->ev_fork, st));
             BG_CUDA(cudaStreamWaitEvent(rs->fstream, rs->ev_fork, 0));
             if ((rc = launch_trace(s, false, Qn.ext_rays_in, 0, Qn.n_ext_in, Qn.ext_hits, nullptr, rs->fstream, nullptr, 1,
-                                   rs->bounce.as<BounceRec>()[b + 1].work, Qn.ext_root_in, &kExtTrace)))
+                                   rs->bounce.as<BounceRec>()[b + 1].work, Qn.ext_root_in, &kExtTrace, most)))
                 return rc;
             BG_CUDA(cudaEventRecord(rs->ev_join, rs->fstream));
             if (ins) { ++ins->launches; ++ins->launches_extend; }
@@ -1127,7 +1129,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
             BG_CUDA(cudaStreamWaitEvent(rs->mstream, rs->ev_fork, 0));
             if (s->dev.has_area) {   // MIS rays go to area lights only (the queue is empty otherwise)
                 if ((rc = launch_trace(s, false, Q.mis_rays, 0, Q.n_mis, Q.mis_hits, nullptr, rs->mstream, nullptr, 1,
-                                       wk + 3, Q.mis_root)))
+                                       wk + 3, Q.mis_root, nullptr, most_mis)))
                     return rc;
                 k_resolve_mis<<<nb, kShadeThreads, 0, rs->mstream>>>(s->dev, P, Q);
             }
@@ -1142,11 +1144,11 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
             BG_CUDA(cudaEventRecord(rs->ev_mjoin, rs->mstream));
         }
         const ShadowResolve sr{Q.sh_contrib, Q.sh_slot, P.slots};   // visible rays land in their slot
-        if ((rc = launch_trace(s, true, Q.sh_rays, 0, Q.n_sh, nullptr, nullptr, st, nullptr, 1, wk + 2, Q.sh_root, &sr)))
+        if ((rc = launch_trace(s, true, Q.sh_rays, 0, Q.n_sh, nullptr, nullptr, st, nullptr, 1, wk + 2, Q.sh_root, &sr, most_sh)))
             return rc;
         if (ins) { ins->mark(1); ins->mark(2); }
         if (!fork && s->dev.has_area &&
-            (rc = launch_trace(s, false, Q.mis_rays, 0, Q.n_mis, Q.mis_hits, nullptr, st, nullptr, 1, wk + 3, Q.mis_root)))
+            (rc = launch_trace(s, false, Q.mis_rays, 0, Q.n_mis, Q.mis_hits, nullptr, st, nullptr, 1, wk + 3, Q.mis_root, nullptr, most_mis)))
             return rc;
         if (ins) { ins->mark(2); ins->launches += s->dev.has_area ? 2 : 1; }
         if (ins && ins->count_trav) {

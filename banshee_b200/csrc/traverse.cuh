@@ -42,8 +42,8 @@ constexpr int kStackSize = 64;     // entries per ray, 4-wide; the builder check
 constexpr int kStackSize8 = 96;    // entries per ray, 8-wide (up to 7 pushes per level)
 // Walks (template parameter WALK): kWalkPlain the plain walk alone; kWalkPacked
 // and kWalkFused the packed arithmetic on QNode4 / QNode8 nodes and on the
-// 128-byte nodes.
-constexpr int kWalkPlain = 0, kWalkPacked = 1, kWalkFused = 3;
+// 128-byte nodes, one ray per lane; kWalkGroup the packed walk by a group of lanes.
+constexpr int kWalkPlain = 0, kWalkPacked = 1, kWalkGroup = 2, kWalkFused = 3;
 
 // stack entries per ray kept in shared memory: 8 for the 4-wide walks, 12 for the
 // packed one (1M-triangle soup, closest / any incoherent: 4 entries 1241 / 1646
@@ -96,6 +96,10 @@ struct RayFast {
 };
 template <int WALK>
 struct Ray : RayFast {};
+template <>
+struct Ray<kWalkGroup> : RayFast {
+    v3 o, d;
+};
 template <>
 struct Ray<kWalkPlain> {
     v3 o, d, inv;
@@ -171,7 +175,9 @@ __device__ __forceinline__ void keep_regs(RAY& r, float4 a, float4 b) {
     r.o = mk(a.x, a.y, a.z);
     r.d = mk(b.x, b.y, b.z);
 }
+__device__ __forceinline__ void keep_ray(const TraceScene&, Ray<kWalkGroup>& r, float4 a, float4 b) { keep_regs(r, a, b); }
 __device__ __forceinline__ void keep_ray(const TraceScene&, Ray<kWalkPlain>& r, float4 a, float4 b) { keep_regs(r, a, b); }
+__device__ __forceinline__ void world_ray(const TraceScene&, const Ray<kWalkGroup>& r, v3& o, v3& d) { o = r.o; d = r.d; }
 __device__ __forceinline__ void world_ray(const TraceScene&, const Ray<kWalkPlain>& r, v3& o, v3& d) { o = r.o; d = r.d; }
 
 // Mesh::IntersectFace (primitive/mesh.cpp:7-45), bit-exact.
@@ -729,6 +735,150 @@ __device__ __forceinline__ bool trav_steps(const TraceScene& S, TravState<WT, WA
         }
     }
     return false;
+}
+
+// ------------------------------------------------- a group of lanes per ray
+// With few rays the time of a launch is the longest ray's chain of dependent
+// visits (about 0.5 us each; a ray of the 1M-triangle soup makes 40, the
+// longest of 4,096 shadow rays 150), whatever the chip could do beside it.  So
+// a group of G = 32 or 8 lanes walks one ray: every step pops up to G entries
+// of the group's stack, each lane visits one of them (a packed node, or a leaf's
+// first triangle), and the lanes push what they found, the nearest lane's
+// children on top.  A step's visits run side by side, so a ray takes about as
+// many steps as the tree has levels; it visits more nodes than the serial walk,
+// as entries are popped before nearer hits have culled them.
+// The answer is that of the packed walk: an any-hit answer and the closest t do
+// not depend on the order, and a closest hit with another one near it, a ray
+// outside the packed arithmetic and a group whose stack runs full (8 entries
+// per lane) are walked again serially on the plain nodes by the group's first
+// lane.
+// (Measured and rejected: four lanes per entry, one per child or triangle: fewer
+// instructions per step, but a quarter of the entries: 4,096 rays 63 us, not 33.)
+// Rays per warp of the grid (2,960 warps on 148 SMs) up to which 32 / 8 lanes walk a
+// ray.  100k-triangle soup, incoherent closest / any, one lane per ray against
+// groups: 256 rays 116 / 90 -> 21 / 22 us, 4,096 127 / 92 -> 32 / 29, 16,384 144 / 100
+// -> 50 / 44, 65,536 169 / 121 -> 131 / 110.  8 lanes at 256 rays 31 / 28, 32 lanes at
+// 16,384 rays 79 / 78.
+constexpr int kCoop32 = 1, kCoop8 = 32;
+
+// Lanes per ray of a launch of n rays on a grid of `warps` warps; 0: too many rays for groups.
+__host__ __device__ __forceinline__ int coop_group(int64_t n, int warps) {
+    return n <= int64_t(warps) * kCoop32 ? 32 : n <= int64_t(warps) * kCoop8 ? 8 : 0;
+}
+
+struct CoopHit {
+    float t, u, v;
+    int prim;       // with the material class in bits 28-29; -1 = none (any hit: >= 0 = occluded)
+    bool writer;    // this lane holds the group's result
+    bool redo;      // (first lane) walk the ray serially
+};
+
+// Lane `g` of the group of G lanes starting at lane `base`; entry j of the group's
+// stack is sm[(j / G) * stride + base + j % G] (sm: the warp's columns).
+// All 32 lanes of the warp call it; `live` = the group has a ray.
+template <bool ANY, bool WT>
+__device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int32_t idx, int root, int G, int g, int base,
+                                             int2* sm, int stride) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const unsigned gmask = G == 32 ? kFull : ((1u << G) - 1u) << base;
+    const unsigned above = gmask & ~((2u << (base + g)) - 1u);   // lanes of the group after this one
+    const int lg = 31 - __clz(G), cap = 8 * G;
+    auto entry = [&](int j) -> int2& { return sm[(j >> lg) * stride + base + (j & (G - 1))]; };
+    TravState<WT, 2> s;
+    if (live) trav_init(s, S, 0u, __ldg(S.rays + 2 * int64_t(idx)), __ldg(S.rays + 2 * int64_t(idx) + 1), idx, root);
+    else trav_init(s, S, 0u, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(1.f, 1.f, 1.f, 0.f), 0, 0);
+    CoopHit r;
+    r.prim = -1;
+    r.t = s.best; r.u = r.v = 0.f;
+    r.redo = live && (s.r.flags & kPlainWalk) != 0;
+    float best = s.best;      // the group's closest t, and the lane that holds it
+    int owner = -1;
+    bool near = false;
+    int count = live && !r.redo ? 1 : 0;
+    if (count && g == 0) entry(0) = make_int2(root, __float_as_int(s.r.tmin));
+    __syncwarp();
+    while (__any_sync(kFull, count > 0)) {
+        // at most (room / 3) entries, as each visit adds up to three
+        const int k = min(min(G, count), (cap - count) / 3);
+        if (count > 0 && k == 0) { r.redo = true; count = 0; }
+        int item = kNone;
+        float entry_t = 0.f;
+        if (count > 0 && g < k) {
+            const int2 e = entry(count - 1 - g);
+            item = e.x;
+            entry_t = __int_as_float(e.y);
+        }
+        if (count > 0) count -= k;
+        const float cull = fmaf(fabsf(best), kFastSlack, best);
+        const float bound = owner >= 0 ? cull : best;   // hits just beyond the closest are found too
+        if (!ANY && entry_t > cull) item = kNone;
+        float ht[4];
+        int hc[4], npush = 0;
+        float t = 0.f, u = 0.f, v = 0.f;
+        int prim = -1;
+        if (item >= 0 && item != kNone) {   // (kNone: none, culled, or an empty slot)
+            box4_packed(S.qnodes, item, s.r, cull, ht, hc);
+            sort4(ht, hc);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) npush += ht[i] < kMiss ? 1 : 0;
+        } else if (item < 0) {
+            const uint32_t code = uint32_t(item);
+            const int start = int(code & uint32_t(kMaxLeafStart)), rest = int((code >> kLeafStartBits) & 15u);
+            // the other triangles of the leaf in up to three entries
+            const int per = (rest + 2) / 3;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const int first = i * per, c = min(per, rest - first);
+                hc[i] = c > 0 ? encode_leaf(start + 1 + first, c) : 0;
+                ht[i] = entry_t;
+                npush += c > 0 ? 1 : 0;
+            }
+            const float4* tp = reinterpret_cast<const float4*>(S.tris + start);
+            const float4 v0 = __ldg(tp), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
+            obj_ray(S, s.r, __float_as_int(v0.w), s.cache);
+            bool hit;
+            if constexpr (WT)
+                hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin, bound, t, u, v);
+            else
+                hit = mt_test(s.cache.o, s.cache.d, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin,
+                              bound, t, u, v);
+            if (hit) prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
+        }
+        const unsigned hits = __ballot_sync(kFull, prim >= 0);
+        if (hits) {
+            if (ANY) {
+                if (hits & gmask) { r.prim = 0; owner = base; count = 0; npush = 0; }
+            } else {
+                float m = prim >= 0 ? t : kMiss;
+                for (int o = G >> 1; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(kFull, m, o));
+                const unsigned close = __ballot_sync(kFull, prim >= 0 && !(t > fmaf(fabsf(m), kFastSlack, m))) & gmask;
+                const unsigned at = __ballot_sync(kFull, prim >= 0 && t == m) & gmask;
+                if (hits & gmask) {
+                    if (owner < 0 || m < best) {
+                        near = (owner >= 0 && !(m < fmaf(fabsf(best), -kFastSlack, best))) || __popc(close) > 1;
+                        best = m;
+                        owner = __ffs(at) - 1;
+                        if (base + g == owner) { r.t = t; r.u = u; r.v = v; r.prim = prim; }
+                    } else {
+                        near = true;
+                    }
+                }
+            }
+        }
+        // pushes: lane 0's children on top, each lane's farthest first
+        const unsigned b0 = __ballot_sync(kFull, npush & 1), b1 = __ballot_sync(kFull, npush & 2), b2 = __ballot_sync(kFull, npush & 4);
+        const int below = count + __popc(b0 & above) + 2 * __popc(b1 & above) + 4 * __popc(b2 & above);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < npush) entry(below + npush - 1 - i) = make_int2(hc[i], __float_as_int(ht[i]));
+        count += __popc(b0 & gmask) + 2 * __popc(b1 & gmask) + 4 * __popc(b2 & gmask);
+        __syncwarp();
+    }
+    if (!ANY && near) r.redo = true;
+    r.writer = live && !r.redo && base + g == (owner >= 0 ? owner : base);
+    r.redo = r.redo && g == 0;
+    return r;
 }
 
 }  // namespace bg
