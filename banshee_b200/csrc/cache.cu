@@ -150,28 +150,43 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* sw, const uint3
 }
 
 // raw query records [n][16] -> encoded bf16 rows [n][128] (the training path;
-// inference encodes inside k_nrc_infer_tc): a pair of lanes per row, each
-// storing its half of the row in 16-byte chunks.
+// inference encodes inside k_nrc_infer_tc).  Eight lanes per row: the pair of lane
+// quarter q encodes levels 4q .. 4q + 3 (encode_level) and one of the four one-blobs,
+// and each lane stores its own words.  A step of 16,384 rows is latency-bound: one
+// lane per row 29.6 us (seven warps per SM), a pair per row 24.9.
 __global__ void __launch_bounds__(128) k_nrc_encode(NrcDev C, const float* __restrict__ feat, const int* n_dev, int64_t n_static,
                                                     int offset, int limit, __nv_bfloat16* __restrict__ X) {
     int64_t n = n_dev ? int64_t(*n_dev) : n_static;
     n = n - offset;
     if (limit > 0 && n > limit) n = limit;
-    const int lane = threadIdx.x & 31, h = lane & 1;
+    const int lane = threadIdx.x & 31, q = (lane >> 1) & 3, h = lane & 1;
     const int64_t warps = int64_t(gridDim.x) * (blockDim.x / 32);
-    for (int64_t w = blockIdx.x * int64_t(blockDim.x / 32) + (threadIdx.x >> 5); w * 16 < n; w += warps) {
-        const int64_t i = w * 16 + (lane >> 1);
-        uint32_t wg[8], wb[16], wt[4];   // a warp stays converged: rows past n repeat the last one
-        encode_pair(C, feat + (size_t(offset) + size_t(i < n ? i : n - 1)) * kNrcFeatFloats, h, wg, wb, wt);
+    for (int64_t w = blockIdx.x * int64_t(blockDim.x / 32) + (threadIdx.x >> 5); w * 4 < n; w += warps) {
+        const int64_t i = w * 4 + (lane >> 3);   // a warp stays converged: rows past n repeat the last one
+        const float4* f = reinterpret_cast<const float4*>(feat + (size_t(offset) + size_t(i < n ? i : n - 1)) * kNrcFeatFloats);
+        const float4 q0 = __ldg(f), q1 = __ldg(f + 1), q2 = __ldg(f + 2), q3 = __ldg(f + 3);
+        const float pos[3] = {q0.x, q0.y, q0.z};
+        float u[3];
+        norm_pos(C, pos, u);
+        uint32_t g[2], b[4];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {   // lane h keeps levels 4q + 2h + k
+            const float lo = encode_level(C, 4 * q + k, u, h), hi = encode_level(C, 4 * q + 2 + k, u, h);
+            const float got = __shfl_xor_sync(0xffffffffu, h ? lo : hi, 1);
+            g[k] = h ? pack_bf16(got, hi) : pack_bf16(lo, got);
+        }
+        float th, ph;
+        if (q < 2) sph(q0.w, q1.x, q1.y, th, ph);
+        else sph(q1.z, q1.w, q2.x, th, ph);
+        one_blob<8>((q & 1) ? ph : th, b, 8 * h);
         if (i >= n) continue;
-        uint4* dst = reinterpret_cast<uint4*>(X + size_t(i) * kNrcIn);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) dst[2 * h + k] = make_uint4(wg[4 * k], wg[4 * k + 1], wg[4 * k + 2], wg[4 * k + 3]);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            dst[4 + 4 * h + k] = make_uint4(wb[4 * k], wb[4 * k + 1], wb[4 * k + 2], wb[4 * k + 3]);
-        dst[12 + h] = h ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(wt[0], wt[1], wt[2], wt[3]);
-        dst[14 + h] = make_uint4(0u, 0u, 0u, 0u);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(X + size_t(i) * kNrcIn);
+        const int c = 2 * q + h;                 // this lane's eighth of the row
+        *reinterpret_cast<uint2*>(dst + 2 * c) = make_uint2(g[0], g[1]);
+        *reinterpret_cast<uint4*>(dst + 16 + 4 * c) = make_uint4(b[0], b[1], b[2], b[3]);
+        *reinterpret_cast<uint2*>(dst + 48 + 2 * c) = c == 0   ? make_uint2(pack_bf16(q2.y, q2.z), pack_bf16(q2.w, q3.x))
+                                                      : c == 1 ? make_uint2(pack_bf16(1.f, 0.f), 0u)
+                                                               : make_uint2(0u, 0u);
     }
 }
 
@@ -347,82 +362,97 @@ __global__ void __launch_bounds__(256) k_nrc_wgrad(const __nv_bfloat16* __restri
     }
 }
 
-// hash-grid backward: scatter dX through the trilinear weights
+// hash-grid backward: scatter dX through the trilinear weights.  One warp per
+// row: lanes 2l and 2l + 1 scatter level l, each its four corners of one x
+// offset, so that an atomic instruction's two lanes of a level meet in one
+// sector (see encode_level).  16,384 rows, 2^19 entries per level: 17.7 us, bound
+// by the L2's atomics; one thread per row (128 blocks, each thread with 128
+// atomics in turn) took 31.  step: when the gradients are applied next, the Adam step
+// count, advanced here for the update that follows on the stream.
 __global__ void __launch_bounds__(128) k_nrc_grid_bwd(NrcDev C, const float* __restrict__ feat, const float* __restrict__ dX,
-                                                      const int* n_dev, int offset, int limit, int Bstatic) {
+                                                      const int* n_dev, int offset, int limit, int Bstatic,
+                                                      int* __restrict__ step) {
+    if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;
     int n = n_dev ? *n_dev - offset : Bstatic;
     if (limit > 0 && n > limit) n = limit;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, l = lane >> 1, h = lane & 1;
+    float* table = C.grid_grad + (size_t(l) << C.log2_T) * 2;
+    const int warps = int(gridDim.x) * (int(blockDim.x) / 32);
+    for (int i = int(blockIdx.x) * (int(blockDim.x) / 32) + int(threadIdx.x >> 5); i < n; i += warps) {
         const float* f = feat + (size_t(offset) + size_t(i)) * kNrcFeatFloats;
-        float fr[3] = {f[0], f[1], f[2]};
+        const float fr[3] = {f[0], f[1], f[2]};
+        const float2 d = *reinterpret_cast<const float2*>(dX + size_t(i) * 32 + 2 * l);
+        if (d.x == 0.f && d.y == 0.f) continue;
         float u[3];
         norm_pos(C, fr, u);
-        for (int l = 0; l < kNrcLevels; ++l) {
-            const float g0 = dX[size_t(i) * 32 + 2 * l], g1 = dX[size_t(i) * 32 + 2 * l + 1];
-            if (g0 == 0.f && g1 == 0.f) continue;
-            GridCorner g = grid_cell(C, l, u);
-#pragma unroll
-            for (int cidx = 0; cidx < 8; ++cidx) {
-                const int dx = cidx & 1, dy = (cidx >> 1) & 1, dz = (cidx >> 2) & 1;
-                const float w = (dx ? g.fx : 1.f - g.fx) * (dy ? g.fy : 1.f - g.fy) * (dz ? g.fz : 1.f - g.fz);
-                const uint32_t idx = grid_index(C, l, g.x0 + dx, g.y0 + dy, g.z0 + dz);
-                float* dst = C.grid_grad + (size_t(l) << C.log2_T) * 2 + size_t(idx) * 2;
-                atomicAdd(reinterpret_cast<float2*>(dst), make_float2(w * g0, w * g1));   // both features, one vector atomic
-            }
-        }
-    }
-}
-
-__global__ void k_nrc_step(int* step) { *step += 1; }
-
-// Adam on fp32 masters; optionally writes a bf16 copy; clears the gradient.
-__global__ void __launch_bounds__(256) k_nrc_adam(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m,
-                                                  float* __restrict__ v, int64_t n, const int* step, float lr, float b1,
-                                                  float b2, float eps, __nv_bfloat16* __restrict__ out) {
-    const int t = *step;
-    const float c1 = 1.f / (1.f - powf(b1, float(t))), c2 = 1.f / (1.f - powf(b2, float(t)));
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float pi = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-        p[i] = pi;
-        g[i] = 0.f;
-        if (out) out[i] = __float2bfloat16_rn(pi);
-    }
-}
-
-// Adam over the hash grid, four parameters per thread.  A quad whose gradient
-// and both moments are zero (table entries no sample has reached yet, among
-// them the unused tails of the densely indexed coarse levels) is left as it
-// is: the update would change none of its values.
-__global__ void __launch_bounds__(256) k_nrc_adam4(float4* __restrict__ p, float4* __restrict__ g,
-                                                   float4* __restrict__ m, float4* __restrict__ v, int64_t n4,
-                                                   const int* step, float lr, float b1, float b2, float eps) {
-    const int t = *step;
-    const float c1 = 1.f / (1.f - powf(b1, float(t))), c2 = 1.f / (1.f - powf(b2, float(t)));
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n4; i += int64_t(gridDim.x) * blockDim.x) {
-        const float4 gi = g[i], mi = m[i], vi = v[i];
-        if (gi.x == 0.f && gi.y == 0.f && gi.z == 0.f && gi.w == 0.f && mi.x == 0.f && mi.y == 0.f && mi.z == 0.f &&
-            mi.w == 0.f && vi.x == 0.f && vi.y == 0.f && vi.z == 0.f && vi.w == 0.f)
-            continue;
-        float4 pi = p[i], mo, vo;
-        const float ga[4] = {gi.x, gi.y, gi.z, gi.w}, ma[4] = {mi.x, mi.y, mi.z, mi.w}, va[4] = {vi.x, vi.y, vi.z, vi.w};
-        float pa[4] = {pi.x, pi.y, pi.z, pi.w}, mn[4], vn[4];
+        const GridCorner g = grid_cell(C, l, u);
+        const float wx = h ? g.fx : 1.f - g.fx;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            mn[k] = b1 * ma[k] + (1.f - b1) * ga[k];
-            vn[k] = b2 * va[k] + (1.f - b2) * ga[k] * ga[k];
-            pa[k] = pa[k] - lr * (mn[k] * c1) / (sqrtf(vn[k] * c2) + eps);
+            const float w = wx * ((k & 1) ? g.fy : 1.f - g.fy) * ((k >> 1) ? g.fz : 1.f - g.fz);
+            const uint32_t idx = grid_index(C, l, g.x0 + h, g.y0 + (k & 1), g.z0 + (k >> 1));
+            atomicAdd(reinterpret_cast<float2*>(table + size_t(idx) * 2), make_float2(w * d.x, w * d.y));   // both features, one vector atomic
         }
-        mo = make_float4(mn[0], mn[1], mn[2], mn[3]);
-        vo = make_float4(vn[0], vn[1], vn[2], vn[3]);
-        m[i] = mo;
-        v[i] = vo;
-        p[i] = make_float4(pa[0], pa[1], pa[2], pa[3]);
-        g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+// One Adam update of four parameters of an fp32 master; clears the gradient.
+// A quad whose gradient and both moments are zero (table entries no sample has
+// reached yet, among them the unused tails of the densely indexed coarse
+// levels) is left as it is: the update would change none of its values.
+struct AdamCoef {
+    float lr, b1, b2, eps, c1, c2;
+};
+struct AdamQuad {
+    float4 p, g, m, v;
+};
+__device__ __forceinline__ bool any4(float4 a) { return a.x != 0.f || a.y != 0.f || a.z != 0.f || a.w != 0.f; }
+__device__ __forceinline__ AdamQuad adam_load(const float4* p, const float4* g, const float4* m, const float4* v, int64_t i) {
+    return AdamQuad{p[i], g[i], m[i], v[i]};
+}
+__device__ __forceinline__ bool adam_quad(const AdamCoef& A, AdamQuad& q, float4* __restrict__ p, float4* __restrict__ g,
+                                          float4* __restrict__ m, float4* __restrict__ v, int64_t i) {
+    if (!any4(q.g) && !any4(q.m) && !any4(q.v)) return false;
+    const float ga[4] = {q.g.x, q.g.y, q.g.z, q.g.w}, ma[4] = {q.m.x, q.m.y, q.m.z, q.m.w}, va[4] = {q.v.x, q.v.y, q.v.z, q.v.w};
+    float pa[4] = {q.p.x, q.p.y, q.p.z, q.p.w}, mn[4], vn[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        mn[k] = A.b1 * ma[k] + (1.f - A.b1) * ga[k];
+        vn[k] = A.b2 * va[k] + (1.f - A.b2) * ga[k] * ga[k];
+        pa[k] = pa[k] - A.lr * (mn[k] * A.c1) / (sqrtf(vn[k] * A.c2) + A.eps);
+    }
+    m[i] = make_float4(mn[0], mn[1], mn[2], mn[3]);
+    v[i] = make_float4(vn[0], vn[1], vn[2], vn[3]);
+    q.p = make_float4(pa[0], pa[1], pa[2], pa[3]);
+    p[i] = q.p;
+    if (any4(q.g)) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return true;
+}
+
+// Adam over the hash grid (grid4 quads) and the network (with its bf16 copy) in one
+// launch.  Bound by HBM: a step whose moments are all set reads 16 and writes 12
+// bytes per parameter.  Each thread has two quads' sixteen-byte loads in flight.
+// 2^19 entries per level, the moments partly set: 79 us as three launches (the
+// step count, grid and network), 69 in one with one quad per turn.
+__global__ void __launch_bounds__(256) k_nrc_adam(NrcDev C, int64_t grid4) {
+    const int t = *C.step;
+    const AdamCoef A{C.lr, C.beta1, C.beta2, C.eps, 1.f / (1.f - powf(C.beta1, float(t))), 1.f / (1.f - powf(C.beta2, float(t)))};
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x, first = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    float4 *w = reinterpret_cast<float4*>(C.w), *wg = reinterpret_cast<float4*>(C.w_grad), *wm = reinterpret_cast<float4*>(C.w_m),
+           *wv = reinterpret_cast<float4*>(C.w_v);
+    for (int64_t i = first; i < kNrcParams / 4; i += stride) {
+        AdamQuad q = adam_load(w, wg, wm, wv, i);
+        if (adam_quad(A, q, w, wg, wm, wv, i))
+            reinterpret_cast<uint2*>(C.wb)[i] = make_uint2(pack2(q.p.x, q.p.y), pack2(q.p.z, q.p.w));
+    }
+    float4 *p = reinterpret_cast<float4*>(C.grid), *g = reinterpret_cast<float4*>(C.grid_grad),
+           *m = reinterpret_cast<float4*>(C.grid_m), *v = reinterpret_cast<float4*>(C.grid_v);
+    for (int64_t i = first; i < grid4; i += 2 * stride) {
+        const int64_t j = i + stride;
+        AdamQuad a = adam_load(p, g, m, v, i), b;
+        if (j < grid4) b = adam_load(p, g, m, v, j);
+        adam_quad(A, a, p, g, m, v, i);
+        if (j < grid4) adam_quad(A, b, p, g, m, v, j);
     }
 }
 
@@ -518,7 +548,7 @@ static constexpr int kInferSmem = kFwTotal * 2;
 static constexpr int kTrainSmem = (kFwTotal + kBwTotal) * 2;
 
 int nrc_encode(bg_cache* c, const float* feat, const int* n_dev, int64_t n_static, int offset, int limit, cudaStream_t st) {
-    k_nrc_encode<<<c->sms * 8, 128, 0, st>>>(c->dev, feat, n_dev, n_static, offset, limit, c->X.as<__nv_bfloat16>());
+    k_nrc_encode<<<c->sms * 16, 128, 0, st>>>(c->dev, feat, n_dev, n_static, offset, limit, c->X.as<__nv_bfloat16>());
     BG_CUDA(cudaGetLastError());
     return BG_OK;
 }
@@ -579,25 +609,10 @@ int nrc_train_step(bg_cache* c, const float* feat, const float4* target, const i
                                                     dW + kNrcW1 + (l - 1) * 4096);
         k_nrc_wgrad<16, 64><<<wg, 256, 0, st>>>(T.DZ5, H + 4 * L, n_dev, offset, B, B, dW + kNrcW5);
     }
-    k_nrc_grid_bwd<<<c->sms * 8, 128, 0, st>>>(c->dev, feat, T.dX, n_dev, offset, B, B);
+    k_nrc_grid_bwd<<<c->sms * 16, 128, 0, st>>>(c->dev, feat, T.dX, n_dev, offset, B, B,
+                                                apply ? c->step.as<int>() : nullptr);
+    if (apply) k_nrc_adam<<<c->sms * 8, 256, 0, st>>>(c->dev, grid_params(c) / 4);   // levels of at least 16 entries: whole quads
     BG_CUDA(cudaGetLastError());
-    if (apply) {
-        k_nrc_step<<<1, 1, 0, st>>>(c->step.as<int>());
-        k_nrc_adam<<<c->sms * 4, 256, 0, st>>>(c->w.as<float>(), dW, c->w_m.as<float>(), c->w_v.as<float>(), kNrcParams,
-                                               c->step.as<int>(), c->dev.lr, c->dev.beta1, c->dev.beta2, c->dev.eps,
-                                               c->wb.as<__nv_bfloat16>());
-        const int64_t gp = grid_params(c);
-        if (gp % 4 == 0)
-            k_nrc_adam4<<<c->sms * 8, 256, 0, st>>>(c->grid.as<float4>(), c->grid_grad.as<float4>(),
-                                                    c->grid_m.as<float4>(), c->grid_v.as<float4>(), gp / 4,
-                                                    c->step.as<int>(), c->dev.lr, c->dev.beta1, c->dev.beta2,
-                                                    c->dev.eps);
-        else
-            k_nrc_adam<<<c->sms * 8, 256, 0, st>>>(c->grid.as<float>(), c->grid_grad.as<float>(), c->grid_m.as<float>(),
-                                                   c->grid_v.as<float>(), gp, c->step.as<int>(), c->dev.lr,
-                                                   c->dev.beta1, c->dev.beta2, c->dev.eps, nullptr);
-        BG_CUDA(cudaGetLastError());
-    }
     return BG_OK;
 }
 

@@ -47,12 +47,15 @@ __device__ __forceinline__ void norm_pos(const NrcDev& C, const float* f, float*
     for (int k = 0; k < 3; ++k) u[k] = fminf(fmaxf((f[k] - C.bmin[k]) * C.bscale[k], 0.f), 1.f);
 }
 
-// one-blob encoding of v in [0,1] into 16 bf16 values, packed two per word
-__device__ __forceinline__ void one_blob(float v, uint32_t* w) {
+// one-blob encoding of v in [0,1] into 16 bf16 values, packed two per word: values
+// first .. first + N - 1 of them
+template <int N = 16>
+__device__ __forceinline__ void one_blob(float v, uint32_t* w, int first = 0) {
 #pragma unroll
-    for (int b = 0; b < 16; b += 2) {
+    for (int k = 0; k < N; k += 2) {
+        const int b = first + k;
         const float d0 = v - (b + 0.5f) * (1.f / 16.f), d1 = v - (b + 1.5f) * (1.f / 16.f);
-        w[b / 2] = pack_bf16(__expf(-d0 * d0 * 128.f), __expf(-d1 * d1 * 128.f));
+        w[k / 2] = pack_bf16(__expf(-d0 * d0 * 128.f), __expf(-d1 * d1 * 128.f));
     }
 }
 

@@ -129,6 +129,45 @@ def test_query_row_counts_match_oracle(ctx, n):
     assert (got[:n, 3] == 0).all() and (got[n:] == 7).all()
 
 
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 127, 129, 38_017])
+def test_training_row_counts_match_oracle(ctx, n):
+    """Rows around the encoding's four per warp and a tile's 128, and more rows than
+    either per-row kernel has warps.  Gradients within the other gradient test's
+    bounds; one Adam step from them moves every parameter of a clear gradient by
+    lr * g / (|g| + eps) to 1e-3 of lr, and leaves those of none untouched."""
+    import torch
+    from oracle import nrc_oracle as O
+    lr = 1e-2
+    gs, cache = _cache(ctx, log2t=10, learning_rate=lr)
+    rng = np.random.default_rng(n)
+    mlp0, grid0, _, _ = cache.params()
+    grid0 = (rng.random(grid0.shape).astype(np.float32) - 0.5) * 0.5
+    cache.set_params(mlp0, grid0)
+    feat = _features(n, rng)
+    target = np.zeros((n, 4), np.float32)
+    target[:, :3] = rng.random((n, 3)) * 2
+    fd, td = torch.from_numpy(feat).cuda(), torch.from_numpy(target).cuda()
+    cache.train(fd.data_ptr(), td.data_ptr(), n, apply=False)
+    mlp, g, dmlp, dgrid = cache.params()
+    res, log2t, bmin, bscale = _oracle_args(cache)
+    _, ref_dmlp, ref_dgrid, _ = O.loss_and_grads(feat.astype(np.float64), target.astype(np.float64), mlp, g,
+                                                 res, log2t, bmin, bscale)
+    for a, b in [(dmlp[O.W_OFFS[k]:O.W_OFFS[k + 1]], ref_dmlp[O.W_OFFS[k]:O.W_OFFS[k + 1]]) for k in range(6)] + \
+                [(dgrid, ref_dgrid)]:
+        a = a.astype(np.float64)
+        assert a @ b > 0.999 * np.linalg.norm(a) * np.linalg.norm(b)
+        assert np.linalg.norm(a - b) < 2e-2 * np.linalg.norm(b)
+    cache.set_params(mlp0, grid0)
+    cache.train(fd.data_ptr(), td.data_ptr(), n, apply=True)
+    mlp1, grid1, dmlp1, dgrid1 = cache.params()
+    assert not dmlp1.any() and not dgrid1.any()
+    for p0, p1, d in ((mlp0, mlp1, dmlp), (grid0, grid1, dgrid)):
+        clear = np.abs(d) > 1e-3 * np.abs(d).max()
+        assert clear.any()
+        assert np.abs(p1.astype(np.float64) - p0 + lr * np.sign(d))[clear].max() < 1e-3 * lr
+        assert (p1[d == 0] == p0[d == 0]).all()
+
+
 @pytest.mark.parametrize("mlp_kernel", [0, 1], ids=["tcgen05", "mma_sync"])
 def test_adam_training_reduces_loss(ctx, mlp_kernel):
     import torch
