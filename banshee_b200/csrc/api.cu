@@ -46,6 +46,11 @@ bool alloc_charge(size_t bytes) {
     return true;
 }
 
+int64_t alloc_budget() {
+    std::lock_guard<std::mutex> lk(g_alloc_mu);
+    return g_alloc_budget;
+}
+
 int DevBuf::ensure(size_t need) {
     if (need <= bytes && ptr) return BG_OK;
     release();

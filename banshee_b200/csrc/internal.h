@@ -37,6 +37,7 @@ struct MeshHost {
 // Charges an allocation against the library's optional cap (bg_alloc_limit)
 // and counts it; false = refused (report BG_ERR_OOM without calling CUDA).
 bool alloc_charge(size_t bytes);
+int64_t alloc_budget();   // bytes the cap still allows (-1: no cap)
 
 // Device buffer that grows on demand (never shrinks until freed).
 struct DevBuf {

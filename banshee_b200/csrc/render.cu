@@ -865,37 +865,44 @@ static int ensure_tracked(RenderState* rs, DevBuf& b, size_t need) {
     return rc;
 }
 
-static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L) {
+// Allocates the path state and queues of a pass of `cap` paths with L lights each
+// (rs), or with rs null only adds up their bytes.  The shadow / MIS / ended-path
+// queues, DI slots and DI throughput come in two halves (bounce parity) for passes
+// that resolve direct light one bounce late; a scene without area lights has no
+// MIS rays, and only batches keep a root per ray.  At L = 2: 0.81 KB per path with
+// area lights off, 1.21 KB with them.
+static int state_buffers(RenderState* rs, int64_t cap, int L, bool area, bool batched, size_t* total) {
+    RenderState none;
+    RenderState& R = rs ? *rs : none;
+    const size_t C = size_t(cap), M = area ? 2 * C * L : 1, B = batched ? C : 1;
+    const struct { DevBuf* b; size_t bytes; } all[] = {
+        {&R.ext_rays[0], C * 32}, {&R.ext_rays[1], C * 32}, {&R.ext_path[0], C * 4}, {&R.ext_path[1], C * 4},
+        {&R.ext_root[0], B * 4}, {&R.ext_root[1], B * 4}, {&R.ext_hits, C * 16},
+        {&R.sh_rays, 2 * C * 2 * L * 32}, {&R.sh_contrib, 2 * C * 2 * L * 16}, {&R.sh_slot, 2 * C * 2 * L * 4},
+        {&R.sh_root, batched ? 2 * C * 2 * L * 4 : 4},
+        {&R.mis_rays, M * 32}, {&R.mis_a, M * 16}, {&R.mis_b, M * 16}, {&R.mis_c, M * 16}, {&R.mis_hits, M * 16},
+        {&R.mis_root, batched ? M * 4 : 4},
+        {&R.end_path, 2 * C * 4}, {&R.cls, 3 * C * 4}, {&R.counts, 256}, {&R.st_key, C * 8}, {&R.st_cnt, C * 4},
+        {&R.st_rng, C * 16}, {&R.st_bs, C * 8}, {&R.st_thr, C * 16}, {&R.st_rad, C * 16}, {&R.st_dithr, 2 * C * 16},
+        {&R.st_flags, C * 4}, {&R.slots, 2 * C * 2 * L * 16}, {&R.sample_rad, C * 16},
+        {&R.cnt_out, (C * 2 * L / 64 + 64) * 16}, {&R.bounce, size_t(kMaxBounces + 1) * sizeof(BounceRec)}};
+    size_t sum = 0;
+    for (const auto& x : all) {
+        sum += x.bytes;
+        if (rs)
+            if (int rc = x.b->ensure(x.bytes)) return rc;
+    }
+    if (total) *total = sum;
+    return BG_OK;
+}
+
+static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L, bool batched) {
     rs->cap = cap;
     rs->nlights = L;
     rs->kmax = 2 * L;
-    const size_t C = size_t(cap);
-    int rc;
-    for (int k = 0; k < 2; ++k) {
-        if ((rc = rs->ext_rays[k].ensure(C * 32)) || (rc = rs->ext_path[k].ensure(C * 4)) ||
-            (rc = rs->ext_root[k].ensure(C * 4)))
-            return rc;
-    }
-    // shadow / MIS / ended-path queues, DI slots and DI throughput come in two
-    // halves (bounce parity) for passes that resolve direct light one bounce late
-    if (C * size_t(rs->kmax) * 2 >= (size_t(1) << 31))
-        return set_error(BG_ERR_UNSUPPORTED, "paths per pass x light slots too large (%zu x %d)", C, rs->kmax);
-    if ((rc = rs->ext_hits.ensure(C * 16)) ||
-        (rc = rs->sh_rays.ensure(2 * C * 2 * L * 32)) || (rc = rs->sh_contrib.ensure(2 * C * 2 * L * 16)) ||
-        (rc = rs->sh_slot.ensure(2 * C * 2 * L * 4)) ||
-        (rc = rs->sh_root.ensure(2 * C * 2 * L * 4)) ||
-        (rc = rs->mis_rays.ensure(2 * C * L * 32)) || (rc = rs->mis_a.ensure(2 * C * L * 16)) ||
-        (rc = rs->mis_b.ensure(2 * C * L * 16)) || (rc = rs->mis_c.ensure(2 * C * L * 16)) ||
-        (rc = rs->mis_hits.ensure(2 * C * L * 16)) || (rc = rs->mis_root.ensure(2 * C * L * 4)) ||
-        (rc = rs->end_path.ensure(2 * C * 4)) || (rc = rs->cls.ensure(3 * C * 4)) ||
-        (rc = rs->counts.ensure(256)) ||
-        (rc = rs->st_key.ensure(C * 8)) || (rc = rs->st_cnt.ensure(C * 4)) || (rc = rs->st_rng.ensure(C * 16)) ||
-        (rc = rs->st_bs.ensure(C * 8)) || (rc = rs->st_thr.ensure(C * 16)) || (rc = rs->st_rad.ensure(C * 16)) ||
-        (rc = rs->st_dithr.ensure(2 * C * 16)) || (rc = rs->st_flags.ensure(C * 4)) ||
-        (rc = rs->slots.ensure(2 * C * rs->kmax * 16)) || (rc = rs->sample_rad.ensure(C * 16)) ||
-        (rc = rs->cnt_out.ensure((C * 2 * L / 64 + 64) * 16)) ||
-        (rc = rs->bounce.ensure(size_t(kMaxBounces + 1) * sizeof(BounceRec))))
-        return rc;
+    if (size_t(cap) * size_t(rs->kmax) * 2 >= (size_t(1) << 31))
+        return set_error(BG_ERR_UNSUPPORTED, "paths per pass x light slots too large (%zu x %d)", size_t(cap), rs->kmax);
+    if (int rc = state_buffers(rs, cap, L, s->dev.has_area != 0, batched, nullptr)) return rc;
     int nb = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade<BG_TRACER_AO, false, false>, kShadeThreads, 0);
     rs->blocks = std::max(1, nb) * s->ctx->num_sms;
@@ -919,12 +926,12 @@ static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L) {
 
 // Path state and queues for passes of `cap` paths with up to maxL lights per
 // job; a failed allocation leaves no state behind (the next call starts over).
-static int ensure_state(bg_scene* s, int64_t cap, int maxL) {
+static int ensure_state(bg_scene* s, int64_t cap, int maxL, bool batched) {
     const int L = std::max(1, maxL);
     if (s->render && s->render->cap >= cap && s->render->nlights == L) return BG_OK;
     if (s->render) render_state_free(s->render);
     s->render = new RenderState();
-    const int rc = alloc_state(s, s->render, cap, L);
+    const int rc = alloc_state(s, s->render, cap, L, batched);
     if (rc) {
         render_state_free(s->render);
         s->render = nullptr;
@@ -1327,6 +1334,34 @@ static void plan_passes(const std::vector<JobSpec>& jobs, int64_t cap, std::vect
     pass_begin.push_back(int(segs.size()));
 }
 
+// Paths per pass of a scene that was not autotuned: up to 2^23 where the device's free
+// memory and the allocation cap hold eight times what they need, never below 2^21.  A
+// pass's deep bounces hold few paths and take about the same time whatever its size, so
+// few large passes beat many small ones (ms at 2^21 / 22 / 23 / 24 paths: 6M-triangle 1080p frame of 8 samples
+// 35.8 / 31.5 / 29.5 / 28.5, eight scenes of 4 samples 10.2 / 8.5 / 7.3 / 6.7).
+constexpr int64_t kPassDefault = int64_t(1) << 21, kPassMost = int64_t(1) << 23;
+template <class F>
+static int64_t default_pass(bg_scene* s, int maxL, bool batched, bool capturing, const F& pass_of) {
+    const int64_t most = pass_of(kPassMost);
+    const int L = std::max(1, maxL);
+    if (most <= kPassDefault) return kPassDefault;
+    if (s->render && s->render->nlights == L) {
+        if (s->render->cap >= most) return kPassMost;                            // it is there already
+        if (capturing) return std::max<int64_t>(kPassDefault, s->render->cap);   // no new one while a stream is captured
+    }
+    size_t free_b = 0, all_b = 0, held = 0;
+    if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess) { cudaGetLastError(); return kPassDefault; }
+    if (s->render) state_buffers(nullptr, s->render->cap, s->render->nlights, s->dev.has_area != 0, batched, &held);
+    size_t room = free_b + held;
+    if (const int64_t budget = alloc_budget(); budget >= 0) room = std::min(room, size_t(budget));
+    for (int64_t t = kPassMost; t > kPassDefault; t >>= 1) {
+        size_t need = 0;
+        state_buffers(nullptr, pass_of(t), L, s->dev.has_area != 0, batched, &need);
+        if (need <= room / 8) return t;
+    }
+    return kPassDefault;
+}
+
 int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, const bg_tracer_desc* tr,
                 bg_render_stats* stats, cudaStream_t st, bool batched) {
     if (!s) return set_error(BG_ERR_INVALID_ARG, "scene is NULL");
@@ -1355,12 +1390,25 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
         total_samples += int64_t(J.W) * J.H * J.spp;
         max_job = std::max(max_job, int64_t(J.W) * J.H * std::max(1, J.spp));
     }
-    const int64_t target = s->tune_paths > 0 ? s->tune_paths : (int64_t(1) << 21);   // paths per pass
-    int64_t cap = std::max<int64_t>(1, std::min<int64_t>(target, std::max<int64_t>(total_samples, 1)));
     // at most 2^26 DI slots (2 per light) per pass, which bounds the shadow / MIS
     // queues too (about 16 GB at the bound): scenes with many lights get smaller passes
-    cap = std::max<int64_t>(1, std::min<int64_t>(cap, (int64_t(1) << 26) / (2 * std::max(1, maxL))));
-    int rc = ensure_state(s, cap, maxL);
+    const int64_t slots = std::max<int64_t>(1, (int64_t(1) << 26) / (2 * std::max(1, maxL)));
+    auto pass_of = [&](int64_t target) {
+        return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(target, std::max<int64_t>(total_samples, 1)), slots));
+    };
+    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
+    BG_CUDA(cudaStreamIsCapturing(st, &cap_st));
+    // (a cached render's training paths are picked by their place in the pass: its size stays)
+    int64_t target = s->tune_paths > 0 ? s->tune_paths
+                     : cache            ? kPassDefault
+                                        : default_pass(s, maxL, batched, cap_st != cudaStreamCaptureStatusNone, pass_of);
+    int64_t cap = pass_of(target);
+    int rc = ensure_state(s, cap, maxL, batched);
+    while (rc == BG_ERR_OOM && s->tune_paths == 0 && target > kPassDefault && cap > kPassDefault) {
+        target >>= 1;                        // no room after all
+        cap = pass_of(target);
+        rc = ensure_state(s, cap, maxL, batched);
+    }
     if (rc) return rc;
     RenderState* rs = s->render;   // buffers may be larger than this call's pass size
     const int maxdepth = tr->kind == BG_TRACER_GI ? tr->maxdepth : 1;
@@ -1379,8 +1427,6 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
     // Graph replay unless statistics were asked for or the caller's stream is
     // capturing (cached renders too: the frame's training-path phase is a
     // parameter of the generate node, the rest of the pass is frame-invariant).
-    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
-    BG_CUDA(cudaStreamIsCapturing(st, &cap_st));
     const bool use_graph = !stats && cap_st == cudaStreamCaptureStatusNone;
     cudaStream_t ws = use_graph ? rs->gstream : st;
     if (use_graph) {
@@ -1501,7 +1547,7 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
             for (int i = 0; i < tsteps; ++i)
                 if ((rc = nrc_train_step(cache, feat, target, ntr_prev, i * tbatch, tbatch, true, ts))) return rc;
             // per step: encode, forward + backward, weight gradients (one tcgen05 kernel or six
-            // mma.sync ones), grid backward, step counter, two Adam kernels
+            // mma.sync ones), grid backward, Adam
             ins.launches += 1 + (cd->mlp_kernel == 0 ? 5 : 10) * tsteps;
             ins.mark(4);
             if (side) BG_CUDA(cudaEventRecord(rs->ev_train, ts));
