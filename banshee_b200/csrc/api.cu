@@ -470,14 +470,14 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
         L.type = d.type;
         L.mesh = d.mesh;
         L.face = d.face;
-        L.matidx = -1;
+        L.prim = -1;
         if (d.type == BG_LIGHT_AREA) {
             if (d.mesh < 0 || d.mesh >= nm || d.face < 0 || d.face >= s->meshes[d.mesh].nfaces)
                 return set_error(BG_ERR_INVALID_ARG, "light %zu: mesh/face out of range", li);
             int mi = s->meshes[d.mesh].m[d.face];
             if (mi < 0 || mi >= nmat || s->mats[mi].type != BG_MAT_EMISSIVE)
                 return set_error(BG_ERR_INVALID_ARG, "AreaLight: The material passed is not an emissive one (light %zu)", li);
-            L.matidx = mi;
+            L.prim = int32_t(start[d.mesh]) + d.face;
             for (int k = 0; k < 3; ++k) L.e[k] = s->mats[mi].e[k];
             const MeshHost& mh = s->meshes[d.mesh];
             const int f = d.face;

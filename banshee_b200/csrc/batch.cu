@@ -170,7 +170,7 @@ int bg_batch_commit(bg_batch* b) {
             BG_CUDA(cudaMemcpy(li.data(), s->lights_d.ptr, li.size() * sizeof(LightRec), cudaMemcpyDeviceToHost));
             for (LightRec& r : li) {
                 if (r.mesh >= 0) r.mesh += int32_t(bo);
-                if (r.matidx >= 0) r.matidx += int32_t(mo);
+                if (r.prim >= 0) r.prim += int32_t(to);
             }
             BG_CUDA(cudaMemcpy(M.lights_d.as<LightRec>() + lo, li.data(), li.size() * sizeof(LightRec), cudaMemcpyHostToDevice));
         }

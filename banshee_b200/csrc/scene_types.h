@@ -46,7 +46,8 @@ struct alignas(16) BundleRec {
     int64_t pad2;
 };
 
-struct MatRec {
+// MatRec and LightRec are read as 16-byte words (load_mat, load_light).
+struct alignas(16) MatRec {
     int32_t type;       // BG_MAT_*
     float kd[3];
     float ks[3];
@@ -54,10 +55,12 @@ struct MatRec {
     float a;            // GGX roughness
     float e[3];
 };
+static_assert(sizeof(MatRec) == 48, "MatRec is 48 bytes");
 
-struct LightRec {
+struct alignas(16) LightRec {
     int32_t type;       // BG_LIGHT_*
-    int32_t mesh, face, matidx;
+    int32_t mesh, face;
+    int32_t prim;       // area: global id of its face
     float dir[3];       // directional: normalize(d) (light/directional_light.h:44)
     float e[3];         // directional radiance / area: emission of the material
     float env[3];       // environment: scale * pow(texel, 1/gamma), precomputed on the host
@@ -65,6 +68,7 @@ struct LightRec {
     float pdf_obj;      // area: FillSample's 1 / area in object space (mesh.cpp:121)
     float pad;
 };
+static_assert(sizeof(LightRec) == 64, "LightRec is 64 bytes");
 
 // material class of a hit (bits 28-29 of a packed primid): 0 misses / emissive,
 // 1 Lambert, 2 GGX; primids stay below 2^27

@@ -12,12 +12,17 @@
 //                                        environment_light.cpp
 //   map_to_hemisphere / orthovector / PowerHeuristic   math/mathutils.h:214-296
 //
-// The BSDF and light-sampling functions are __noinline__: k_shade calls them
-// from several places, and one shared copy keeps the shading kernel inside the
-// instruction cache (measured: the fully inlined kernel stalled on instruction
-// fetch).  fill_hit, called once, is inlined so that its hit record stays in
-// registers instead of the call frame (measured: +6.7 % frame throughput
-// together with inlining emit_di).
+// The BSDF and light-sampling functions come in two forms.  k_shade, which
+// reads the material of each hit, calls them out of line from several places:
+// one shared copy keeps it inside the instruction cache.  The material-class
+// kernels hold their own class's only, inline; bound by latency at 20 warps per
+// SM, they gain from every instruction and local-memory access less.  GiTracer
+// of the Cornell box, 64 spp, 256 x 256, 5.91 -> 5.06 ms a frame with:
+//   area lights sampled inline, from values (the calls kept the light and half
+//   of the hit in a local-memory frame), and a light's record holding its face;
+//   materials and lights read as 16-byte words;
+//   one hemisphere frame per Lambert hit for all its directions (5.28 without);
+//   sine and cosine of an angle by one call.
 #pragma once
 
 #include "device_common.cuh"
@@ -40,9 +45,11 @@ struct SHit {            // ShapeBundle::Hit (primitive/shapebundle.h:156-176)
 
 __device__ __forceinline__ v3 f4xyz(float4 a) { return mk(a.x, a.y, a.z); }
 
-__device__ __forceinline__ void load_xf(const BundleRec* b, float* m, float* minv) {
+// a bundle's transform or its inverse; by words: 16-byte loads cost this kernel
+// its last registers (GiTracer of the Cornell box: 5.06 -> 5.23 ms a frame)
+__device__ __forceinline__ void load_xf(const float* src, float* m) {
 #pragma unroll
-    for (int k = 0; k < 12; ++k) { m[k] = __ldg(b->m + k); minv[k] = __ldg(b->minv + k); }
+    for (int k = 0; k < 12; ++k) m[k] = __ldg(src + k);
 }
 
 // orthovector, math/mathutils.h:214-227
@@ -71,7 +78,10 @@ __device__ __forceinline__ void fill_hit(const DevScene& S, int prim, float a, f
     const BundleRec* B = S.bundles + h.bundle;
     const bool ident = __ldg(&B->identity) != 0;
     float m[12], mi[12];
-    if (!ident) load_xf(B, m, mi);
+    if (!ident) {          // loaded here, ahead of the arithmetic: where they are used, their latency showed
+        load_xf(B->m, m);
+        load_xf(B->minv, mi);
+    }
     float w0 = 1.f - a - b;
     v3 p = add(add(muls(p1, w0), muls(p2, a)), muls(p3, b));
     h.p = ident ? p : xf_point(m, p);
@@ -97,16 +107,23 @@ __device__ __forceinline__ void fill_hit(const DevScene& S, int prim, float a, f
     h.v = t1y * w0 + t2y * a + t3y * b;
 }
 
-// map_to_hemisphere(n, s, e), math/mathutils.h:230-244
-__device__ __forceinline__ v3 map_to_hemisphere_body(v3 n, float sx, float sy, float e) {
-    v3 u = orthovector(n);
-    v3 v = cross(u, n);
+// map_to_hemisphere(n, s, e), math/mathutils.h:230-244: the frame about n, and a
+// direction in it.  A Lambert hit makes two or more directions in one frame.
+__device__ __forceinline__ void hemisphere_frame(v3 n, v3& u, v3& v) {
+    v = cross(orthovector(n), n);
     u = cross(n, v);
-    float sinpsi = sinf(2 * BG_PI * sx);
-    float cospsi = cosf(2 * BG_PI * sx);
+}
+__device__ __forceinline__ v3 hemisphere_dir(v3 n, v3 u, v3 v, float sx, float sy, float e) {
+    float sinpsi, cospsi;
+    sincosf(2 * BG_PI * sx, &sinpsi, &cospsi);   // the bits of sinf and cosf (every float of sx in [0, 1])
     float costheta = powf(1.f - sy, 1.f / (e + 1.f));
     float sintheta = sqrtf(1.f - costheta * costheta);
     return normalize(add(add(muls(muls(u, sintheta), cospsi), muls(muls(v, sintheta), sinpsi)), muls(n, costheta)));
+}
+__device__ __forceinline__ v3 map_to_hemisphere_body(v3 n, float sx, float sy, float e) {
+    v3 u, v;
+    hemisphere_frame(n, u, v);
+    return hemisphere_dir(n, u, v, sx, sy, e);
 }
 __device__ __noinline__ v3 map_to_hemisphere(v3 n, float sx, float sy, float e) { return map_to_hemisphere_body(n, sx, sy, e); }
 // INL: inline copy (the material-class shading kernels) or the shared out-of-line one
@@ -214,17 +231,21 @@ __device__ __noinline__ float microfacet_pdf(float a, v3 hn, v3 wi, v3 wo) {
     return microfacet_pdf_body(a, hn, wi, wo);
 }
 // Lambert::Sample (bsdf/lambert.h:66-86)
-__device__ __forceinline__ BsdfSample lambert_sample_body(v3 kd, v3 hn, v3 ng, float sx, float sy, v3 wi) {
-    v3 n = dot(wi, ng) >= 0.f ? hn : neg(hn);
+// about n, the normal on wi's side (lambert_side), in its frame (u, v)
+__device__ __forceinline__ v3 lambert_side(v3 hn, v3 ng, v3 wi) { return dot(wi, ng) >= 0.f ? hn : neg(hn); }
+__device__ __forceinline__ BsdfSample lambert_sample_body(v3 kd, v3 n, v3 u, v3 v, float sx, float sy) {
     BsdfSample r;
-    r.wo = map_to_hemisphere_body(n, sx, sy, 1.f);
+    r.wo = hemisphere_dir(n, u, v, sx, sy, 1.f);
     float invpi = 1.f / BG_PI;
     r.pdf = dot(n, r.wo) * invpi;
     r.f = muls(kd, invpi);
     return r;
 }
 __device__ __noinline__ BsdfSample lambert_sample(v3 kd, v3 hn, v3 ng, float sx, float sy, v3 wi) {
-    return lambert_sample_body(kd, hn, ng, sx, sy, wi);
+    const v3 n = lambert_side(hn, ng, wi);
+    v3 u, v;
+    hemisphere_frame(n, u, v);
+    return lambert_sample_body(kd, n, u, v, sx, sy);
 }
 __device__ __forceinline__ v3 lambert_eval(const MatRec& M, const SHit& h, v3 wi, v3 wo) {
     float sameside = dot(wi, h.ng) * dot(wo, h.ng);
@@ -239,21 +260,17 @@ __device__ __forceinline__ float lambert_pdf(const SHit& h, v3 wi, v3 wo) {
     }
     return 0.f;
 }
-__device__ __forceinline__ v3 emissive_le(const MatRec& M, v3 n, v3 wo) {
+__device__ __forceinline__ v3 emissive_le(v3 e, v3 n, v3 wo) {
     float ndotwo = dot(n, wo);
-    if (ndotwo > 0.f) return muls(mk(M.e[0], M.e[1], M.e[2]), ndotwo);
+    if (ndotwo > 0.f) return muls(e, ndotwo);
     return mk(0.f, 0.f, 0.f);
 }
+__device__ __forceinline__ v3 emissive_le(const MatRec& M, v3 n, v3 wo) { return emissive_le(mk(M.e[0], M.e[1], M.e[2]), n, wo); }
 
 __device__ __forceinline__ MatRec load_mat(const DevScene& S, int m) {
-    MatRec r;
-    const MatRec* p = S.mats + m;
-    r.type = __ldg(&p->type);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) { r.kd[k] = __ldg(p->kd + k); r.ks[k] = __ldg(p->ks + k); r.e[k] = __ldg(p->e + k); }
-    r.eta = __ldg(&p->eta);
-    r.a = __ldg(&p->a);
-    return r;
+    const float4* p = reinterpret_cast<const float4*>(S.mats + m);
+    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+    return MatRec{__float_as_int(a.x), {a.y, a.z, a.w}, {b.x, b.y, b.z}, b.w, c.x, {c.y, c.z, c.w}};
 }
 
 // SimpleMaterial / Emissive dispatch (material/simplematerial.h:54-70, emissive.h:55-81)
@@ -262,7 +279,7 @@ __device__ __forceinline__ v3 mat_sample(const MatRec& M, const SHit& h, float s
     if (M.type == BG_MAT_LAMBERT) {
         type = kBsdfReflection | kBsdfDiffuse;
         const v3 kd = mk(M.kd[0], M.kd[1], M.kd[2]);
-        const BsdfSample r = INL ? lambert_sample_body(kd, h.n, h.ng, sx, sy, wi) : lambert_sample(kd, h.n, h.ng, sx, sy, wi);
+        const BsdfSample r = INL ? lambert_sample_body(kd, lambert_side(h.n, h.ng, wi), h.dpdu, h.dpdv, sx, sy) : lambert_sample(kd, h.n, h.ng, sx, sy, wi);
         wo = r.wo;
         pdf = r.pdf;
         return r.f;
@@ -298,61 +315,60 @@ __device__ __forceinline__ float mat_pdf(const MatRec& M, const SHit& h, v3 wi, 
 
 // --------------------------------------------------------------- lights
 __device__ __forceinline__ LightRec load_light(const DevScene& S, int i) {
-    LightRec L;
-    const LightRec* p = S.lights + i;
-    L.type = __ldg(&p->type);
-    L.mesh = __ldg(&p->mesh);
-    L.face = __ldg(&p->face);
-    L.matidx = __ldg(&p->matidx);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) { L.dir[k] = __ldg(p->dir + k); L.e[k] = __ldg(p->e + k); L.env[k] = __ldg(p->env + k); }
-    L.area_world = __ldg(&p->area_world);
-    L.pdf_obj = __ldg(&p->pdf_obj);
-    return L;
+    const float4* p = reinterpret_cast<const float4*>(S.lights + i);
+    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+    return LightRec{__float_as_int(a.x), __float_as_int(a.y), __float_as_int(a.z), __float_as_int(a.w),
+                    {b.x, b.y, b.z}, {b.w, c.x, c.y}, {c.z, c.w, d.x}, d.y, d.z, d.w};
 }
 
 // AreaLight::GetSample (light/arealight.cpp:25-51) with Mesh::GetSampleOnShape /
 // FillSample (primitive/mesh.cpp:99-123,323-336); the area pdf 1/area in object
 // space is precomputed on the host (same float ops).
-__device__ __noinline__ v3 area_getsample(const DevScene& S, const LightRec& L, v3 hp, float ux, float uy, v3& d, float& pdf) {
-    const int prim = int(__ldg(&S.bundles[L.mesh].start)) + L.face;
+struct LightSample {
+    v3 le, d;
+    float pdf;
+};
+__device__ __forceinline__ LightSample area_getsample_body(const DevScene& S, int prim, int mesh, v3 e, float pdf_obj, v3 hp,
+                                                           float ux, float uy) {
     const float4* sr = reinterpret_cast<const float4*>(S.shade + prim);
     float4 ra = __ldg(sr), rb = __ldg(sr + 1), rc = __ldg(sr + 2), rd = __ldg(sr + 3), re = __ldg(sr + 4), rf = __ldg(sr + 5);
     float a = sqrtf(ux) * (1.f - uy);
     float b = sqrtf(ux) * uy;
     float w0 = 1.f - a - b;
-    const BundleRec* B = S.bundles + L.mesh;
-    const bool ident = __ldg(&B->identity) != 0;
-    float m[12], mi[12];
-    if (!ident) load_xf(B, m, mi);
+    const BundleRec* B = S.bundles + mesh;
     v3 sp = add(add(muls(f4xyz(ra), w0), muls(f4xyz(rb), a)), muls(f4xyz(rc), b));
-    if (!ident) sp = xf_point(m, sp);
     v3 sn = add(add(muls(f4xyz(rd), w0), muls(f4xyz(re), a)), muls(f4xyz(rf), b));
-    sn = normalize(ident ? sn : xf_normal(mi, sn));
-    d = sub(sp, hp);
-    if (L.pdf_obj > 0.f && dot(sn, neg(normalize(d))) > 0.f) {
-        pdf = L.pdf_obj;
-        float d2inv = 1.f / sqnorm(d);
-        MatRec M = load_mat(S, L.matidx);
-        return muls(emissive_le(M, sn, neg(normalize(d))), d2inv);
+    if (!__ldg(&B->identity)) {
+        float m[12];
+        load_xf(B->m, m);
+        sp = xf_point(m, sp);
+        load_xf(B->minv, m);
+        sn = xf_normal(m, sn);
     }
-    pdf = 0.f;
-    return mk(0.f, 0.f, 0.f);
+    sn = normalize(sn);
+    const v3 d = sub(sp, hp), nd = neg(normalize(d));
+    if (pdf_obj > 0.f && dot(sn, nd) > 0.f) {
+        float d2inv = 1.f / sqnorm(d);
+        return LightSample{muls(emissive_le(e, sn, nd), d2inv), d, pdf_obj};
+    }
+    return LightSample{mk(0.f, 0.f, 0.f), d, 0.f};
+}
+__device__ __noinline__ LightSample area_getsample(const DevScene& S, int prim, int mesh, v3 e, float pdf_obj, v3 hp, float ux,
+                                                   float uy) {
+    return area_getsample_body(S, prim, mesh, e, pdf_obj, hp, ux, uy);
 }
 
 // AreaLight::GetPdf -> Mesh::GetPdfOnShape (primitive/mesh.cpp:354-378): intersect the
 // light's own triangle from p along w with t in (0.001, 1e5].
-__device__ __noinline__ float area_getpdf(const DevScene& S, const LightRec& L, v3 hp, v3 w) {
-    const int prim = int(__ldg(&S.bundles[L.mesh].start)) + L.face;
+__device__ __forceinline__ float area_getpdf_body(const DevScene& S, int prim, int mesh, float area_world, v3 hp, v3 w) {
     const float4* sr = reinterpret_cast<const float4*>(S.shade + prim);
     float4 ra = __ldg(sr), rb = __ldg(sr + 1), rc = __ldg(sr + 2);
     v3 p1 = f4xyz(ra), p2 = f4xyz(rb), p3 = f4xyz(rc);
-    const BundleRec* B = S.bundles + L.mesh;
+    const BundleRec* B = S.bundles + mesh;
     v3 o = hp, d = w;
     if (!__ldg(&B->identity)) {
         float mi[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) mi[k] = __ldg(B->minv + k);
+        load_xf(B->minv, mi);
         o = xf_point(mi, hp);
         d = xf_vector(mi, w);
     }
@@ -362,9 +378,13 @@ __device__ __noinline__ float area_getpdf(const DevScene& S, const LightRec& L, 
     fill_hit(S, prim, a, b, h);
     if (dot(neg(w), h.n) > 0.f) {
         v3 dd = sub(hp, h.p);
-        return sqnorm(dd) / (dot(normalize(dd), h.n) * L.area_world);
+        return sqnorm(dd) / (dot(normalize(dd), h.n) * area_world);
     }
     return 0.f;
+}
+
+__device__ __noinline__ float area_getpdf(const DevScene& S, int prim, int mesh, float area_world, v3 hp, v3 w) {
+    return area_getpdf_body(S, prim, mesh, area_world, hp, w);
 }
 
 __device__ __forceinline__ bool light_singular(const LightRec& L) { return L.type == BG_LIGHT_DIRECTIONAL; }
@@ -373,7 +393,14 @@ __device__ __forceinline__ bool light_singular(const LightRec& L) { return L.typ
 // area-light code; its lights are directional or environment lights).
 template <bool AREA, bool INL = false>
 __device__ __forceinline__ v3 light_getsample(const DevScene& S, const LightRec& L, const SHit& h, float sx, float sy, v3& d, float& pdf) {
-    if (AREA && L.type == BG_LIGHT_AREA) return area_getsample(S, L, h.p, sx, sy, d, pdf);
+    if (AREA && L.type == BG_LIGHT_AREA) {
+        const v3 e = mk(L.e[0], L.e[1], L.e[2]);
+        const LightSample r = INL ? area_getsample_body(S, L.prim, L.mesh, e, L.pdf_obj, h.p, sx, sy)
+                                  : area_getsample(S, L.prim, L.mesh, e, L.pdf_obj, h.p, sx, sy);
+        d = r.d;
+        pdf = r.pdf;
+        return r.le;
+    }
     if (L.type == BG_LIGHT_DIRECTIONAL) {                       // directional_light.cpp:5-14
         d = muls(neg(mk(L.dir[0], L.dir[1], L.dir[2])), 100000000.f);
         pdf = 1.f;
@@ -385,9 +412,11 @@ __device__ __forceinline__ v3 light_getsample(const DevScene& S, const LightRec&
     d = muls(d, 10000000.f);
     return mk(L.env[0], L.env[1], L.env[2]);
 }
-template <bool AREA>
+template <bool AREA, bool INL = false>
 __device__ __forceinline__ float light_getpdf(const DevScene& S, const LightRec& L, const SHit& h, v3 w) {
-    if (AREA && L.type == BG_LIGHT_AREA) return area_getpdf(S, L, h.p, w);
+    if (AREA && L.type == BG_LIGHT_AREA) 
+        return INL ? area_getpdf_body(S, L.prim, L.mesh, L.area_world, h.p, w)
+                   : area_getpdf(S, L.prim, L.mesh, L.area_world, h.p, w);
     if (L.type == BG_LIGHT_DIRECTIONAL) return 0.f;
     return dot(h.n, normalize(w)) * (1.f / BG_PI);
 }
