@@ -153,7 +153,9 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* sw, const uint3
 // inference encodes inside k_nrc_infer_tc).  Eight lanes per row: the pair of lane
 // quarter q encodes levels 4q .. 4q + 3 (encode_level) and one of the four one-blobs,
 // and each lane stores its own words.  A step of 16,384 rows is latency-bound: one
-// lane per row 29.6 us (seven warps per SM), a pair per row 24.9.
+// lane per row 29.6 us (seven warps per SM), a pair per row 24.9, eight lanes 12.
+// Inside k_nrc_train_tc the same took 28: its shared memory leaves an L1 of some
+// 200 lines, which is how many gathers can then be on their way.
 __global__ void __launch_bounds__(128) k_nrc_encode(NrcDev C, const float* __restrict__ feat, const int* n_dev, int64_t n_static,
                                                     int offset, int limit, __nv_bfloat16* __restrict__ X) {
     int64_t n = n_dev ? int64_t(*n_dev) : n_static;
@@ -362,13 +364,10 @@ __global__ void __launch_bounds__(256) k_nrc_wgrad(const __nv_bfloat16* __restri
     }
 }
 
-// hash-grid backward: scatter dX through the trilinear weights.  One warp per
-// row: lanes 2l and 2l + 1 scatter level l, each its four corners of one x
-// offset, so that an atomic instruction's two lanes of a level meet in one
-// sector (see encode_level).  16,384 rows, 2^19 entries per level: 17.7 us, bound
-// by the L2's atomics; one thread per row (128 blocks, each thread with 128
-// atomics in turn) took 31.  step: when the gradients are applied next, the Adam step
-// count, advanced here for the update that follows on the stream.
+// hash-grid backward of the mma.sync path: scatter dX through the trilinear
+// weights.  One warp per row: lanes 2l and 2l + 1 scatter level l.  step: when the
+// gradients are applied next, the Adam step count, advanced here for the update
+// that follows on the stream.
 __global__ void __launch_bounds__(128) k_nrc_grid_bwd(NrcDev C, const float* __restrict__ feat, const float* __restrict__ dX,
                                                       const int* n_dev, int offset, int limit, int Bstatic,
                                                       int* __restrict__ step) {
@@ -376,7 +375,6 @@ __global__ void __launch_bounds__(128) k_nrc_grid_bwd(NrcDev C, const float* __r
     int n = n_dev ? *n_dev - offset : Bstatic;
     if (limit > 0 && n > limit) n = limit;
     const int lane = threadIdx.x & 31, l = lane >> 1, h = lane & 1;
-    float* table = C.grid_grad + (size_t(l) << C.log2_T) * 2;
     const int warps = int(gridDim.x) * (int(blockDim.x) / 32);
     for (int i = int(blockIdx.x) * (int(blockDim.x) / 32) + int(threadIdx.x >> 5); i < n; i += warps) {
         const float* f = feat + (size_t(offset) + size_t(i)) * kNrcFeatFloats;
@@ -385,14 +383,7 @@ __global__ void __launch_bounds__(128) k_nrc_grid_bwd(NrcDev C, const float* __r
         if (d.x == 0.f && d.y == 0.f) continue;
         float u[3];
         norm_pos(C, fr, u);
-        const GridCorner g = grid_cell(C, l, u);
-        const float wx = h ? g.fx : 1.f - g.fx;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float w = wx * ((k & 1) ? g.fy : 1.f - g.fy) * ((k >> 1) ? g.fz : 1.f - g.fz);
-            const uint32_t idx = grid_index(C, l, g.x0 + h, g.y0 + (k & 1), g.z0 + (k >> 1));
-            atomicAdd(reinterpret_cast<float2*>(table + size_t(idx) * 2), make_float2(w * d.x, w * d.y));   // both features, one vector atomic
-        }
+        scatter_level(C, l, u, h, d.x, d.y);
     }
 }
 
@@ -490,6 +481,8 @@ static std::atomic<uint64_t> g_cache_ids{1};
 // `query_rows` queries at a time.  The tcgen05 inference kernel encodes its
 // queries in shared memory and needs none; the mma.sync path encodes them
 // into X first.  (Sizing everything by the pass, 2^24 paths, took 28.6 GB.)
+// Scratch: encoded rows, and for the mma.sync kernels a training set's activations and
+// gradients (the tcgen05 one keeps those of a tile on the chip).
 static int cache_scratch(bg_cache* c, int64_t train_rows, int64_t query_rows) {
     const int64_t xr = std::max(train_rows, c->desc.mlp_kernel == 0 ? int64_t(0) : query_rows);
     if (train_rows <= c->train_cap && xr <= c->x_cap) return BG_OK;
@@ -500,6 +493,10 @@ static int cache_scratch(bg_cache* c, int64_t train_rows, int64_t query_rows) {
         c->x_cap = xr;
     }
     if (train_rows > c->train_cap) {
+        if (c->desc.mlp_kernel == 0) {
+            c->train_cap = train_rows;
+            return BG_OK;
+        }
         const size_t R = size_t(train_rows);
         if ((rc = c->H.ensure(5 * R * 64 * 2)) || (rc = c->DZ.ensure(5 * R * 64 * 2)) || (rc = c->DZ5.ensure(R * 16 * 2)) ||
             (rc = c->dX.ensure(R * 32 * 4)))
@@ -576,41 +573,35 @@ int nrc_query(bg_cache* c, const float* feat, const int* n_dev, int64_t n_static
 // One Adam step on rows [offset, offset + B) of (feat, target); n from n_dev or B.
 int nrc_train_step(bg_cache* c, const float* feat, const float4* target, const int* n_dev, int offset, int B, bool apply,
                    cudaStream_t st) {
+    int* step = apply ? c->step.as<int>() : nullptr;
     int rc;
     if ((rc = nrc_encode(c, feat, n_dev, B, offset, B, st))) return rc;
-    TrainBufs T;
-    T.X = c->X.as<__nv_bfloat16>();
-    T.target = target + offset;
-    T.H = c->H.as<__nv_bfloat16>();
-    T.DZ = c->DZ.as<__nv_bfloat16>();
-    T.DZ5 = c->DZ5.as<__nv_bfloat16>();
-    T.dX = c->dX.as<float>();
-    T.loss = c->loss.as<float>();
-    T.B = B;
     if (c->desc.mlp_kernel == 0) {
-        TcTrainArgs A{T.X, T.target, T.H, T.DZ, T.DZ5, T.dX, T.loss, T.B};
-        k_nrc_train_tc<<<c->sms * 2, 128, kTtSmem, st>>>(c->dev, A, n_dev, offset, B, c->scene->dev.errflags);
+        TcTrainArgs A{feat, c->X.as<__nv_bfloat16>(), target, c->w_grad.as<float>(), c->loss.as<float>(), step, B};
+        k_nrc_train_tc<<<c->sms, kTtThreads, kTtSmem, st>>>(c->dev, A, n_dev, offset, B, c->scene->dev.errflags);
     } else {
+        TrainBufs T;
+        T.X = c->X.as<__nv_bfloat16>();
+        T.target = target + offset;
+        T.H = c->H.as<__nv_bfloat16>();
+        T.DZ = c->DZ.as<__nv_bfloat16>();
+        T.DZ5 = c->DZ5.as<__nv_bfloat16>();
+        T.dX = c->dX.as<float>();
+        T.loss = c->loss.as<float>();
+        T.B = B;
         k_nrc_train<<<c->sms * 2, 128, kTrainSmem, st>>>(c->dev, T, n_dev, offset, B);
-    }
-    const int wg = c->sms;
-    const __nv_bfloat16* H = c->H.as<__nv_bfloat16>();
-    const __nv_bfloat16* DZ = c->DZ.as<__nv_bfloat16>();
-    float* dW = c->w_grad.as<float>();
-    const size_t L = size_t(B) * 64;
-    if (c->desc.mlp_kernel == 0) {
-        // all six weight gradients in one tcgen05 kernel
-        TcWgradArgs W{T.X, H, DZ, T.DZ5, dW, B};
-        k_nrc_wgrad_tc<<<wg, kWgThreads, kWgSmem, st>>>(c->dev, W, n_dev, offset, B, c->scene->dev.errflags);
-    } else {
+        const int wg = c->sms;
+        const __nv_bfloat16* H = c->H.as<__nv_bfloat16>();
+        const __nv_bfloat16* DZ = c->DZ.as<__nv_bfloat16>();
+        float* dW = c->w_grad.as<float>();
+        const size_t L = size_t(B) * 64;
         k_nrc_wgrad<64, 128><<<wg, 256, 0, st>>>(DZ, T.X, n_dev, offset, B, B, dW + kNrcW0);
         for (int l = 1; l < 5; ++l)
             k_nrc_wgrad<64, 64><<<wg, 256, 0, st>>>(DZ + l * L, H + (l - 1) * L, n_dev, offset, B, B,
                                                     dW + kNrcW1 + (l - 1) * 4096);
         k_nrc_wgrad<16, 64><<<wg, 256, 0, st>>>(T.DZ5, H + 4 * L, n_dev, offset, B, B, dW + kNrcW5);
+        k_nrc_grid_bwd<<<c->sms * 16, 128, 0, st>>>(c->dev, feat, T.dX, n_dev, offset, B, B, step);
     }
-    k_nrc_grid_bwd<<<c->sms * 16, 128, 0, st>>>(c->dev, feat, T.dX, n_dev, offset, B, B,
-                                                apply ? c->step.as<int>() : nullptr);
     if (apply) k_nrc_adam<<<c->sms * 8, 256, 0, st>>>(c->dev, grid_params(c) / 4);   // levels of at least 16 entries: whole quads
     BG_CUDA(cudaGetLastError());
     return BG_OK;
@@ -736,7 +727,6 @@ int bg_cache_create(bg_scene* s, const bg_cache_desc* d, bg_cache** out) {
     cudaFuncSetAttribute(k_nrc_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem);
     cudaFuncSetAttribute(k_nrc_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTiSmem);
     cudaFuncSetAttribute(k_nrc_train_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTtSmem);
-    cudaFuncSetAttribute(k_nrc_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
     cudaFuncSetAttribute(k_nrc_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
     if ((rc = cache_init_params(c))) { bg_cache_destroy(c); return rc; }
     // the scratch of one Adam step over train_batch rows, here rather than in

@@ -80,9 +80,7 @@ __device__ __forceinline__ void sph(float x, float y, float z, float& th, float&
 // exchange their corners so that lane h sums feature h of every level over the
 // corners in the order x, y, z of one lane alone: the same sums, bit for bit.
 // Both lanes of a pair must call it, with all 32 lanes of the warp converged.
-// Measured: queries as k_nrc_infer_tc says; the training rows' encoding of a
-// step of 16,384 rows 29.6 us with one lane per row (128 blocks of four warps,
-// each lane's 128 gathers in turn), 22 us with pairs.
+// Measured: queries as k_nrc_infer_tc says, training rows as k_nrc_encode does.
 __device__ __forceinline__ float encode_level(const NrcDev& C, int l, const float* u, int h) {
     const GridCorner g = grid_cell(C, l, u);
     const float2* table = reinterpret_cast<const float2*>(C.grid) + (size_t(l) << C.log2_T);
@@ -123,6 +121,21 @@ __device__ __forceinline__ void encode_pair(const NrcDev& C, const float* __rest
     t[1] = pack_bf16(q2.w, q3.x);
     t[2] = pack_bf16(1.f, 0.f);
     t[3] = 0u;
+}
+
+// Scatters a row's gradient (dx, dy) of level l's features over the table: the
+// four corners of x offset h, so that a pair of lanes covers the cell and meets
+// in one sector (see encode_level).
+__device__ __forceinline__ void scatter_level(const NrcDev& C, int l, const float* u, int h, float dx, float dy) {
+    const GridCorner g = grid_cell(C, l, u);
+    float* table = C.grid_grad + (size_t(l) << C.log2_T) * 2;
+    const float wx = h ? g.fx : 1.f - g.fx;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float w = wx * ((k & 1) ? g.fy : 1.f - g.fy) * ((k >> 1) ? g.fz : 1.f - g.fz);
+        const uint32_t idx = grid_index(C, l, g.x0 + h, g.y0 + (k & 1), g.z0 + (k >> 1));
+        atomicAdd(reinterpret_cast<float2*>(table + size_t(idx) * 2), make_float2(w * dx, w * dy));   // both features, one vector atomic
+    }
 }
 
 }  // namespace bg

@@ -103,6 +103,17 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 8 of them
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 __device__ __forceinline__ uint32_t tc_pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -279,53 +290,90 @@ __global__ void __launch_bounds__(kTiThreads, kTiCtasPerSm) k_nrc_infer_tc(NrcDe
 
 
 // ------------------------------------------------------------- training
-// Fused forward + backward of one Adam step's rows on tcgen05, same outputs as
-// the mma.sync k_nrc_train: hidden activations H[l] and layer-output gradients
-// DZ[l] (bf16, for the weight-gradient kernels), DZ5, the hash-grid feature
-// gradient dX (fp32, 32 columns) and the summed relative-L2 loss.
-//
-// The backward products dH = dZ * W need B = W with the layer's input features
-// as N: the forward weight tiles already hold W[out][in] in 8x8 core matrices
-// of 8 rows (out) x 16 contiguous bytes (in), which is exactly an MN-major B
-// core matrix (8 K-rows x 8 contiguous N elements), so the backward reads the
-// same shared memory through MN-major descriptors (SBO = 128 bytes between
+// The gradients of one Adam step's encoded rows in one kernel: forward, loss,
+// backward, the six weight gradients and the hash grid's.  One CTA per SM; a
+// tile of 128 rows stays on the chip from its inputs to its gradients:
+//   X            the encoded rows (k_nrc_encode), K-major, 16 chunks per row
+//   P1, P2, P3   the hidden activations [H0 | H1], [H2 | H3], [H4 | 0], laid out as X
+//   dZ           two buffers for the layer-output gradients, by the layer's parity
+//   dZ5          the output layer's
+// Forward: H_l = relu(A_l W_l) with A_0 = X, A_l = H_{l-1}.  Backward products
+// dH = dZ W need B = W with the layer's inputs as N: the forward weight tiles hold
+// W[out][in] in 8x8 core matrices of 8 rows (out) x 16 contiguous bytes (in), which
+// is exactly an MN-major B core matrix (8 K-rows x 8 contiguous N elements), so
+// the backward reads them through MN-major descriptors (SBO = 128 bytes between
 // groups of 8 inputs, LBO = KC * 128 bytes between groups of 8 outputs).
-// Each thread keeps its row's ReLU masks (64 bits per hidden layer) in registers.
-constexpr int kTtA0 = kTcA0;                 // input tile; reused for the dZ5 tile after layer 0
-constexpr int kTtSmem = kTcSmem;
+// Weight gradients dW_l[o][i] = sum_s A_l[s][i] dZ_l[s][o] have the rows as K:
+// both tiles read as MN-major operands (LBO = the stride between groups of 8
+// rows, SBO = 128 bytes between groups of 8 features).  Every product has M =
+// 128: the two layers of a P tile are multiplied by each one's dZ in turn, and
+// the half of the lanes that belongs to the other layer is not used.  They are
+// issued behind the backward product that the chain waits for, accumulate in
+// TMEM over the CTA's tiles (cols 64 + 64 l for layer l, transposed, D[i][o]),
+// and are added to global memory once per CTA.
+// Threads: warp w reads TMEM lanes 32 (w % 4) .. + 31 (lane = tile row), 16
+// columns (w / 4) .. of the 64; each keeps its ReLU masks in registers.  A step of
+// 16,384 rows is one tile per SM and a chain of twelve dependent products, so
+// it is bound by latency: 4 us of weights and TMEM, 9 of the chain, 11 of the
+// scatter's atomics (L2), 4 of the weight gradients' atomics.
+// Forward and backward, weight gradients and scatter as kernels of their own,
+// with the activations and gradients through global memory, took 25 + 19 + 17
+// us at 16,384 rows and 2^19 entries per level; this one takes 35.
+constexpr int kTtThreads = 512;
+constexpr int kTtX = kTcA0;                                // X, P1, P2, P3
+constexpr int kTtTile = kTcRows * 128 * 2;
+constexpr int kTtDz = kTtX + 4 * kTtTile;                  // two of [128 x 64]
+constexpr int kTtDzB = kTcRows * 64 * 2;
+constexpr int kTtDz5 = kTtDz + 2 * kTtDzB;                 // [128 x 16]
+constexpr int kTtBar = kTtDz5 + kTcRows * 16 * 2;          // mbarrier (8 B) + TMEM base (4 B)
+constexpr int kTtSmem = kTtBar + 16;
+constexpr uint32_t kTtCols = 512;                          // TMEM columns: accumulator 0-63, weight gradients 64-399
+static_assert(kTtSmem <= 227 * 1024, "training shared memory");
 
 struct TcTrainArgs {
-    const __nv_bfloat16* X;      // encoded inputs of this step's rows [B][128]
-    const float4* target;        // this step's targets [B] (already offset)
-    __nv_bfloat16* H;            // [5][B][64]
-    __nv_bfloat16* DZ;           // [5][B][64]
-    __nv_bfloat16* DZ5;          // [B][16]
-    float* dX;                   // [B][32]
+    const float* feat;           // raw records of the whole set; this step's rows start at `offset`
+    const __nv_bfloat16* X;      // encoded rows of this step [B][128]
+    const float4* target;        // targets of the whole set
+    float* dW;                   // [kNrcParams], accumulated
     float* loss;
+    int* step;                   // Adam's step count, advanced for the update that follows (null: none follows)
     int B;
 };
 
-__global__ void __launch_bounds__(128, 2) k_nrc_train_tc(NrcDev C, TcTrainArgs T, const int* n_dev, int offset,
-                                                         int limit, unsigned* __restrict__ errflags) {
+__global__ void __launch_bounds__(kTtThreads, 1) k_nrc_train_tc(NrcDev C, TcTrainArgs T, const int* n_dev, int offset,
+                                                                int limit, unsigned* __restrict__ errflags) {
     extern __shared__ __align__(1024) unsigned char tt_smem[];
     unsigned char* smem = tt_smem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = (warp & 3) * 32 + lane, cg = warp >> 2;   // TMEM lane, group of 16 columns
     const uint32_t sbase = uint32_t(__cvta_generic_to_shared(smem));
-    const uint32_t bar = sbase + kTcBar;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kTcBar + 8);
-    __shared__ int abort_flag;
+    const uint32_t bar = sbase + kTtBar;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kTtBar + 8);
+    // set by a wait that gave up, one flag per mbarrier parity: a thread already in the
+    // next wait must not change the flag that others still read for this one
+    __shared__ int abort_flag[2];
+
+    if (T.step && blockIdx.x == 0 && tid == 0) *T.step += 1;
+    int n = n_dev ? *n_dev - offset : T.B;
+    if (limit > 0 && n > limit) n = limit;
+    if (n < 0) n = 0;
+    const int ntiles = (n + kTcRows - 1) / kTcRows;
+    if (int(blockIdx.x) >= ntiles) return;   // (uniform per CTA, before any TMEM allocation)
+    const float invn = 1.f / (3.f * float(n));
 
     tc_load_weights(C.wb + kNrcW0, 64, 128, smem + kTcW0);
     for (int l = 0; l < 4; ++l) tc_load_weights(C.wb + kNrcW1 + l * 4096, 64, 64, smem + kTcW1 + l * 8192);
     tc_load_weights(C.wb + kNrcW5, 16, 64, smem + kTcW5);
+    for (int v = tid; v < kTcRows * 8; v += kTtThreads)      // the zero half of P3, once
+        *reinterpret_cast<uint4*>(smem + kTtX + 3 * kTtTile + tc_off(v & 127, 8 + (v >> 7), 16)) = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0) {
-        abort_flag = 0;
+        abort_flag[0] = abort_flag[1] = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(sbase + kTcBar + 8), "r"(kTcCols) : "memory");
+                     :: "r"(sbase + kTtBar + 8), "r"(kTtCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_async_smem();
@@ -333,106 +381,98 @@ __global__ void __launch_bounds__(128, 2) k_nrc_train_tc(NrcDev C, TcTrainArgs T
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t trow = tmem + (uint32_t(warp * 32) << 16);
-
-    int n = n_dev ? *n_dev - offset : T.B;
-    if (limit > 0 && n > limit) n = limit;
-    if (n < 0) n = 0;
-    const float invn = n > 0 ? 1.f / (3.f * float(n)) : 0.f;
-    const int ntiles = (n + kTcRows - 1) / kTcRows;
+    const uint32_t trow = tmem + (uint32_t((warp & 3) * 32) << 16);
     uint32_t phase = 0;
     float lsum = 0.f;
+    bool first = true, gave_up = false;
 
-    // one MMA group on the tile in `a` (K-major, KC chunks) with weights at `b`
-    auto run = [&](uint32_t a, int KC, uint32_t b, uint32_t b_lbo, uint32_t b_sbo, uint32_t b_kstep, uint32_t idesc) {
-        if (tid == 0) {
-            tc_fence_after();
-            for (int s = 0; s < KC / 2; ++s)
-                tc_mma(tmem, tc_desc(a + s * 256, 128, KC * 128), tc_desc(b + s * b_kstep, b_lbo, b_sbo), idesc,
-                       s > 0 ? 1u : 0u);
-            tc_commit(bar);
-        }
+    // the chain's next product into columns 0 .. N - 1: the tile at `a` (K-major, a_sbo bytes
+    // between its 8-row groups, K / 16 = steps) by the weights at `b`; thread 0 only
+    auto product = [&](uint32_t a, uint32_t a_sbo, int steps, uint32_t b, uint32_t b_lbo, uint32_t b_sbo, uint32_t b_kstep,
+                       uint32_t idesc) {
+        tc_fence_after();
+        for (int s = 0; s < steps; ++s)
+            tc_mma(tmem, tc_desc(a + s * 256, 128, a_sbo), tc_desc(b + s * b_kstep, b_lbo, b_sbo), idesc, s > 0 ? 1u : 0u);
+        tc_commit(bar);
+    };
+    // a weight gradient into the accumulator at `col`: activations at `a`, dZ at `b` (b_lbo
+    // bytes between its 8-row groups); thread 0 only
+    auto wgrad = [&](uint32_t a, uint32_t b, uint32_t b_lbo, int N, uint32_t col) {
+        const uint32_t idesc = tc_idesc(N, true) | (1u << 15);   // A and B MN-major
+        for (int k = 0; k < kTcRows / 16; ++k)
+            tc_mma(tmem + col, tc_desc(a + k * 2 * 2048, 2048, 128), tc_desc(b + k * 2 * b_lbo, b_lbo, 128), idesc,
+                   (first && k == 0) ? 0u : 1u);
+    };
+    // every thread waits for the last commit; false (in all of them) after a timeout
+    auto wait = [&]() {
         if (!tc_wait(bar, phase, C.wait_polls)) {
             atomicOr(errflags, BG_FLAG_TIMEOUT);
-            abort_flag = 1;
+            abort_flag[phase] = 1;
         }
-        phase ^= 1u;
         tc_fence_after();
         __syncthreads();
-        return abort_flag == 0;
+        gave_up = abort_flag[phase] != 0;
+        phase ^= 1u;
+        return !gave_up;
     };
-    // this thread's accumulator row (64 columns) -> 8 bf16 chunks, optionally masked / rectified
-    auto row64 = [&](uint32_t (&packed)[32], uint32_t (&mask)[2], bool relu, bool apply_mask) {
-#pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
-            float v[16];
-            tc_ld16(trow + uint32_t(c4 * 16), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int col = c4 * 16 + j;
-                if (relu) {
-                    if (v[j] > 0.f) mask[col >> 5] |= 1u << (col & 31);
-                    v[j] = fmaxf(v[j], 0.f);
-                }
-                if (apply_mask && !((mask[col >> 5] >> (col & 31)) & 1u)) v[j] = 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) packed[c4 * 8 + j] = tc_pack(v[2 * j], v[2 * j + 1]);
-        }
-    };
-    auto store_row = [&](const uint32_t (&packed)[32], __nv_bfloat16* g, int64_t grow, bool to_global) {
-        const int r = tid;
-#pragma unroll
-        for (int kc = 0; kc < 8; ++kc) {
-            const uint4 v = make_uint4(packed[4 * kc], packed[4 * kc + 1], packed[4 * kc + 2], packed[4 * kc + 3]);
-            *reinterpret_cast<uint4*>(smem + kTcA1 + tc_off(r, kc, 8)) = v;
-            if (to_global) reinterpret_cast<uint4*>(g + size_t(grow) * 64)[kc] = v;
-        }
-    };
-
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t row0 = int64_t(tile) * kTcRows;
-        const int64_t grow = row0 + tid;
-        const bool live = grow < n;
-        for (int j = 0; j < 16; ++j) {
-            const int u = j * 4 + warp, rg = u >> 2, kq4 = u & 3;
-            const int r = rg * 8 + (lane & 7), kc = kq4 * 4 + (lane >> 3);
-            const int64_t g = row0 + r;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (g < n) v = *reinterpret_cast<const uint4*>(T.X + size_t(g) * kNrcIn + kc * 8);
-            *reinterpret_cast<uint4*>(smem + kTtA0 + tc_off(r, kc, 16)) = v;
-        }
+    // shared memory written, TMEM read: thread 0 may issue the next product
+    auto ready = [&]() {
         tc_fence_async_smem();
         tc_fence_before();
         __syncthreads();
-        uint32_t masks[5][2];
-#pragma unroll
-        for (int l = 0; l < 5; ++l) masks[l][0] = masks[l][1] = 0u;
-        bool ok = true;
+    };
+    auto pack16 = [&](const float (&v)[16], uint4& p0, uint4& p1) {
+        p0 = make_uint4(tc_pack(v[0], v[1]), tc_pack(v[2], v[3]), tc_pack(v[4], v[5]), tc_pack(v[6], v[7]));
+        p1 = make_uint4(tc_pack(v[8], v[9]), tc_pack(v[10], v[11]), tc_pack(v[12], v[13]), tc_pack(v[14], v[15]));
+    };
+    const uint32_t sX = sbase + kTtX, sP = sX + kTtTile, sDz = sbase + kTtDz, sDz5 = sbase + kTtDz5;
+
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int row0 = tile * kTcRows;
+        const bool live = row0 + row < n;
+        // ---- the encoded rows; those past n repeat the last one (their dZ is zero)
+        for (int j = 0; j < 4; ++j) {                        // eight lanes load one core matrix: no bank conflicts
+            const int r = warp * 8 + (lane & 7), kc = j * 4 + (lane >> 3);
+            *reinterpret_cast<uint4*>(smem + kTtX + tc_off(r, kc, 16)) =
+                *reinterpret_cast<const uint4*>(T.X + size_t(min(row0 + r, n - 1)) * kNrcIn + kc * 8);
+        }
+        ready();
+        uint32_t mask[5];
         // ---- forward: hidden layers
 #pragma unroll
-        for (int l = 0; l < 5 && ok; ++l) {
-            ok = l == 0 ? run(sbase + kTtA0, 16, sbase + kTcW0, 128, 16 * 128, 256, tc_idesc(64))
-                        : run(sbase + kTcA1, 8, sbase + kTcW1 + (l - 1) * 8192, 128, 8 * 128, 256, tc_idesc(64));
-            if (!ok) break;
-            uint32_t packed[32];
-            row64(packed, masks[l], true, false);
-            store_row(packed, T.H + size_t(l) * T.B * 64, grow, live);
-            tc_fence_async_smem();
-            tc_fence_before();
-            __syncthreads();
-        }
-        if (!ok) break;
-        // ---- output layer and the loss gradient (columns 0..2 of 16)
-        if (!run(sbase + kTcA1, 8, sbase + kTcW5, 128, 8 * 128, 256, tc_idesc(16))) break;
-        {
+        for (int l = 0; l < 5; ++l) {
+            if (tid == 0) {
+                if (l == 0) product(sX, 2048, 8, sbase + kTcW0, 128, 16 * 128, 256, tc_idesc(64));
+                else product(sP + ((l - 1) >> 1) * kTtTile + ((l - 1) & 1) * 1024, 2048, 4, sbase + kTcW1 + (l - 1) * 8192, 128,
+                             8 * 128, 256, tc_idesc(64));
+            }
+            if (!wait()) break;
             float v[16];
+            tc_ld16(trow + uint32_t(cg * 16), v);
+            mask[l] = 0u;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (v[j] > 0.f) mask[l] |= 1u << j;
+                v[j] = fmaxf(v[j], 0.f);
+            }
+            uint4 p0, p1;
+            pack16(v, p0, p1);
+            unsigned char* dst = smem + kTtX + (1 + (l >> 1)) * kTtTile;
+            *reinterpret_cast<uint4*>(dst + tc_off(row, 8 * (l & 1) + 2 * cg, 16)) = p0;
+            *reinterpret_cast<uint4*>(dst + tc_off(row, 8 * (l & 1) + 2 * cg + 1, 16)) = p1;
+            ready();
+        }
+        if (gave_up) break;
+        // ---- output layer and the loss gradient (columns 0..2 of 16)
+        if (tid == 0) product(sP + 2 * kTtTile, 2048, 4, sbase + kTcW5, 128, 8 * 128, 256, tc_idesc(16));
+        if (!wait()) break;
+        if (cg == 0) {
+            float v[16], g[16];
             tc_ld16(trow, v);
-            float g[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) g[j] = 0.f;
             if (live) {
-                const float* y = reinterpret_cast<const float*>(T.target + grow);
+                const float* y = reinterpret_cast<const float*>(T.target + size_t(offset) + size_t(row0 + row));
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     const float p = v[j], den = p * p + 0.01f, d = p - y[j];
@@ -441,236 +481,96 @@ __global__ void __launch_bounds__(128, 2) k_nrc_train_tc(NrcDev C, TcTrainArgs T
                 }
             }
             uint4 z0, z1;
-            z0.x = tc_pack(g[0], g[1]); z0.y = tc_pack(g[2], g[3]); z0.z = tc_pack(g[4], g[5]); z0.w = tc_pack(g[6], g[7]);
-            z1.x = tc_pack(g[8], g[9]); z1.y = tc_pack(g[10], g[11]); z1.z = tc_pack(g[12], g[13]); z1.w = tc_pack(g[14], g[15]);
-            // dZ5 tile [128 x 16] (K-major, 2 chunks) in the free input-tile space
-            *reinterpret_cast<uint4*>(smem + kTtA0 + tc_off(tid, 0, 2)) = z0;
-            *reinterpret_cast<uint4*>(smem + kTtA0 + tc_off(tid, 1, 2)) = z1;
-            if (live) {
-                reinterpret_cast<uint4*>(T.DZ5 + size_t(grow) * 16)[0] = z0;
-                reinterpret_cast<uint4*>(T.DZ5 + size_t(grow) * 16)[1] = z1;
-            }
+            pack16(g, z0, z1);
+            *reinterpret_cast<uint4*>(smem + kTtDz5 + tc_off(row, 0, 2)) = z0;
+            *reinterpret_cast<uint4*>(smem + kTtDz5 + tc_off(row, 1, 2)) = z1;
         }
-        tc_fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        // ---- backward: dH4 = dZ5 W5 (K = 16 outputs, N = 64 inputs), then dH_{l-1} = dZ_l W_l
-        if (!run(sbase + kTtA0, 2, sbase + kTcW5, 8 * 128, 128, 2 * 8 * 128, tc_idesc(64, true))) break;
+        ready();
+        // ---- backward: dH_{l-1} = dZ_l W_l; each dW_l behind the product the chain waits for.
+        // A dZ buffer is written again two layers on, when the wait for the layer between
+        // has covered the weight gradient that read it.
+        if (tid == 0) {
+            product(sDz5, 256, 1, sbase + kTcW5, 8 * 128, 128, 2 * 8 * 128, tc_idesc(64, true));
+            wgrad(sP + 2 * kTtTile, sDz5, 256, 16, 384);
+        }
 #pragma unroll
-        for (int l = 4; l >= 0 && ok; --l) {
-            uint32_t packed[32];
-            row64(packed, masks[l], false, true);              // dZ_l = dH_l masked by ReLU'(z_l)
-            store_row(packed, T.DZ + size_t(l) * T.B * 64, grow, live);
-            tc_fence_async_smem();
-            tc_fence_before();
-            __syncthreads();
-            if (l > 0) {
-                ok = run(sbase + kTcA1, 8, sbase + kTcW1 + (l - 1) * 8192, 8 * 128, 128, 2 * 8 * 128,
-                         tc_idesc(64, true));
-            } else {
-                // dX = dZ0 W0, hash-grid columns 0..31 only
-                ok = run(sbase + kTcA1, 8, sbase + kTcW0, 16 * 128, 128, 2 * 16 * 128, tc_idesc(32, true));
-                if (ok) {
-                    float v0[16], v1[16];
-                    tc_ld16(trow, v0);
-                    tc_ld16(trow + 16u, v1);
-                    if (live) {
-                        float4* dst = reinterpret_cast<float4*>(T.dX + size_t(grow) * 32);
+        for (int l = 4; l >= 0; --l) {
+            if (!wait()) break;
+            float v[16];
+            tc_ld16(trow + uint32_t(cg * 16), v);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) dst[q] = make_float4(v0[4 * q], v0[4 * q + 1], v0[4 * q + 2], v0[4 * q + 3]);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) dst[4 + q] = make_float4(v1[4 * q], v1[4 * q + 1], v1[4 * q + 2], v1[4 * q + 3]);
-                    }
-                    tc_fence_before();
-                    __syncthreads();
+            for (int j = 0; j < 16; ++j)
+                if (!((mask[l] >> j) & 1u)) v[j] = 0.f;              // dZ_l = dH_l masked by ReLU'(z_l)
+            uint4 p0, p1;
+            pack16(v, p0, p1);
+            unsigned char* dst = smem + kTtDz + (l & 1) * kTtDzB;
+            *reinterpret_cast<uint4*>(dst + tc_off(row, 2 * cg, 8)) = p0;
+            *reinterpret_cast<uint4*>(dst + tc_off(row, 2 * cg + 1, 8)) = p1;
+            ready();
+            if (tid == 0) {
+                const uint32_t z = sDz + (l & 1) * kTtDzB;
+                if (l > 0) {
+                    product(z, 1024, 4, sbase + kTcW1 + (l - 1) * 8192, 8 * 128, 128, 2 * 8 * 128, tc_idesc(64, true));
+                    wgrad(sP + ((l - 1) >> 1) * kTtTile, z, 1024, 64, 64 + 64 * l);
+                } else {   // dX = dZ0 W0, hash-grid columns 0..31 only
+                    product(z, 1024, 4, sbase + kTcW0, 16 * 128, 128, 2 * 16 * 128, tc_idesc(32, true));
+                    wgrad(sX, z, 1024, 64, 64);
                 }
             }
         }
-        if (!ok || abort_flag) break;
+        if (gave_up || !wait()) break;
+        first = false;
+        // ---- the tile's last weight gradients complete behind the scatter of dX
+        if (tid == 0) tc_commit(bar);
+        {
+            float d[8], u[3];
+            tc_ld8(trow + uint32_t(cg * 8), d);              // levels 4 cg .. 4 cg + 3 of this row
+            const float* f = T.feat + (size_t(offset) + size_t(min(row0 + row, n - 1))) * kNrcFeatFloats;
+            const float fr[3] = {f[0], f[1], f[2]};
+            norm_pos(C, fr, u);
+            for (int k = 0; k < 2; ++k) {                    // the pair of lanes scatters its two rows in turn
+                const int src = (lane & ~1) | k;
+                const float uk[3] = {__shfl_sync(0xffffffffu, u[0], src), __shfl_sync(0xffffffffu, u[1], src),
+                                     __shfl_sync(0xffffffffu, u[2], src)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float dx = __shfl_sync(0xffffffffu, d[2 * j], src), dy = __shfl_sync(0xffffffffu, d[2 * j + 1], src);
+                    if (dx != 0.f || dy != 0.f) scatter_level(C, 4 * cg + j, uk, lane & 1, dx, dy);
+                }
+            }
+        }
+        tc_fence_before();
+        if (!wait()) break;
+    }
+    if (!gave_up) {
+        const int i = row;                                   // TMEM lane = input feature
+        auto out = [&](uint32_t col0, float* dst, int ld, int ioff) {
+            float v[16];
+            tc_ld16(trow + col0, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) atomicAdd(dst + size_t(j) * ld + (i - ioff), v[j]);
+        };
+        const uint32_t c = uint32_t(cg * 16);                // this warp's 16 outputs o
+        out(64 + c, T.dW + kNrcW0 + size_t(c) * 128, 128, 0);                          // dW0[o][i], i = 0..127
+        const int up = i >= 64 ? 1 : 0;                                                // (uniform per warp)
+        out(128 + 64 * up + c, T.dW + kNrcW1 + up * 4096 + size_t(c) * 64, 64, 64 * up);         // dW1, dW2
+        out(256 + 64 * up + c, T.dW + kNrcW1 + (2 + up) * 4096 + size_t(c) * 64, 64, 64 * up);   // dW3, dW4
+        if (cg == 0 && !up) out(384, T.dW + kNrcW5, 64, 0);                            // dW5
     }
     for (int off = 16; off > 0; off >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, off);
     if (lane == 0 && lsum != 0.f) atomicAdd(T.loss, lsum);
-    if (abort_flag && tid == 0) tc_wait(bar, phase ^ 1u);
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTcCols) : "memory");
-    }
-}
-
-
-// ------------------------------------------------------------- weight gradients
-// The six weight-gradient GEMMs of one Adam step, dW_l[o][i] = sum_s dZ_l[s][o]
-// A_l[s][i] (A_0 = the encoded rows X, A_l = H_{l-1}), on tcgen05 in one kernel.
-// The samples s are the reduction dimension K: a CTA stages kWgS samples of
-// every operand as plain row copies (row s of an operand at tc_off(s, chunk,
-// width / 8)), which read as MN-major operands (8 K-rows of 8 contiguous
-// M / N elements per core matrix: LBO = the stride between groups of 8
-// samples, SBO = 128 bytes between groups of 8 features), exactly as the
-// training backward reads its weights.  Every MMA has M = 128: layer 0's A is
-// X (128 features); the 64-wide inputs of two layers are stacked into one
-// 128-wide A (P1 = [H0 | H1], P2 = [H2 | H3], P3 = [H4 | 0]), and each of them
-// is multiplied by the two layers' dZ in turn, so the products needed sit in
-// the accumulator's top or bottom 64 lanes (the other half of each product is
-// not used).  Accumulators (transposed, D[i][o]) stay in TMEM over the CTA's
-// chunks: cols 0-63 dW0^T, 64-127 dW1^T (lanes 0-63), 128-191 dW2^T (lanes
-// 64-127), 192-255 dW3^T (0-63), 256-319 dW4^T (64-127), 320-335 dW5^T (0-63);
-// at the end each CTA adds them into dW with coalesced float atomics (split K
-// over CTAs, as the mma.sync kernels do).
-constexpr int kWgS = 128;                                  // samples per staged chunk
-constexpr int kWgThreads = 256;
-constexpr int kWgX = 0;                                    // [kWgS x 128] A tiles: X, P1, P2, P3
-constexpr int kWgA = kWgS * 128 * 2;                       // bytes per A tile
-constexpr int kWgDz = 4 * kWgA;                            // [kWgS x 64] x 5: dZ0..dZ4
-constexpr int kWgDzB = kWgS * 64 * 2;
-constexpr int kWgDz5 = kWgDz + 5 * kWgDzB;                 // [kWgS x 16]
-constexpr int kWgBar = kWgDz5 + kWgS * 16 * 2;
-constexpr int kWgSmem = kWgBar + 16;
-constexpr uint32_t kWgCols = 512;
-static_assert(kWgSmem <= 227 * 1024, "weight-gradient shared memory");
-
-struct TcWgradArgs {
-    const __nv_bfloat16* X;      // [B][128] encoded rows
-    const __nv_bfloat16* H;      // [5][B][64]
-    const __nv_bfloat16* DZ;     // [5][B][64]
-    const __nv_bfloat16* DZ5;    // [B][16]
-    float* dW;                   // [kNrcParams], accumulated
-    int B;
-};
-
-__global__ void __launch_bounds__(kWgThreads, 1) k_nrc_wgrad_tc(NrcDev C, TcWgradArgs T, const int* n_dev, int offset,
-                                                                int limit, unsigned* __restrict__ errflags) {
-    extern __shared__ __align__(1024) unsigned char wg_smem[];
-    unsigned char* smem = wg_smem;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const uint32_t sbase = uint32_t(__cvta_generic_to_shared(smem));
-    const uint32_t bar = sbase + kWgBar;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kWgBar + 8);
-    __shared__ int abort_flag;
-
-    int n = n_dev ? *n_dev - offset : T.B;
-    if (limit > 0 && n > limit) n = limit;
-    if (n < 0) n = 0;
-    const int nchunks = (n + kWgS - 1) / kWgS;
-    if (int(blockIdx.x) >= nchunks) return;   // (uniform per CTA, before any TMEM allocation)
-
-    // the zero half of P3 is written once
-    for (int v = tid; v < kWgS * 8; v += kWgThreads) {
-        const int sl = v >> 3, kc = 8 + (v & 7);
-        *reinterpret_cast<uint4*>(smem + kWgX + 3 * kWgA + tc_off(sl, kc, 16)) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (tid == 0) {
-        abort_flag = 0;
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(sbase + kWgBar + 8), "r"(kWgCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    // after a timeout, give the outstanding products, the weight gradients issued behind the
+    // last commit among them, one more bounded wait each before their TMEM is freed
+    if (gave_up && tid == 0) {
+        tc_commit(bar);
+        tc_wait(bar, phase ^ 1u);
+        tc_wait(bar, phase);
     }
     tc_fence_before();
     __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const size_t L = size_t(T.B) * 64;
-    uint32_t phase = 0;
-    bool first = true;
-    for (int chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {
-        const int s0 = chunk * kWgS;
-        // stage: 16-byte pieces of sample rows; rows past n are zero
-        for (int v = tid; v < kWgS * 16; v += kWgThreads) {              // X: 16 chunks per row
-            const int sl = v >> 4, kc = v & 15;
-            uint4 x = make_uint4(0u, 0u, 0u, 0u);
-            if (s0 + sl < n) x = *reinterpret_cast<const uint4*>(T.X + size_t(s0 + sl) * 128 + kc * 8);
-            *reinterpret_cast<uint4*>(smem + kWgX + tc_off(sl, kc, 16)) = x;
-        }
-        for (int v = tid; v < kWgS * 8 * 5; v += kWgThreads) {           // H0..H4 into P1, P2, P3
-            const int l = v / (kWgS * 8), r = v % (kWgS * 8), sl = r >> 3, kc = r & 7;
-            uint4 x = make_uint4(0u, 0u, 0u, 0u);
-            if (s0 + sl < n) x = *reinterpret_cast<const uint4*>(T.H + size_t(l) * L + size_t(s0 + sl) * 64 + kc * 8);
-            const int tile = 1 + (l >> 1), half = l & 1;
-            *reinterpret_cast<uint4*>(smem + kWgX + tile * kWgA + tc_off(sl, kc + 8 * half, 16)) = x;
-        }
-        for (int v = tid; v < kWgS * 8 * 5; v += kWgThreads) {           // dZ0..dZ4
-            const int l = v / (kWgS * 8), r = v % (kWgS * 8), sl = r >> 3, kc = r & 7;
-            uint4 x = make_uint4(0u, 0u, 0u, 0u);
-            if (s0 + sl < n) x = *reinterpret_cast<const uint4*>(T.DZ + size_t(l) * L + size_t(s0 + sl) * 64 + kc * 8);
-            *reinterpret_cast<uint4*>(smem + kWgDz + l * kWgDzB + tc_off(sl, kc, 8)) = x;
-        }
-        for (int v = tid; v < kWgS * 2; v += kWgThreads) {               // dZ5
-            const int sl = v >> 1, kc = v & 1;
-            uint4 x = make_uint4(0u, 0u, 0u, 0u);
-            if (s0 + sl < n) x = *reinterpret_cast<const uint4*>(T.DZ5 + size_t(s0 + sl) * 16 + kc * 8);
-            *reinterpret_cast<uint4*>(smem + kWgDz5 + tc_off(sl, kc, 2)) = x;
-        }
-        tc_fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            // (A tile, its LBO) x (B tile, its LBO, N) -> TMEM columns
-            auto gemm = [&](uint32_t a, uint32_t b, uint32_t b_lbo, int N, uint32_t col) {
-                const uint32_t idesc = tc_idesc(N, true) | (1u << 15);   // A and B MN-major
-                for (int k = 0; k < kWgS / 16; ++k)
-                    tc_mma(tmem + col, tc_desc(a + k * 2 * 2048, 2048, 128), tc_desc(b + k * 2 * b_lbo, b_lbo, 128),
-                           idesc, (first && k == 0) ? 0u : 1u);
-            };
-            const uint32_t A0 = sbase + kWgX, P1 = A0 + kWgA, P2 = A0 + 2 * kWgA, P3 = A0 + 3 * kWgA;
-            const uint32_t Z = sbase + kWgDz;
-            gemm(A0, Z + 0 * kWgDzB, 1024, 64, 0);
-            gemm(P1, Z + 1 * kWgDzB, 1024, 64, 64);
-            gemm(P1, Z + 2 * kWgDzB, 1024, 64, 128);
-            gemm(P2, Z + 3 * kWgDzB, 1024, 64, 192);
-            gemm(P2, Z + 4 * kWgDzB, 1024, 64, 256);
-            gemm(P3, sbase + kWgDz5, 256, 16, 320);
-            tc_commit(bar);
-        }
-        first = false;
-        if (!tc_wait(bar, phase, C.wait_polls)) {
-            atomicOr(errflags, BG_FLAG_TIMEOUT);
-            abort_flag = 1;
-        }
-        phase ^= 1u;
-        tc_fence_after();
-        __syncthreads();   // the MMAs have read this chunk's tiles before they are overwritten
-        if (abort_flag) break;
-    }
-    if (!abort_flag) {
-        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (lane = feature i); warps w and w + 4
-        // split the columns
-        const int q = warp & 3, half = warp >> 2;
-        const int i = q * 32 + (tid & 31);
-        const uint32_t trow = tmem + (uint32_t(q * 32) << 16);
-        auto out = [&](uint32_t col0, int ncols, float* dst, int ld, int ioff) {
-            for (int c = 0; c < ncols; c += 16) {
-                float v[16];
-                tc_ld16(trow + col0 + uint32_t(c), v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) atomicAdd(dst + size_t(c + j) * ld + (i - ioff), v[j]);
-            }
-        };
-        float* dW = T.dW;
-        if (half == 0) {
-            out(0, 64, dW + kNrcW0, 128, 0);                                   // dW0[o][i], i = 0..127
-            if (i < 64) out(64, 64, dW + kNrcW1, 64, 0);                       // dW1 = H0^T dZ1
-            else out(128, 64, dW + kNrcW1 + 4096, 64, 64);                     // dW2 = H1^T dZ2
-        } else {
-            if (i < 64) {
-                out(192, 64, dW + kNrcW1 + 2 * 4096, 64, 0);                   // dW3 = H2^T dZ3
-                out(320, 16, dW + kNrcW5, 64, 0);                              // dW5 = H4^T dZ5
-            } else {
-                out(256, 64, dW + kNrcW1 + 3 * 4096, 64, 64);                  // dW4 = H3^T dZ4
-            }
-        }
-    }
-    // after a timeout, give the outstanding MMA group one more bounded wait before freeing its TMEM
-    if (abort_flag && tid == 0) tc_wait(bar, phase ^ 1u);
-    tc_fence_before();
-    __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kWgCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTtCols) : "memory");
     }
 }
 
