@@ -151,7 +151,7 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* sw, const uint3
 
 // raw query records [n][16] -> encoded bf16 rows [n][128] (the training path;
 // inference encodes inside k_nrc_infer_tc).  Eight lanes per row: the pair of lane
-// quarter q encodes levels 4q .. 4q + 3 (encode_level) and one of the four one-blobs,
+// quarter q encodes levels 4q .. 4q + 3 (encode_levels) and one of the four one-blobs,
 // and each lane stores its own words.  A step of 16,384 rows is latency-bound: one
 // lane per row 29.6 us (seven warps per SM), a pair per row 24.9, eight lanes 12.
 // Inside k_nrc_train_tc the same took 28: its shared memory leaves an L1 of some
@@ -172,11 +172,7 @@ __global__ void __launch_bounds__(128) k_nrc_encode(NrcDev C, const float* __res
         norm_pos(C, pos, u);
         uint32_t g[2], b[4];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {   // lane h keeps levels 4q + 2h + k
-            const float lo = encode_level(C, 4 * q + k, u, h), hi = encode_level(C, 4 * q + 2 + k, u, h);
-            const float got = __shfl_xor_sync(0xffffffffu, h ? lo : hi, 1);
-            g[k] = h ? pack_bf16(got, hi) : pack_bf16(lo, got);
-        }
+        for (int k = 0; k < 2; ++k) g[k] = encode_levels(C, 4 * q + k, 4 * q + 2 + k, u, h);   // lane h: levels 4q + 2h + k
         float th, ph;
         if (q < 2) sph(q0.w, q1.x, q1.y, th, ph);
         else sph(q1.z, q1.w, q2.x, th, ph);

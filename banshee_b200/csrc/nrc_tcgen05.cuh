@@ -142,9 +142,9 @@ __device__ __forceinline__ void tc_load_weights(const __nv_bfloat16* __restrict_
 // says how they are paired.  Two groups per SM overlap one group's MMA chain
 // with the other's gathers.  Measured for 200,003 / 1,000,000 / 5,000 rows
 // (tables of 2^19 entries): one lane per row, 128 threads per tile, 109 / 500 /
-// 18.5 us; pairs of lanes, 256 threads, two CTAs of one group 92 / 410 / 17.5;
-// one CTA of two groups 100 / 436 / 22, of three 93 / 398 / 27 (fewer CTAs
-// start later), one group per SM 120 / 565 / 16.5.
+// 18.5 us; pairs of lanes, 256 threads, two CTAs of one group 85 / 382 / 16.5;
+// one CTA of two groups 94 / 430 / 16.5, of three 90 / 410 / 16.5 (their tiles
+// spread over the SMs), one group per SM some 120 / 565.
 constexpr int kTiGroups = 1;
 constexpr int kTiCtasPerSm = 2;                            // CTAs per SM in the grid
 constexpr int kTiGroupThreads = 256;
