@@ -4,7 +4,8 @@ A cast of a few rays goes to groups of 32 or 8 lanes per ray, a larger one to on
 lane per ray on packed nodes or, below 1,000 triangles, to the plain walk; the
 host entry points read a few rays in place.  The same rays cast in pieces of
 every size around those limits must give the same ids, t, u, v and occlusion
-bits as one large cast, ties between coincident triangles included.
+bits as one large cast, ties between coincident triangles included.  Scenes of a few nodes
+have a walk of their own in large launches: the same bits again.
 """
 import numpy as np
 import pytest
@@ -152,3 +153,55 @@ def test_coordinates_beyond_the_packed_range_keep_the_plain_walk(ctx, oracle_bui
     assert (want["primid"] >= 0).mean() > 0.05
     assert (got["primid"] == want["primid"]).all()
     assert (got["t"].view(np.uint32) == want["t"].view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("intersect", [0, 1], ids=["moller", "watertight"])
+@pytest.mark.parametrize("ntris", [1, 3, 6, 10])
+def test_scenes_of_few_nodes_give_the_bits_of_the_groups(ctx, oracle_built, ntris, intersect):
+    """One to four nodes, every third triangle there three times: one large cast against
+    casts small enough for groups of lanes, and t against the oracle."""
+    import torch
+    from banshee_b200 import capi
+    sc = _ties(ntris)
+    gs = capi.GpuScene(ctx, sc, intersect=intersect)
+    n = 32 * WARPS + 20_000
+    rays = _rays(n, 17)
+    dev = torch.from_numpy(rays.view(np.uint8).reshape(n, 32)).cuda()
+
+    def cast(lo, hi):
+        h = torch.full((hi - lo, 4), -5.0, device="cuda")
+        o = torch.full((hi - lo,), 9, dtype=torch.uint8, device="cuda")
+        piece = dev[lo:hi].contiguous()
+        gs.intersect_closest(piece.data_ptr(), h.data_ptr(), hi - lo)
+        gs.intersect_any(piece.data_ptr(), o.data_ptr(), hi - lo)
+        torch.cuda.synchronize()
+        return h.cpu().numpy().view(np.uint32), o.cpu().numpy()
+
+    whole, occ = cast(0, n)
+    for lo in range(0, n, 32 * WARPS):
+        h, o = cast(lo, min(n, lo + 32 * WARPS))
+        assert (h == whole[lo:lo + 32 * WARPS]).all()
+        assert (o == occ[lo:lo + 32 * WARPS]).all()
+    if intersect == 0:
+        plain = scenes.soup_rays(n, "incoherent", seed=18)
+        got = gs.intersect_closest_host(plain)
+        want = oracle_built.Oracle(sc).intersect_closest(plain)
+        assert (got["t"].view(np.uint32) == want["t"].view(np.uint32)).all()
+    assert gs.error_flags() == 0
+
+
+@pytest.mark.parametrize("spp", [1, 3])
+def test_cornell_renders_the_same_in_a_batch(ctx, spp):
+    """A pass of more paths than groups of lanes take: one scene of nine nodes against
+    the same scene as a batch, whose rays walk the tree from a root of their own."""
+    import torch
+    from banshee_b200 import capi
+    w, h = 320, 304
+    gs = capi.GpuScene(ctx, scenes.cornell(w, h))
+    assert gs.info()["nnodes"] <= 16
+    want = gs.render_host(w, h, spp, seed=3, maxdepth=5)
+    batch = capi.Batch(ctx, [gs])
+    acc = torch.zeros((h, w, 4), device="cuda")
+    batch.render([dict(scene=0, width=w, height=h, spp=spp, seed=3, accum_dev=acc.data_ptr())], maxdepth=5)
+    torch.cuda.synchronize()
+    assert (acc.cpu().numpy().view(np.uint32) == want.view(np.uint32)).all()
