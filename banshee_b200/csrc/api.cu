@@ -682,8 +682,6 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
             return set_error(BG_ERR_UNSUPPORTED, "8-wide BVH needs a %d-entry traversal stack (> %d)", ms8, kStackSize8);
         nn8 = 0;
     }
-    bool packed = false;
-    if (nn4 && (rc = device_pack_nodes(s->nodes.as<WideNode4>(), nn4, s->qnodes, &packed))) return rc;
     const auto tb1 = std::chrono::steady_clock::now();
     // traversal records in leaf order, shading records in primitive order
     if ((rc = s->tris.ensure(size_t(ntris) * sizeof(TriRec))) || (rc = s->shade.ensure(size_t(ntris) * sizeof(ShadeRec))))
@@ -705,6 +703,8 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
         (rc = s->err.ensure(sizeof(unsigned))) ||
         (rc = s->work.ensure(kWorkSlots * sizeof(unsigned long long))))
         return rc;
+    bool packed = false;
+    if (nn4 && (rc = device_pack_nodes(s->nodes.as<WideNode4>(), nn4, s->qnodes, &packed))) return rc;
     BG_CUDA(cudaMemcpy(s->mats_d.ptr, mats.data(), mats.size() * sizeof(MatRec), cudaMemcpyHostToDevice));
     if (!lights.empty())
         BG_CUDA(cudaMemcpy(s->lights_d.ptr, lights.data(), lights.size() * sizeof(LightRec), cudaMemcpyHostToDevice));

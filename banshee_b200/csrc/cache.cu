@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(128) k_nrc_encode(NrcDev C, const float* __res
         float th, ph;
         if (q < 2) sph(q0.w, q1.x, q1.y, th, ph);
         else sph(q1.z, q1.w, q2.x, th, ph);
-        one_blob<8>((q & 1) ? ph : th, b, 8 * h);
+        one_blob<8>((q & 1) ? ph : th, (q & 1) ? 1.f : kPolar, b, 8 * h);
         if (i >= n) continue;
         uint32_t* dst = reinterpret_cast<uint32_t*>(X + size_t(i) * kNrcIn);
         const int c = 2 * q + h;                 // this lane's eighth of the row

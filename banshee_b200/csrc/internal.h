@@ -169,7 +169,8 @@ int device_world_boxes(MeshArrays& A, const BundleRec* bundles, int64_t ntris, f
 int device_records(const MeshArrays& A, const BundleRec* bundles, const int32_t* order, int64_t ntris,
                    TriRec* tris, ShadeRec* shade, bool vertices, const int32_t* mat_class, int nmat);
 // nodes packed for traversal (QNode4) into `out`; *packed = false when some
-// node's planes are outside the packed range (the traversal then walks `nodes`)
+// node's planes are outside the packed range or there is no memory for them (the
+// traversal then walks `nodes`)
 int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* packed);
 constexpr int kWorkSlots = 256;
 unsigned long long* next_work_counter(bg_scene* s);

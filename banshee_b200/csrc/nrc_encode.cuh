@@ -35,10 +35,12 @@ struct GridCorner {
 __device__ __forceinline__ GridCorner grid_cell(const NrcDev& C, int level, const float* u) {
     GridCorner g;
     const float N = float(C.res[level]);
-    float x = u[0] * N, y = u[1] * N, z = u[2] * N;
+    // (every rounding that reaches an encoded value is spelled out here and below: which
+    // product the compiler would fuse into an add depends on the code around it)
+    float x = __fmul_rn(u[0], N), y = __fmul_rn(u[1], N), z = __fmul_rn(u[2], N);
     float fx0 = fminf(floorf(x), N - 1.f), fy0 = fminf(floorf(y), N - 1.f), fz0 = fminf(floorf(z), N - 1.f);
     g.x0 = int(fx0); g.y0 = int(fy0); g.z0 = int(fz0);
-    g.fx = x - fx0; g.fy = y - fy0; g.fz = z - fz0;
+    g.fx = __fsub_rn(x, fx0); g.fy = __fsub_rn(y, fy0); g.fz = __fsub_rn(z, fz0);
     return g;
 }
 
@@ -47,22 +49,24 @@ __device__ __forceinline__ void norm_pos(const NrcDev& C, const float* f, float*
     for (int k = 0; k < 3; ++k) u[k] = fminf(fmaxf((f[k] - C.bmin[k]) * C.bscale[k], 0.f), 1.f);
 }
 
-// one-blob encoding of v in [0,1] into 16 bf16 values, packed two per word: values
-// first .. first + N - 1 of them
+// one-blob encoding of v = a * m in [0,1] into 16 bf16 values, packed two per word:
+// values first .. first + N - 1 of them
 template <int N = 16>
-__device__ __forceinline__ void one_blob(float v, uint32_t* w, int first = 0) {
+__device__ __forceinline__ void one_blob(float a, float m, uint32_t* w, int first = 0) {
 #pragma unroll
     for (int k = 0; k < N; k += 2) {
         const int b = first + k;
-        const float d0 = v - (b + 0.5f) * (1.f / 16.f), d1 = v - (b + 1.5f) * (1.f / 16.f);
+        const float d0 = __fmaf_rn(a, m, -((b + 0.5f) * (1.f / 16.f))), d1 = __fmaf_rn(a, m, -((b + 1.5f) * (1.f / 16.f)));
         w[k / 2] = pack_bf16(__expf(-d0 * d0 * 128.f), __expf(-d1 * d1 * 128.f));
     }
 }
 
+// polar angle (radians) and azimuth in [0,1]
 __device__ __forceinline__ void sph(float x, float y, float z, float& th, float& ph) {
-    th = acosf(fminf(fmaxf(z, -1.f), 1.f)) * (1.f / BG_PI);
-    ph = atan2f(y, x) * (0.5f / BG_PI) + 0.5f;
+    th = acosf(fminf(fmaxf(z, -1.f), 1.f));
+    ph = __fmaf_rn(atan2f(y, x), 0.5f / BG_PI, 0.5f);
 }
+constexpr float kPolar = 1.f / BG_PI;   // polar angle to [0,1]
 
 // The encoded row of one raw query record (16 floats: position, outgoing
 // direction, shading normal, roughness, albedo) is 64 words: 0-15 the grid
@@ -124,8 +128,8 @@ __device__ __forceinline__ void encode_pair(const NrcDev& C, const float* __rest
     for (int l = 0; l < kNrcLevels / 2; ++l) g[l] = encode_levels(C, l, l + kNrcLevels / 2, u, h);
     float th, ph;
     sph(h ? q1.z : q0.w, h ? q1.w : q1.x, h ? q2.x : q1.y, th, ph);
-    one_blob(th, b);
-    one_blob(ph, b + 8);
+    one_blob(th, kPolar, b);
+    one_blob(ph, 1.f, b + 8);
     t[0] = pack_bf16(q2.y, q2.z);
     t[1] = pack_bf16(q2.w, q3.x);
     t[2] = pack_bf16(1.f, 0.f);

@@ -253,7 +253,10 @@ int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* pack
     *packed = false;
     ScratchBuf bad;
     int rc;
-    if ((rc = out.ensure(size_t(n) * sizeof(QNode4))) || (rc = bad.ensure(sizeof(unsigned)))) return rc;
+    if ((rc = out.ensure(size_t(n) * sizeof(QNode4))) || (rc = bad.ensure(sizeof(unsigned)))) {
+        out.release();
+        return rc == BG_ERR_OOM ? BG_OK : rc;   // no room: the plain walk needs none
+    }
     BG_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned), 0));
     k_pack_nodes<<<grid_for(n), kRT>>>(nodes, n, out.as<QNode4>(), bad.as<unsigned>());
     BG_CUDA(cudaGetLastError());

@@ -316,7 +316,8 @@ int bg_intersect_any(bg_scene* scene, const bg_ray* rays_dev, uint8_t* occluded_
 int bg_intersect_closest_host(bg_scene* scene, const bg_ray* rays, bg_hit* hits, int64_t n);
 int bg_intersect_any_host(bg_scene* scene, const bg_ray* rays, uint8_t* occluded, int64_t n);
 
-/* Instrumented replay of the same traversal: total nodes fetched and
+/* Instrumented replay on the nodes whose order defines the results (large
+ * launches may walk other nodes to the same hits): total nodes fetched and
  * triangles tested over the n rays (the per-ray byte model of the roofline).
  * Runs on the scene's device and gives the calling thread's current device
  * back; synchronous on `stream`.  A replay whose traversal stack overflowed

@@ -205,3 +205,26 @@ def test_cornell_renders_the_same_in_a_batch(ctx, spp):
     batch.render([dict(scene=0, width=w, height=h, spp=spp, seed=3, accum_dev=acc.data_ptr())], maxdepth=5)
     torch.cuda.synchronize()
     assert (acc.cpu().numpy().view(np.uint32) == want.view(np.uint32)).all()
+
+
+def test_commit_without_room_for_the_packed_nodes(ctx):
+    """The packed nodes are allocated last: a budget one byte short of a commit's needs
+    leaves the scene to the plain walk, with the same hits."""
+    from banshee_b200 import capi
+    sc = scenes.soup(20_000, seed=14)
+    rays = scenes.soup_rays(32 * WARPS + 5_000, "incoherent", seed=15)
+    full = capi.GpuScene(ctx, sc, commit=False)
+    before = capi.alloc_stats()["bytes"]
+    full.commit()
+    need = capi.alloc_stats()["bytes"] - before
+    tight = capi.GpuScene(ctx, sc, commit=False)
+    capi.alloc_limit(need - 1)
+    try:
+        tight.commit()
+    finally:
+        capi.alloc_limit(None)
+    want = full.intersect_closest_host(rays)
+    got = tight.intersect_closest_host(rays)
+    assert (want["primid"] >= 0).mean() > 0.05
+    assert (got.view(np.uint32) == want.view(np.uint32)).all()
+    assert (tight.intersect_any_host(rays) == full.intersect_any_host(rays)).all()
