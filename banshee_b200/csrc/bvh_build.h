@@ -53,7 +53,7 @@ struct alignas(32) QNode8 {
 static_assert(sizeof(QNode8) == 96, "compressed node must be three 32-byte sectors");
 
 // 64-byte form of a WideNode4 (same index, same child codes): what the
-// traversal walks.  Per axis a plane byte q lies at o_a + (2^15 + q) * s_a
+// packed and group walks read.  Per axis a plane byte q lies at o_a + (2^15 + q) * s_a
 // (o_a: the grid origin less 2^15 s_a), which the traversal evaluates as
 // fmaf(2^15 + q, s_a / d_a, (o_a - ray origin_a) / d_a): the byte is placed in
 // the mantissa of the float 2^15 + q.  lo bytes are rounded down and hi bytes

@@ -31,11 +31,7 @@ constexpr int kTcRows = 128;                               // rows per tile (UMM
 constexpr int kTcW0 = 0;                                   // [64 x 128]
 constexpr int kTcW1 = kTcW0 + 64 * 128 * 2;                // 4 x [64 x 64]
 constexpr int kTcW5 = kTcW1 + 4 * 64 * 64 * 2;             // [16 x 64]
-constexpr int kTcA0 = kTcW5 + 16 * 64 * 2;                 // [128 x 128]
-constexpr int kTcA1 = kTcA0 + kTcRows * 128 * 2;           // [128 x 64]
-constexpr int kTcBar = kTcA1 + kTcRows * 64 * 2;           // mbarrier (8 B) + TMEM base (4 B)
-constexpr int kTcSmem = kTcBar + 16;
-constexpr uint32_t kTcCols = 64;                           // TMEM columns allocated
+constexpr int kTcA0 = kTcW5 + 16 * 64 * 2;                 // end of the weights, first tile
 constexpr uint32_t kTcWaitLimit = 1u << 24;                // mbarrier polls before giving up
 
 // byte offset of core-matrix row `r`, 16-byte chunk `kc` in a K-major tile with KC chunks per row
