@@ -306,7 +306,7 @@ k_trace_flat(DevScene scene, int nnodes, const float4* __restrict__ rays, int n_
                     if (!(tn[i] < kMiss) || ch[i] == kEmptyChild) continue;
                     if (ch[i] >= 0) {
                         open |= 1u << ch[i];
-                        if (ch[i] <= k) s.r.flags |= kNearTie;   // (no builder numbers a child before its parent)
+                        if (ch[i] <= k) s.r.flags |= kPlainWalk;   // (no builder numbers a child before its parent)
                     } else {
                         mask |= 1ull << (4 * k + i);
                         if (tn[i] < first) { first = tn[i]; bit = 4 * k + i; }

@@ -82,7 +82,7 @@ constexpr float kFastSlack = 1e-5f;
 // Ray::flags: bits 0-2 sign of 1/d per axis
 constexpr uint32_t kOctMask = 7u;
 constexpr uint32_t kPlainWalk = 8u;   // walk the plain nodes
-constexpr uint32_t kNearTie = 16u;    // packed walk: a second triangle near the closest one
+constexpr uint32_t kNearTie = 16u;    // packed walk: a second triangle near the closest one, or a hit by an edge
 
 // kWalkPacked and kWalkFused keep the ray's origin and direction, which they need
 // only for a new bundle's object-space ray and for a plain visit, in shared memory:
@@ -277,6 +277,14 @@ __device__ __forceinline__ bool wt_test(const ObjRayWT& c, v3 p1, v3 p2, v3 p3, 
     b = W * rcp;
     return true;
 }
+
+// Whether a hit at barycentrics a, b lies by an edge of its triangle.  The true hit may
+// then lie outside the triangle and its boxes by the test's rounding, where the plain
+// walk's box test can cull it (a ray along a wall, from the border of the box): the other
+// walks, with wider boxes, ask the plain one.  (18 of 671M rays inside a Cornell box
+// differed without this, none with it.  A bound from the operands' sizes instead of a
+// constant cost casts 4-12 %.)
+__device__ __forceinline__ bool near_edge(float a, float b) { return !(min3(a, b, 1.f - a - b) > 1e-4f); }
 
 // entry distance of a child that is not hit: +inf
 #define kMiss __int_as_float(0x7f800000)
@@ -702,6 +710,11 @@ __device__ __forceinline__ bool trav_leaf(const TraceScene& S, TravState<WT, WAL
         hit = mt_test(s.cache.o, s.cache.d, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z),
                       s.r.tmin, tmax, t, a, b);
     if (hit) {
+        const bool edge = WALK != kWalkPlain && !(s.r.flags & kPlainWalk) && near_edge(a, b);
+        if (ANY && edge) {   // an occluder if another one is found or the plain walk finds it
+            s.r.flags |= kNearTie;
+            return false;
+        }
         if (margin) {
             // near the hit it replaces (or is replaced by): a tie; clearly closer: none any more
             if (t < fmaf(fabsf(s.best), -kFastSlack, s.best)) s.r.flags &= ~kNearTie;
@@ -709,7 +722,11 @@ __device__ __forceinline__ bool trav_leaf(const TraceScene& S, TravState<WT, WAL
             if (t > s.best) return false;
         }
         s.prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
-        if (ANY) return true;
+        if (ANY) {
+            s.r.flags &= ~kNearTie;
+            return true;
+        }
+        if (edge) s.r.flags |= kNearTie;
         s.best = t; s.u = a; s.v = b;
         s.cull = trav_cull(s, t);
     }
@@ -816,6 +833,7 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
         int hc[4], npush = 0;
         float t = 0.f, u = 0.f, v = 0.f;
         int prim = -1;
+        bool edge = false;
         if (item >= 0 && item != kNone) {   // (kNone: none, culled, or an empty slot)
             box4_packed(S.qnodes, item, s.r, cull, ht, hc);
             sort4(ht, hc);
@@ -842,9 +860,11 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
             else
                 hit = mt_test(s.cache.o, s.cache.d, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin,
                               bound, t, u, v);
-            if (hit) prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
+            edge = hit && near_edge(u, v);
+            if (hit && !(ANY && edge)) prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
         }
-        const unsigned hits = __ballot_sync(kFull, prim >= 0);
+        const unsigned hits = __ballot_sync(kFull, prim >= 0), edges = __ballot_sync(kFull, edge) & gmask;
+        if (ANY && edges) near = true;
         if (hits) {
             if (ANY) {
                 if (hits & gmask) { r.prim = 0; owner = base; count = 0; npush = 0; }
@@ -858,6 +878,7 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
                         near = (owner >= 0 && !(m < fmaf(fabsf(best), -kFastSlack, best))) || __popc(close) > 1;
                         best = m;
                         owner = __ffs(at) - 1;
+                        near = near || ((edges >> owner) & 1u);
                         if (base + g == owner) { r.t = t; r.u = u; r.v = v; r.prim = prim; }
                     } else {
                         near = true;
@@ -875,7 +896,7 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
         count += __popc(b0 & gmask) + 2 * __popc(b1 & gmask) + 4 * __popc(b2 & gmask);
         __syncwarp();
     }
-    if (!ANY && near) r.redo = true;
+    if (near && (!ANY || owner < 0)) r.redo = true;
     r.writer = live && !r.redo && base + g == (owner >= 0 ? owner : base);
     r.redo = r.redo && g == 0;
     return r;

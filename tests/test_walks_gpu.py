@@ -228,3 +228,40 @@ def test_commit_without_room_for_the_packed_nodes(ctx):
     assert (want["primid"] >= 0).mean() > 0.05
     assert (got.view(np.uint32) == want.view(np.uint32)).all()
     assert (tight.intersect_any_host(rays) == full.intersect_any_host(rays)).all()
+
+
+@pytest.mark.parametrize("n", [1, 33, 4000])
+def test_rays_along_a_wall_give_the_bits_of_the_plain_walk(ctx, n):
+    """Rays from the walls of a Cornell box that leave its box by a millionth of their way:
+    the first three hit a wall's edge in boxes that the plain walk culls."""
+    import torch
+    from banshee_b200 import capi
+    gs = capi.GpuScene(ctx, scenes.cornell(64, 64))
+    h = float.fromhex
+    rays = scenes.soup_rays(32 * WARPS + 4096, "incoherent", seed=21)
+    rng = np.random.default_rng(22)
+    k = len(rays)
+    o, d = rng.random((k, 3)).astype(np.float32), rng.normal(size=(k, 3)).astype(np.float32)
+    axis = rng.integers(0, 3, k)
+    o[np.arange(k), axis] = rng.integers(0, 2, k)
+    d[np.arange(k), axis] = np.ldexp(rng.normal(size=k), -rng.integers(16, 28, k))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    fixed = [("0x1.a7aa62p-4", "0x1p+0", "0x1.327fd8p-5", "-0x1.ffff98p-1", "0x1.c56ca6p-21", "0x1.45e482p-9"),
+             ("0x1.76e478p-2", "0x1p+0", "0x1.f532fep-4", "0x1.e4f704p-3", "0x1.4dc444p-22", "-0x1.f17020p-1"),
+             ("0x1p+0", "0x1.fcb3d2p-1", "0x1.e313e4p-2", "0x1.57aa4cp-20", "0x1.338888p-1", "0x1.99598cp-1")]
+    for i, f in enumerate(fixed):
+        o[i], d[i] = [h(x) for x in f[:3]], [h(x) for x in f[3:]]
+    rays["o"], rays["d"], rays["tmin"], rays["tmax"] = o, d, 0.01, 1e6
+    dev = torch.from_numpy(rays.view(np.uint8).reshape(k, 32)).cuda()
+
+    def cast(m):
+        out, occ = torch.zeros((m, 4), device="cuda"), torch.zeros((m,), dtype=torch.uint8, device="cuda")
+        gs.intersect_closest(dev.data_ptr(), out.data_ptr(), m)
+        gs.intersect_any(dev.data_ptr(), occ.data_ptr(), m)
+        torch.cuda.synchronize()
+        return out.cpu().numpy().view(np.uint32), occ.cpu().numpy()
+
+    whole, occ = cast(k)                        # more rays than groups take: the plain walk
+    got, gocc = cast(n)                         # groups of lanes
+    assert (got == whole[:n]).all() and (gocc == occ[:n]).all()
+    assert (whole[:min(n, 3), 1].view(np.int32) == -1).all()
