@@ -146,9 +146,12 @@ __device__ __forceinline__ void make_ray(RayFast& r, float extent, uint32_t walk
     // the packed arithmetic's range (comparisons false for NaN: plain walk)
     const bool ok = ai.x <= 1e15f && ai.y <= 1e15f && ai.z <= 1e15f && min3(ai.x, ai.y, ai.z) >= 1e-15f && far <= 1e15f;
     r.flags = octant(r.inv) | (ok ? walk : kPlainWalk);
-    // every rounding of a plane's distance (of 1/d, of the intercepts, of the final
-    // multiply-add) is at most 2^-24 of (|plane| + |o|) / |d|; five of them add up
-    const float e = (extent + far) * 4.8e-7f;
+    // the bound of the roundings: those of a plane's distance here (of the intercepts and
+    // the final multiply-add) are together at most 3 x 2^-24 of (|plane| + |o|) / |d|, and the
+    // plain test reaches, by its slack and its own three roundings, 7e-7 of the distance
+    // further than the exact one, on either plane.  So with 1e-6 this one enters every box
+    // that the plain one enters.  (With 4.8e-7 a hit just behind tmin could be lost.)
+    const float e = (extent + far) * 1e-6f;
     const float ex = fmaf(e, ai.x, 1e-36f), ey = fmaf(e, ai.y, 1e-36f), ez = fmaf(e, ai.z, 1e-36f);
     const float ox = a.x * r.inv.x, oy = a.y * r.inv.y, oz = a.z * r.inv.z;
     r.cn = mk(-ox - ex, -oy - ey, -oz - ez);
