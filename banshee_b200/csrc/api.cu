@@ -151,8 +151,8 @@ k_trace(DevScene scene, const float4* __restrict__ rays, int64_t n_static, const
     TraceScene S;
     static_cast<DevScene&>(S) = scene;
     S.rays = rays;
-    constexpr bool kOwn = WALK == kWalkPacked || WALK == kWalkFused;
-    __shared__ float4 own[kOwn ? 2 : 1][kOwn ? THREADS : 1];
+    constexpr bool kOwn = kKeeps<WALK>;
+    __shared__ float4 own[kOwn ? 3 : 1][kOwn ? THREADS : 1];
     S.own = &own[0][kOwn ? threadIdx.x : 0];
     S.ownstep = THREADS;
     const int n_all = n_dev ? *n_dev : int(n_static);   // (at most 2^30: launch_trace)
@@ -165,8 +165,21 @@ k_trace(DevScene scene, const float4* __restrict__ rays, int64_t n_static, const
     TravState<WT, WALK> s;
     Counters cnt{0ull, 0ull, 0ull};
     bool active = false, again = false;   // again: the lane's ray is walked again on the plain nodes
+    bool done = false;                    // the lane's ray waits for its answer
     bool exhausted = false;
     for (;;) {
+        // (Answered here, not where its walk ended: with the test there the compiler kept less of
+        // the walk's state in registers, casts 5-13 % slower, C3 30.6 ms instead of 29.8.)
+        if constexpr (kOwn) {
+            if (done) {
+                done = false;
+                again = s.r.flags & kTie;   // the plain walk decides
+                if (!again && !(s.r.flags & kPlainWalk) && s.prim >= 0)
+                    again = !plain_reaches<WT>(scene, __float_as_int(S.own[2 * THREADS].x), s.prim,
+                                               ANY ? S.own[2 * THREADS].y : s.best, &S.own[0].x, s.r.inv, s.r.tmin);
+                if (!again) trace_emit<ANY>(res, hits, occ, s.r.idx, s.prim, s.best, s.u, s.v);   // (best = tmax on a miss)
+            }
+        }
         const unsigned need = __ballot_sync(0xffffffffu, !active && !again);
         int my = n;
         if (need && !exhausted) {
@@ -199,7 +212,7 @@ k_trace(DevScene scene, const float4* __restrict__ rays, int64_t n_static, const
         }
         if (active && trav_steps<ANY, COUNT, WIDTH>(S, s, stack, refill_steps<ANY, WALK>(), fused, cnt)) {
             active = false;
-            if (WALK != kWalkPlain && (s.r.flags & kNearTie)) again = true;   // the plain walk decides
+            if (kOwn) done = true;
             else trace_emit<ANY>(res, hits, occ, COUNT ? s.r.idx / stride : s.r.idx, s.prim, s.best, s.u, s.v);   // (best = tmax on a miss)
         }
     }
@@ -264,7 +277,7 @@ k_trace_coop(DevScene scene, const float4* __restrict__ rays, int n_static, cons
 // closest hit.  In k_trace the lanes of a warp are at nodes and at leaves by turns, and
 // each turn costs both: 10 of 32 lanes are active in a Cornell box's secondary rays.
 // The boxes are the fused walk's, so at least the leaves of the plain walk are tested;
-// a near tie and a ray outside the fused arithmetic go to the plain walk.
+// ties and rays outside the fused arithmetic go to the plain walk.
 //   renders  16 nodes (a bit per child): a Cornell box, where a ray enters most of the
 //            few boxes, 5.06 -> 4.78 ms (64 samples, 256 x 256)
 //   casts    4 nodes (closest / any hits in Grays/s, tree walk -> boxes first, rays from
@@ -277,7 +290,7 @@ template <bool ANY, bool WT>
 __global__ void __launch_bounds__(kFlatThreads, kFlatBlocks)
 k_trace_flat(DevScene scene, int nnodes, const float4* __restrict__ rays, int n_static, const int* __restrict__ n_dev,
              bg_hit* __restrict__ hits, uint8_t* __restrict__ occ, ShadowResolve res) {
-    __shared__ float4 own[2][kFlatThreads];
+    __shared__ float4 own[3][kFlatThreads];
     __shared__ int2 sstack[8][kFlatThreads];
     int2 lstack[kStackSize - 8];
     TraceScene S;
@@ -337,7 +350,9 @@ k_trace_flat(DevScene scene, int nnodes, const float4* __restrict__ rays, int n_
                 if (trav_leaf<ANY, false>(S, s, s.item, none)) break;
             }
         }
-        if (s.r.flags & (kPlainWalk | kNearTie)) {
+        if ((s.r.flags & (kPlainWalk | kTie)) ||
+            (s.prim >= 0 && !plain_reaches<WT>(scene, __float_as_int(S.own[2 * kFlatThreads].x), s.prim,
+                                               ANY ? S.own[2 * kFlatThreads].y : s.best, &ra.x, s.r.inv, ra.w))) {
             const RayStack<8> stack{&sstack[0][threadIdx.x], lstack, kFlatThreads};
             TravState<WT, kWalkPlain> q;
             trav_init(q, S, kPlainWalk, ra, rb, idx, 0);

@@ -21,10 +21,15 @@
 //   packed one fused multiply-add per plane with a per-ray bound of the roundings,
 //          on the 64-byte QNode4 nodes, on the 128-byte nodes (fused) or on the
 //          8-wide nodes, slack 1e-5.  Its boxes contain the plain ones, its order
-//          differs in detail.  A closest-hit ray that ends with a second triangle
-//          within 1e-5 (relative) of its closest t is walked again on the plain
-//          nodes, so ids, t, u and v are those of the plain walk, ties included;
-//          an any-hit answer does not depend on the order.
+//          differs in detail.  The plain walk decides, by a second walk of the ray on
+//          the plain nodes, when two triangles share the closest t to the last bit and
+//          when it might not come to the triangle that was hit (plain_reaches).  So an
+//          any-hit answer is that of the plain walk, and so are ids, t, u and v, ties
+//          included, unless the rounding of a triangle's t takes it in front of the
+//          triangle's own box by more than 1e-5 of t: whether such a triangle hides a
+//          surface within that distance behind it depends on which the walk comes to
+//          first.  (t rounds by at most 12 x 2^-24 (t + 2 edges) / c, c = sine of the corner
+//          x cosine of incidence: for triangles small against t, c above 0.07 rules it out.)
 // Rays the packed arithmetic does not cover (a direction component of 0 or out
 // of range, not finite) take the plain walk from the start, as does the
 // instrumented replay (COUNT).
@@ -75,18 +80,19 @@ constexpr float kBoxSlack = 4e-7f;
 // is huge for rays nearly parallel to an axis, so such rays visited most of the
 // tree: C3 ran at 8 instead of 500 Msamples/s.)
 
-// Slack of the packed walk: its box tests, its culling of popped entries and
-// the distance within which a second hit sends the ray to the plain walk.
+// Slack of the packed walk: its box tests and its culling of popped entries.
 constexpr float kFastSlack = 1e-5f;
 
 // Ray::flags: bits 0-2 sign of 1/d per axis
 constexpr uint32_t kOctMask = 7u;
 constexpr uint32_t kPlainWalk = 8u;   // walk the plain nodes
-constexpr uint32_t kNearTie = 16u;    // packed walk: a second triangle near the closest one, or a hit by an edge
+constexpr uint32_t kTie = 16u;        // packed walk: two triangles at the closest t, or no room on the stack
 
 // kWalkPacked and kWalkFused keep the ray's origin and direction, which they need
 // only for a new bundle's object-space ray and for a plain visit, in shared memory:
 // six registers less during the walk (from global memory, C3 was 3 % slower).
+template <int WALK>
+constexpr bool kKeeps = WALK == kWalkPacked || WALK == kWalkFused;
 struct RayFast {
     v3 inv;          // 1 / d
     v3 cn, cf;       // -o / d less / plus a bound of the roundings: near / far planes
@@ -111,7 +117,9 @@ struct Ray<kWalkPlain> {
 // the scene and the ray array of one launch
 struct TraceScene : DevScene {
     const float4* rays;
-    float4* own;      // this lane's ray in shared memory (kWalkPacked, kWalkFused): o at own[0], d at own[ownstep]
+    // kWalkPacked, kWalkFused: this lane's in shared memory, its ray at own[0] and
+    // own[ownstep], its closest hit's TriRec and (any hit) t at own[2 ownstep]
+    float4* own;
     int ownstep;
 };
 
@@ -281,13 +289,52 @@ __device__ __forceinline__ bool wt_test(const ObjRayWT& c, v3 p1, v3 p2, v3 p3, 
     return true;
 }
 
-// Whether a hit at barycentrics a, b lies by an edge of its triangle.  The true hit may
-// then lie outside the triangle and its boxes by the test's rounding, where the plain
-// walk's box test can cull it (a ray along a wall, from the border of the box): the other
-// walks, with wider boxes, ask the plain one.  (18 of 671M rays inside a Cornell box
-// differed without this, none with it.  A bound from the operands' sizes instead of a
-// constant cost casts 4-12 %.)
-__device__ __forceinline__ bool near_edge(float a, float b) { return !(min3(a, b, 1.f - a - b) > 1e-4f); }
+// Whether the plain walk comes to the triangle of a hit at t that another walk, with wider
+// boxes, has found: the plain box test, with t as the closest hit so far, of a box inside the
+// triangle's own.  Every box that holds the triangle has its planes at least as far out, the
+// plain walk's closest hit is never closer (what it tests, the other walk has tested), and
+// subtraction, multiplication, minimum and maximum round monotonously: if the plain test lets
+// this box pass, it lets all those pass.  (Without it a ray by an edge, or to a point on a
+// surface, got other answers from other walks: the rounding of the triangle's test grows with
+// distance over edge length and with incidence, and takes the true hit out of the box.)
+// Moller-Trumbore's record holds p2 - p1, rounded, not p2.  A little less of it, added to p1,
+// comes out between p1 and p2, as the rounding of a sum is monotone and p2 a float.
+// Once per ray, at its end: casts are 0-4 % slower with it (1M-triangle soup, closest /
+// any incoherent 1400 / 1797 -> 1409 / 1800 Mrays/s, any coherent 3845 -> 3680), a 6M-triangle
+// frame 29.0 -> 29.8 ms.  Also measured: bounds of the test's rounding instead, at every hit
+// casts 4-12 % slower, at the ray's end (the plain walk for what they leave open) C3 44.6 ms;
+// a call out of line C3 31.6 ms.
+template <bool WT>
+__device__ __forceinline__ bool plain_reaches(const DevScene& S, int tri, int prim, float t, const float* o, v3 inv, float tmin) {
+    const float* f = reinterpret_cast<const float*>(S.tris + tri);
+    const int bundle = __float_as_int(__ldg(f + 3));
+    float t0 = tmin, t1 = t;
+    auto axis = [&](int k, float i) {
+        float x, y, z;
+        if (bundle >= 0) {
+            const float* m = S.bundles[bundle].m + 4 * k;
+            const float* c = reinterpret_cast<const float*>(S.shade + (prim & kPrimMask));   // the corners themselves
+            x = __ldg(m) * __ldg(c) + __ldg(m + 1) * __ldg(c + 1) + __ldg(m + 2) * __ldg(c + 2) + __ldg(m + 3);
+            y = __ldg(m) * __ldg(c + 4) + __ldg(m + 1) * __ldg(c + 5) + __ldg(m + 2) * __ldg(c + 6) + __ldg(m + 3);
+            z = __ldg(m) * __ldg(c + 8) + __ldg(m + 1) * __ldg(c + 9) + __ldg(m + 2) * __ldg(c + 10) + __ldg(m + 3);
+        } else {
+            x = __ldg(f + k);
+            y = __ldg(f + 4 + k);
+            z = __ldg(f + 8 + k);
+            if (!WT) {
+                y = fmaf(y, 1.f - 0x1p-20f, x);
+                z = fmaf(z, 1.f - 0x1p-20f, x);
+            }
+        }
+        const float s0 = (min3(x, y, z) - o[k]) * i, s1 = (max3(x, y, z) - o[k]) * i;
+        t0 = fmaxf(t0, fminf(s0, s1));
+        t1 = fminf(t1, fmaxf(s0, s1));
+    };
+    axis(0, inv.x);
+    axis(1, inv.y);
+    axis(2, inv.z);
+    return t0 <= fmaf(fabsf(t1), kBoxSlack, t1);
+}
 
 // entry distance of a child that is not hit: +inf
 #define kMiss __int_as_float(0x7f800000)
@@ -672,7 +719,7 @@ __device__ __forceinline__ bool trav_node(const TraceScene& S, TravState<WT, WAL
         // (the commit has checked that no walk needs more than kStackSize entries; the packed
         // boxes can only let in an empty slot besides)
         if (s.sp + 3 > kStackSize) {
-            s.r.flags |= kNearTie;   // no room to spare: the plain walk decides
+            s.r.flags |= kTie;   // no room to spare: the plain walk decides
             return false;
         }
 #pragma unroll
@@ -702,34 +749,22 @@ __device__ __forceinline__ bool trav_leaf(const TraceScene& S, TravState<WT, WAL
     float4 v0 = __ldg(tp), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
     if (COUNT) ++cnt.tris;
     obj_ray(S, s.r, __float_as_int(v0.w), s.cache);
-    // packed walk: a hit just beyond the closest one is found too (near tie)
-    const bool margin = WALK != kWalkPlain && !ANY && s.prim >= 0 && !(s.r.flags & kPlainWalk);
-    const float tmax = margin ? s.cull : s.best;
     float t, a, b;
     bool hit;
     if constexpr (WT)
-        hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin, tmax, t, a, b);
+        hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin, s.best, t, a, b);
     else
         hit = mt_test(s.cache.o, s.cache.d, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z),
-                      s.r.tmin, tmax, t, a, b);
+                      s.r.tmin, s.best, t, a, b);
     if (hit) {
-        const bool edge = WALK != kWalkPlain && !(s.r.flags & kPlainWalk) && near_edge(a, b);
-        if (ANY && edge) {   // an occluder if another one is found or the plain walk finds it
-            s.r.flags |= kNearTie;
-            return false;
-        }
-        if (margin) {
-            // near the hit it replaces (or is replaced by): a tie; clearly closer: none any more
-            if (t < fmaf(fabsf(s.best), -kFastSlack, s.best)) s.r.flags &= ~kNearTie;
-            else s.r.flags |= kNearTie;
-            if (t > s.best) return false;
-        }
+        if (kKeeps<WALK> && !ANY && !(s.r.flags & kPlainWalk))   // (at tmax: a tie too, asked once more)
+            s.r.flags = t == s.best ? s.r.flags | kTie : s.r.flags & ~kTie;
         s.prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
-        if (ANY) {
-            s.r.flags &= ~kNearTie;
-            return true;
+        if (kKeeps<WALK>) {
+            S.own[2 * S.ownstep].x = __int_as_float(start);
+            if (ANY) S.own[2 * S.ownstep].y = t;
         }
-        if (edge) s.r.flags |= kNearTie;
+        if (ANY) return true;
         s.best = t; s.u = a; s.v = b;
         s.cull = trav_cull(s, t);
     }
@@ -768,7 +803,7 @@ __device__ __forceinline__ bool trav_steps(const TraceScene& S, TravState<WT, WA
 // many steps as the tree has levels; it visits more nodes than the serial walk,
 // as entries are popped before nearer hits have culled them.
 // The answer is that of the packed walk: an any-hit answer and the closest t do
-// not depend on the order, and a closest hit with another one near it, a ray
+// not depend on the order, and a closest hit with another one at the same t, a ray
 // outside the packed arithmetic and a group whose stack runs full (8 entries
 // per lane) are walked again serially on the plain nodes by the group's first
 // lane.
@@ -813,7 +848,8 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
     r.redo = live && (s.r.flags & kPlainWalk) != 0;
     float best = s.best;      // the group's closest t, and the lane that holds it
     int owner = -1;
-    bool near = false;
+    bool tie = false;
+    int found = 0;            // (owner) TriRec of its hit
     int count = live && !r.redo ? 1 : 0;
     if (count && g == 0) entry(0) = make_int2(root, __float_as_int(s.r.tmin));
     __syncwarp();
@@ -830,13 +866,11 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
         }
         if (count > 0) count -= k;
         const float cull = fmaf(fabsf(best), kFastSlack, best);
-        const float bound = owner >= 0 ? cull : best;   // hits just beyond the closest are found too
         if (!ANY && entry_t > cull) item = kNone;
         float ht[4];
         int hc[4], npush = 0;
         float t = 0.f, u = 0.f, v = 0.f;
-        int prim = -1;
-        bool edge = false;
+        int prim = -1, tri = 0;
         if (item >= 0 && item != kNone) {   // (kNone: none, culled, or an empty slot)
             box4_packed(S.qnodes, item, s.r, cull, ht, hc);
             sort4(ht, hc);
@@ -859,32 +893,34 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
             obj_ray(S, s.r, __float_as_int(v0.w), s.cache);
             bool hit;
             if constexpr (WT)
-                hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin, bound, t, u, v);
+                hit = wt_test(s.cache, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin, best, t, u, v);
             else
                 hit = mt_test(s.cache.o, s.cache.d, mk(v0.x, v0.y, v0.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), s.r.tmin,
-                              bound, t, u, v);
-            edge = hit && near_edge(u, v);
-            if (hit && !(ANY && edge)) prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
+                              best, t, u, v);
+            if (hit) prim = __float_as_int(e1.w) | (__float_as_int(e2.w) << kClassShift);
+            tri = start;
         }
-        const unsigned hits = __ballot_sync(kFull, prim >= 0), edges = __ballot_sync(kFull, edge) & gmask;
-        if (ANY && edges) near = true;
+        const unsigned hits = __ballot_sync(kFull, prim >= 0);
         if (hits) {
             if (ANY) {
-                if (hits & gmask) { r.prim = 0; owner = base; count = 0; npush = 0; }
+                if (hits & gmask) {
+                    owner = __ffs(hits & gmask) - 1;
+                    if (base + g == owner) { r.t = t; r.u = u; r.v = v; r.prim = prim; found = tri; }
+                    count = 0;
+                    npush = 0;
+                }
             } else {
                 float m = prim >= 0 ? t : kMiss;
                 for (int o = G >> 1; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(kFull, m, o));
-                const unsigned close = __ballot_sync(kFull, prim >= 0 && !(t > fmaf(fabsf(m), kFastSlack, m))) & gmask;
                 const unsigned at = __ballot_sync(kFull, prim >= 0 && t == m) & gmask;
                 if (hits & gmask) {
                     if (owner < 0 || m < best) {
-                        near = (owner >= 0 && !(m < fmaf(fabsf(best), -kFastSlack, best))) || __popc(close) > 1;
+                        tie = __popc(at) > 1;
                         best = m;
                         owner = __ffs(at) - 1;
-                        near = near || ((edges >> owner) & 1u);
-                        if (base + g == owner) { r.t = t; r.u = u; r.v = v; r.prim = prim; }
+                        if (base + g == owner) { r.t = t; r.u = u; r.v = v; r.prim = prim; found = tri; }
                     } else {
-                        near = true;
+                        tie = true;      // (m = best)
                     }
                 }
             }
@@ -899,7 +935,11 @@ __device__ __forceinline__ CoopHit coop_walk(const TraceScene& S, bool live, int
         count += __popc(b0 & gmask) + 2 * __popc(b1 & gmask) + 4 * __popc(b2 & gmask);
         __syncwarp();
     }
-    if (near && (!ANY || owner < 0)) r.redo = true;
+    bool unsure = false;
+    if (owner >= 0 && base + g == owner)
+        unsure = !plain_reaches<WT>(S, found, r.prim, r.t, &s.r.o.x, s.r.inv, s.r.tmin);
+    const unsigned doubts = __ballot_sync(kFull, unsure) & gmask;   // (all lanes, tie or not)
+    if (tie || doubts) r.redo = true;
     r.writer = live && !r.redo && base + g == (owner >= 0 ? owner : base);
     r.redo = r.redo && g == 0;
     return r;

@@ -1,13 +1,14 @@
 """Every other walk against the plain one, where rounding decides.
 
-The plain walk is had by itself: a scene committed with no room for its packed nodes
-casts on it at every size.
+The plain walk is had by itself in two ways: a scene committed with no room for its
+packed nodes casts on it at every size, and a batch that also holds a scene 4e15 units
+across renders on it, with node arrays that are copies of the scenes' own.
 """
 import numpy as np
 import pytest
 
 from banshee_b200 import abi, scenes
-from banshee_b200.scene import Mesh, Scene, lambert
+from banshee_b200.scene import Mesh, Scene, camera, environment_light, lambert
 
 pytestmark = pytest.mark.gpu
 
@@ -66,6 +67,33 @@ def _scene(tri, moved):
     return sc
 
 
+def _edge_rays(tri, n, seed):
+    """Rays at the edges of the triangles, by up to a thousandth of an edge inside or out, from 10 to 100,000
+    edges away, most of them grazing; a quarter ends at the triangle by a few roundings more or less."""
+    rng = np.random.default_rng(seed)
+    t = tri[rng.integers(0, len(tri), n)].astype(np.float64)
+    t = np.take_along_axis(t, rng.permuted(np.tile(np.arange(3), (n, 1)), axis=1)[:, :, None], 1)
+    w = rng.random((n, 1))
+    out = np.where(rng.random((n, 1)) < 0.5, -1, 1) * 10.0 ** rng.uniform(-7, -3, (n, 1))
+    p = (t[:, 0] * w + t[:, 1] * (1 - w)) * (1 - out) + t[:, 2] * out
+    nrm = np.cross(t[:, 1] - t[:, 0], t[:, 2] - t[:, 0])
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    d = rng.normal(size=(n, 3))
+    d -= (d * nrm).sum(1, keepdims=True) * nrm
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    d += nrm * 10.0 ** rng.uniform(-4, 0.5, (n, 1)) * rng.choice([-1, 1], (n, 1))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    dist = np.linalg.norm(t[:, 1] - t[:, 0], axis=1, keepdims=True) * 10.0 ** rng.uniform(1, 5, (n, 1))
+    r = np.zeros(n, abi.RAY_DTYPE)
+    r["o"], r["d"], r["tmin"] = p - d * dist, d, 0.0
+    o, d = r["o"].astype(np.float64), r["d"].astype(np.float64)
+    along = ((p - o) * d).sum(1) / (d * d).sum(1)
+    r["tmax"] = np.where(rng.random(n) < 0.25, along * (1 + rng.integers(-8, 9, n) * 2.0 ** -24), 1e30)
+    near = rng.random(n) < 0.1
+    r["tmin"] = np.where(near, along * (1 + rng.integers(-8, 9, n) * 2.0 ** -24), 0.0)
+    return r
+
+
 def _cast(gs, dev, lo, hi):
     import torch
     h = torch.full((hi - lo, 4), -5.0, device="cuda")
@@ -88,6 +116,26 @@ def _same(full, tight, rays, piece, most=0.98):
             got, occ = _cast(full, dev, lo, min(n, lo + size))
             assert (got == want[lo:lo + size]).all(), (size, np.nonzero((got != want[lo:lo + size]).any(1))[0][:5] + lo)
             assert (occ == wocc[lo:lo + size]).all(), (size, np.nonzero(occ != wocc[lo:lo + size])[0][:5] + lo)
+
+
+@pytest.mark.parametrize("moved", [False, True], ids=["identity", "transformed"])
+@pytest.mark.parametrize("intersect", [0, 1], ids=["moller", "watertight"])
+def test_rays_at_the_edges_of_small_triangles(ctx, intersect, moved):
+    tri = _small_triangles(3000, 31)
+    sc = _scene(tri, moved)
+    full, tight = _plain_twin(ctx, sc, dict(intersect=intersect))
+    world = sc.meshes[0].world_vertices().reshape(-1, 3, 3)
+    for seed in range(6):
+        _same(full, tight, _edge_rays(world, 1 << 20, 40 + seed), 2000)
+
+
+@pytest.mark.parametrize("intersect", [0, 1], ids=["moller", "watertight"])
+@pytest.mark.parametrize("name", ["grid", "ties"])
+def test_ties_and_shared_edges(ctx, name, intersect):
+    from tests.test_walks_gpu import _rays, _scene as walks_scene
+    sc, builder = walks_scene(name)
+    full, tight = _plain_twin(ctx, sc, dict(builder=builder, intersect=intersect))
+    _same(full, tight, _rays(LARGE, 51), 3001)
 
 
 # Slivers in planes of constant x and rays from the other side of the scene whose tmin lies just
@@ -119,3 +167,45 @@ def test_hits_just_behind_tmin(ctx):
     r = np.zeros(len(v), abi.RAY_DTYPE)
     r["o"], r["d"], r["tmin"], r["tmax"] = v[:, 9:12], v[:, 12:15], v[:, 15], 1e30
     _same(full, tight, np.repeat(r, LARGE // len(v) // 32 * 32), 0, most=1.0)
+
+
+def _huge():
+    """One triangle 4e15 units away: a batch with it renders on the plain walk."""
+    sc = scenes.production(8, 8, nterrain=4, nspheres=0, sphere_seg=4, seed=1)
+    v = sc.meshes[0].vertices.reshape(-1, 3)
+    v[sc.meshes[0].vidx.reshape(-1, 3)[0]] = np.float32(4e15)
+    return sc
+
+
+def _far_grid(height, n=48):
+    """A grid of small quads seen from `height` quads above: camera rays at its vertices and edges."""
+    from tests.test_walks_gpu import _grid
+    sc = _grid(n)
+    sc.lights = [environment_light((1.0, 0.9, 0.8))]
+    h = height / n
+    sc.camera = camera((0.5, 0.5, 0.25 + h), (0.5, 0.5, 0.0), (0, 1, 0), 1e-4, 1e6, float(np.degrees(2 * np.arctan(0.6 / h))), 1.0)
+    return sc
+
+
+RENDERS = {"cornell": lambda: scenes.cornell(64, 64),
+           "production": lambda: scenes.production(64, 64, nterrain=40, nspheres=6, sphere_seg=12, seed=3),
+           "grid from 30 quads": lambda: _far_grid(30), "grid from 30,000 quads": lambda: _far_grid(30_000)}
+
+
+@pytest.mark.parametrize("width", [4, 8])
+@pytest.mark.parametrize("name", list(RENDERS))
+def test_renders_on_every_walk(ctx, name, width):
+    """48 x 48 paths (groups of lanes), 640 x 384 (fused, boxes-first or 8-wide packed walk)."""
+    import torch
+    from banshee_b200 import capi
+    gs = capi.GpuScene(ctx, RENDERS[name](), node_width=width)
+    plain = capi.Batch(ctx, [gs, capi.GpuScene(ctx, _huge(), node_width=width)])
+    for w, h, spp in ((48, 48, 1), (640, 384, 2)):
+        for tracer in (abi.BG_TRACER_GI, abi.BG_TRACER_AO):
+            kw = dict(tracer=tracer, ao_radius=0.5)
+            want, got = torch.zeros((h, w, 4), device="cuda"), torch.zeros((h, w, 4), device="cuda")
+            plain.render([dict(scene=0, width=w, height=h, spp=spp, seed=4, accum_dev=want.data_ptr())], maxdepth=4, **kw)
+            gs.render(got.data_ptr(), w, h, spp, seed=4, maxdepth=4, stats=False, **kw)
+            torch.cuda.synchronize()
+            assert want[..., :3].max() > 0
+            assert (got.view(torch.int32) == want.view(torch.int32)).all(), (w, tracer)
