@@ -246,7 +246,7 @@ k_trace_coop(DevScene scene, const float4* __restrict__ rays, int n_static, cons
     static_cast<DevScene&>(S) = scene;
     S.rays = rays;
     const int n = n_dev ? *n_dev : n_static;
-    const int G = max(8, coop_group(n, warps));
+    const int G = coop_group(n, warps);
     const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5), per = 32 / G, base = lane & ~(G - 1);
     const int step = int(gridDim.x) * (kCoopThreads / 32) * per;
     for (int first = (int(blockIdx.x) * (kCoopThreads / 32) + warp) * per; first < n; first += step) {
@@ -480,9 +480,21 @@ static void launch_layout(bg_scene* s, bool render, bool any_hit, const float4* 
     else launch_width<4, false>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
 }
 
-// Whether a launch of at most n rays goes to groups of lanes (k_trace_coop).
-static bool groups_walk(const bg_scene* s, int64_t n) {
-    return s->dev.width == 4 && packed_walk<4>(s->dev) && coop_group(n, s->ctx->num_sms * kCoopBlocks * (kCoopThreads / 32)) != 0;
+// Whether a launch of at most n rays goes to groups of lanes (k_trace_coop): up to so many
+// rays per warp of its grid.  A group takes eight lanes' time for a ray and saves the depth of
+// the tree, so the line rises with the triangles.  Casts, 8 lanes per ray against one (us,
+// incoherent closest hits, on either side of the line): Cornell box, 11,840 rays 16.6 / 18.6,
+// 23,680 24.5 / 19.4; 1,000 triangles, 23,680 20.5 / 22.3, 32,768 26.5 / 23.8; 20,000, 47,360
+// 62 / 70, 65,536 79 / 77; 1M, 94,720 246 / 295, 131,072 321 / 327.  A render's bound is the
+// longest its queues can get, and most are far shorter (92,416 paths of 40,000 / 800,000
+// triangles: 408 / 529 us, one lane per ray 447 / 596), except where boxes come first
+// (k_trace_flat, Cornell box: 25,600 paths 208 us in groups, 192 there).
+static bool groups_walk(const bg_scene* s, int64_t n, bool long_bound) {
+    if (s->dev.width != 4 || !packed_walk<4>(s->dev)) return false;
+    int l = 0;                           // log2 of the triangles, rounded up
+    while ((int64_t(1) << l) < s->dev.ntris) ++l;
+    const int per = long_bound ? kCoop8 : s->dev.ntris < 64 ? 4 : std::min(kCoop8, std::max(8, l * l / 12));
+    return n <= int64_t(s->ctx->num_sms) * kCoopBlocks * (kCoopThreads / 32) * per;
 }
 
 int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
@@ -497,7 +509,10 @@ int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static
     // at most `n_most` rays, few enough for groups of lanes
     const int64_t most = n_dev ? n_most : n_static;
     const int warps = s->ctx->num_sms * kCoopBlocks * (kCoopThreads / 32);
-    if (!counters && most > 0 && groups_walk(s, most)) {
+    const bool small = !counters && !roots && s->dev.width == 4 && packed_walk<4>(s->dev) && s->nnodes4 <= (n_dev ? kFlatNodes : kFlatNodesCast);
+    const bool few = !counters && most > 0 && groups_walk(s, most, n_dev && !small);
+    const bool flat = small && !err_out && !(n_dev && few);   // (casts: 16,384 rays of one triangle 9.2 us, 9.9 in groups)
+    if (few && !flat) {
         const int grid = int(std::min<int64_t>(s->ctx->num_sms * kCoopBlocks, (most * coop_group(most, warps) + kCoopThreads - 1) / kCoopThreads));
         auto go = [&](auto kernel) { kernel<<<grid, kCoopThreads, 0, st>>>(s->dev, rays, int(n_static), n_dev, hits, occ, roots, res, warps, err_out); };
         const bool wt = s->dev.watertight != 0;
@@ -506,7 +521,6 @@ int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static
         BG_CUDA(cudaGetLastError());
         return BG_OK;
     }
-    const bool flat = !counters && !roots && s->dev.width == 4 && packed_walk<4>(s->dev) && s->nnodes4 <= (n_dev ? kFlatNodes : kFlatNodesCast);
     if (!work && !flat) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
     // ray indices are 32-bit in the kernel: a larger array goes in pieces
     // (counting replays keep one output per ray replayed: pieces are whole strides)
@@ -1106,7 +1120,7 @@ static int host_cast(bg_scene* s, const bg_ray* rays, void* out, int64_t n, bool
     char* hp = static_cast<char*>(c->pinned);
     memcpy(hp, rays, rb);
     memset(hp + rb + ob16, 0, sizeof(unsigned));
-    if (n <= kHostInPlace && groups_walk(s, n)) {
+    if (n <= kHostInPlace && groups_walk(s, n, false)) {
         // the kernel reads the rays from the pinned staging and writes the results and
         // the error word there: one launch and no copies
         rc = launch_trace(s, any, reinterpret_cast<const float4*>(hp), n, nullptr, any ? nullptr : reinterpret_cast<bg_hit*>(hp + rb),

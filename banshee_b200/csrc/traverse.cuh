@@ -809,17 +809,13 @@ __device__ __forceinline__ bool trav_steps(const TraceScene& S, TravState<WT, WA
 // lane.
 // (Measured and rejected: four lanes per entry, one per child or triangle: fewer
 // instructions per step, but a quarter of the entries: 4,096 rays 63 us, not 33.)
-// Rays per warp of the grid (2,960 warps on 148 SMs) up to which 32 / 8 lanes walk a
-// ray.  100k-triangle soup, incoherent closest / any, one lane per ray against
-// groups: 256 rays 116 / 90 -> 21 / 22 us, 4,096 127 / 92 -> 32 / 29, 16,384 144 / 100
-// -> 50 / 44, 65,536 169 / 121 -> 131 / 110.  8 lanes at 256 rays 31 / 28, 32 lanes at
-// 16,384 rays 79 / 78.
+// Rays per warp of the grid (2,960 warps on 148 SMs) up to which 32 lanes walk a ray, and
+// the most up to which 8 do (groups_walk says where).  100k-triangle soup, incoherent closest,
+// 32 / 8 lanes: 256 rays 14 / 21 us, 1,024 14 / 24, 2,960 19 / 25, 4,096 25 / 27, 16,384 72 / 46.
 constexpr int kCoop32 = 1, kCoop8 = 32;
 
-// Lanes per ray of a launch of n rays on a grid of `warps` warps; 0: too many rays for groups.
-__host__ __device__ __forceinline__ int coop_group(int64_t n, int warps) {
-    return n <= int64_t(warps) * kCoop32 ? 32 : n <= int64_t(warps) * kCoop8 ? 8 : 0;
-}
+// Lanes per ray of a launch of n rays on a grid of `warps` warps.
+__host__ __device__ __forceinline__ int coop_group(int64_t n, int warps) { return n <= int64_t(warps) * kCoop32 ? 32 : 8; }
 
 struct CoopHit {
     float t, u, v;
