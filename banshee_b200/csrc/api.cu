@@ -352,10 +352,10 @@ k_trace_flat(DevScene scene, int nnodes, const float4* __restrict__ rays, int n_
         }
         if ((s.r.flags & (kPlainWalk | kTie)) ||
             (s.prim >= 0 && !plain_reaches<WT>(scene, __float_as_int(S.own[2 * kFlatThreads].x), s.prim,
-                                               ANY ? S.own[2 * kFlatThreads].y : s.best, &ra.x, s.r.inv, ra.w))) {
+                                               ANY ? S.own[2 * kFlatThreads].y : s.best, &S.own[0].x, s.r.inv, s.r.tmin))) {
             const RayStack<8> stack{&sstack[0][threadIdx.x], lstack, kFlatThreads};
             TravState<WT, kWalkPlain> q;
-            trav_init(q, S, kPlainWalk, ra, rb, idx, 0);
+            trav_init(q, S, kPlainWalk, S.own[0], S.own[kFlatThreads], idx, 0);
             while (!trav_steps<ANY, false, 4>(S, q, stack, 64, false, none)) {}
             trace_emit<ANY>(res, hits, occ, idx, q.prim, q.best, q.u, q.v);
         } else {

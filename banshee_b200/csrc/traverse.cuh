@@ -30,8 +30,8 @@
 //          surface within that distance behind it depends on which the walk comes to
 //          first.  (t rounds by at most 12 x 2^-24 (t + 2 edges) / c, c = sine of the corner
 //          x cosine of incidence: for triangles small against t, c above 0.07 rules it out.)
-// Rays the packed arithmetic does not cover (a direction component of 0 or out
-// of range, not finite) take the plain walk from the start, as does the
+// Rays the packed arithmetic does not cover (components out of its range, not
+// finite) take the plain walk from the start, as does the
 // instrumented replay (COUNT).
 #pragma once
 
@@ -82,6 +82,7 @@ constexpr float kBoxSlack = 4e-7f;
 
 // Slack of the packed walk: its box tests and its culling of popped entries.
 constexpr float kFastSlack = 1e-5f;
+constexpr float kZeroInv = 2e15f;    // its 1 / d for a component of 0
 
 // Ray::flags: bits 0-2 sign of 1/d per axis
 constexpr uint32_t kOctMask = 7u;
@@ -149,11 +150,22 @@ __device__ __forceinline__ void make_ray(RayFast& r, float extent, uint32_t walk
     r.idx = idx;
     r.tmin = a.w;
     r.inv = mk(1.f / b.x, 1.f / b.y, 1.f / b.z);
-    const v3 ai = mk(fabsf(r.inv.x), fabsf(r.inv.y), fabsf(r.inv.z));
     const float far = max3(fabsf(a.x), fabsf(a.y), fabsf(a.z));
+    const v3 ad = mk(fabsf(b.x), fabsf(b.y), fabsf(b.z));
+    // A component of 0 (a camera's middle column) counts as 5e-16 while another is 1e-8 or
+    // more and tmin is not negative: distances to its planes are then negative or beyond the
+    // scene, as with the infinite inverse, except within the bound of the roundings.
+    const bool zeros = a.w >= 0.f && max3(ad.x, ad.y, ad.z) >= 1e-8f;
     // the packed arithmetic's range (comparisons false for NaN: plain walk)
-    const bool ok = ai.x <= 1e15f && ai.y <= 1e15f && ai.z <= 1e15f && min3(ai.x, ai.y, ai.z) >= 1e-15f && far <= 1e15f;
+    auto in = [&](float x) { return x == 0.f ? zeros : x >= 1e-15f && x <= 1e15f; };
+    const bool ok = far <= 1e15f && in(ad.x) && in(ad.y) && in(ad.z);
+    if (ok && walk == 0u) {
+        if (b.x == 0.f) r.inv.x = copysignf(kZeroInv, b.x);
+        if (b.y == 0.f) r.inv.y = copysignf(kZeroInv, b.y);
+        if (b.z == 0.f) r.inv.z = copysignf(kZeroInv, b.z);
+    }
     r.flags = octant(r.inv) | (ok ? walk : kPlainWalk);
+    const v3 ai = mk(fabsf(r.inv.x), fabsf(r.inv.y), fabsf(r.inv.z));
     // the bound of the roundings: those of a plane's distance here (of the intercepts and
     // the final multiply-add) are together at most 3 x 2^-24 of (|plane| + |o|) / |d|, and the
     // plain test reaches, by its slack and its own three roundings, 7e-7 of the distance
@@ -326,6 +338,7 @@ __device__ __forceinline__ bool plain_reaches(const DevScene& S, int tri, int pr
                 z = fmaf(z, 1.f - 0x1p-20f, x);
             }
         }
+        if (fabsf(i) == kZeroInv) i = copysignf(__int_as_float(0x7f800000), i);   // the plain walk's 1 / 0
         const float s0 = (min3(x, y, z) - o[k]) * i, s1 = (max3(x, y, z) - o[k]) * i;
         t0 = fmaxf(t0, fminf(s0, s1));
         t1 = fminf(t1, fmaxf(s0, s1));

@@ -169,6 +169,37 @@ def test_hits_just_behind_tmin(ctx):
     _same(full, tight, np.repeat(r, LARGE // len(v) // 32 * 32), 0, most=1.0)
 
 
+@pytest.mark.parametrize("intersect", [0, 1], ids=["moller", "watertight"])
+@pytest.mark.parametrize("name", ["grid", "soup", "small triangles"])
+def test_rays_along_an_axis_plane(ctx, name, intersect):
+    """One or two direction components are 0 or -0; a third of the origins lie on planes of the scene."""
+    from tests.test_walks_gpu import _scene as walks_scene
+    tri = _small_triangles(3000, 31, 0.02)
+    sc, builder = (_scene(tri, False), 0) if name == "small triangles" else walks_scene(name)
+    full, tight = _plain_twin(ctx, sc, dict(builder=builder, intersect=intersect))
+    rng = np.random.default_rng(71)
+    n = 1 << 19
+    corners = sc.meshes[0].world_vertices().reshape(-1, 3)
+    r = np.zeros(n, abi.RAY_DTYPE)
+    r["o"], r["d"] = rng.random((n, 3)), rng.normal(size=(n, 3))
+    d = r["d"]
+    for k in range(2):
+        zero = np.arange(n) if k == 0 else np.arange(0, n, 3)
+        d[zero, rng.integers(0, 3, len(zero))] = rng.choice(np.float32([0, -0.0]), len(zero))
+    d[(d == 0).all(1)] = (0, 1, 0)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    i = np.arange(0, n, 2)
+    hit = corners[rng.integers(0, len(corners), len(i))] + 1e-3 * rng.normal(size=(len(i), 3))
+    on = np.arange(len(i)) % 3 == 0
+    hit[on] = corners[rng.integers(0, len(corners), on.sum())]
+    r["o"][i] = hit - d[i] * rng.random((len(i), 1))
+    flat = d[i] == 0
+    r["o"][i] = np.where(flat, hit, r["o"][i])
+    r["tmax"] = np.where(np.arange(n) % 4 == 3, rng.random(n), 8.0)
+    r["tmin"] = np.where(np.arange(n) % 16 == 5, -0.25, 0.0)
+    _same(full, tight, r, 2500)
+
+
 def _huge():
     """One triangle 4e15 units away: a batch with it renders on the plain walk."""
     sc = scenes.production(8, 8, nterrain=4, nspheres=0, sphere_seg=4, seed=1)

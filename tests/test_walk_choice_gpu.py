@@ -50,3 +50,20 @@ def test_fewer_rays_take_no_longer(ctx, tris, kind):
             times.append(_us(lambda: cast(rays.data_ptr(), out.data_ptr(), n)))
         for i, t in enumerate(times):
             assert t <= 1.4 * min(times[i:]), (occlusion, [round(x, 1) for x in times])
+
+
+def test_rays_of_a_middle_column_take_no_longer(ctx):
+    """A camera of odd width has rays whose x component is exactly 0."""
+    import torch
+    from banshee_b200 import capi
+    gs = capi.GpuScene(ctx, scenes.soup(100_000, seed=3), builder=3)
+    for side in (91, 363):
+        times = []
+        for w in (side, side + 1):
+            n = w * w
+            rays = scenes.soup_rays(n, "coherent", seed=61)
+            assert (rays["d"][:, 0] == 0).any() == (w == side)
+            dev = torch.from_numpy(rays.view("u1").reshape(n, 32)).cuda()
+            out = torch.zeros((n, 16), dtype=torch.uint8, device="cuda")
+            times.append(_us(lambda: gs.intersect_closest(dev.data_ptr(), out.data_ptr(), n)))
+        assert times[0] <= 1.25 * times[1], times
