@@ -373,7 +373,8 @@ __device__ __forceinline__ void sort4(float (&t)[4], int32_t (&c)[4]) {
 // one that is not hit.  A ray with infinite direction components can enter an empty
 // slot (all its slabs are 0 or NaN); such a child is dropped when it is popped, or
 // here (DROP) where the walk's pops do not test for it: that test in every pop cost
-// the fused any-hit walk 5 %.  (The near / far planes of each axis are picked by load
+// the fused any-hit walk 5 % (the plain one: 100 triangles, any hits 17.2 against 17.9
+// Grays/s, 4.7 against 4.8 with 4,000).  (The near / far planes of each axis are picked by load
 // address: the node stores lo and hi of an axis in adjacent float4s.)
 struct Children4 {
     float t[4];
@@ -659,7 +660,7 @@ __device__ __forceinline__ bool trav_pop(TravState<WT, WALK>& s, const STACK& st
         const int2 e = stack.get(--s.sp);
         // the entry distance carries the box test's rounding: cull with its slack
         if (!ANY && __int_as_float(e.y) > s.cull) continue;
-        if (WALK != kWalkFused && e.x == kNone) continue;   // an empty slot (box4_packed, box4_plain)
+        if (WALK != kWalkFused && WALK != kWalkPlain && e.x == kNone) continue;   // an empty slot (box4_packed)
         item = e.x;
         return true;
     }
@@ -712,7 +713,7 @@ __device__ __forceinline__ bool trav_node(const TraceScene& S, TravState<WT, WAL
     }
     if (plain) {
         world_ray(S, s.r, o, d);
-        const Children4 h = box4_plain<WALK == kWalkFused>(reinterpret_cast<const float4*>(S.nodes + item), o, s.r.inv, s.r.flags, s.r.tmin, s.best);
+        const Children4 h = box4_plain<WALK == kWalkFused || WALK == kWalkPlain>(reinterpret_cast<const float4*>(S.nodes + item), o, s.r.inv, s.r.flags, s.r.tmin, s.best);
         if (h.nh == 0) { s.item = kNone; return true; }
         // push the farther ones (farthest first), continue with the nearest
         if (s.sp + h.nh - 1 > kStackSize) {
