@@ -375,13 +375,22 @@ k_trace_flat(DevScene scene, int nnodes, const float4* __restrict__ rays, int n_
 //   renders     fused: their rays are issue-bound (16 K to 800 K triangles: 1.83,
 //               2.14, 2.48, 2.75 ms -> 1.70, 2.02, 2.25, 2.65; packed bytes alone 5 %
 //               slower than plain).
-//   8-wide      packed: half the instructions of its decode (1000 -> 1090 incoherent
-//               closest, 1360 -> 1448 any, 2447 -> 2904 coherent any).
-constexpr int64_t kPackTriangles = 1000;
+//   8-wide      packed: half the instructions of its decode (1M-triangle soup, coherent /
+//               incoherent closest 1417 -> 1555 / 1000 -> 1060, incoherent / coherent any
+//               1360 -> 1415 / 2447 -> 2800 Mrays/s).  With fewer rays than two in three lanes a
+//               launch is as long as its slowest ray, whose second walk and longer chain show:
+//               32,768 rays of 100,000 triangles, incoherent any, 98 us on the plain walk, 107
+//               packed, 131,072 188 and 186; and below 64 triangles the bytes bring more visits
+//               (Cornell box, 1M rays, 125 and 138 us).
+constexpr int64_t kPackTriangles = 1000, kPackTriangles8 = 64;
 template <int WIDTH>
-static int choose_walk(const DevScene& d, bool render) {
+static int choose_walk(const bg_scene* s, bool render, int64_t most) {
+    const DevScene& d = s->dev;
     if (!packed_walk<WIDTH>(d)) return kWalkPlain;
-    if (WIDTH == 8) return kWalkPacked;
+    if (WIDTH == 8) {
+        const int64_t lanes = int64_t(s->trace_blocks[kWalkPacked][1][0][0][0]) * 128;
+        return d.ntris < kPackTriangles8 || most * 3 < lanes * 2 ? kWalkPlain : kWalkPacked;
+    }
     if (render) return kWalkFused;
     return d.ntris < kPackTriangles ? kWalkPlain : kWalkPacked;
 }
@@ -455,10 +464,10 @@ static void launch_walk(bg_scene* s, bool any_hit, const float4* rays, int64_t n
 }
 
 template <int WIDTH, bool WT>
-static void launch_width(bg_scene* s, bool render, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
+static void launch_width(bg_scene* s, int64_t most, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                          bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
                          unsigned long long* w, const int* roots, const ShadowResolve& res) {
-    const int walk = counters ? kWalkPlain : choose_walk<WIDTH>(s->dev, render);   // (counting replays: the plain walk)
+    const int walk = counters ? kWalkPlain : choose_walk<WIDTH>(s, n_dev != nullptr, most);   // (counting replays: the plain walk)
     if (walk == kWalkPacked)
         launch_walk<WIDTH, WT, kWalkPacked>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
     else if (walk == kWalkFused)
@@ -467,17 +476,17 @@ static void launch_width(bg_scene* s, bool render, bool any_hit, const float4* r
         launch_walk<WIDTH, WT, kWalkPlain>(s, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
 }
 
-// The traversal kernel of the scene's node layout and intersection test.
-static void launch_layout(bg_scene* s, bool render, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
+// The traversal kernel of the scene's node layout and intersection test for at most `most` rays.
+static void launch_layout(bg_scene* s, int64_t most, bool any_hit, const float4* rays, int64_t n_static, const int* n_dev,
                           bg_hit* hits, uint8_t* occ, cudaStream_t st, unsigned long long* counters, int stride,
                           unsigned long long* w, const int* roots, const ShadowResolve& res) {
     // (Measured and rejected: any-hit rays on the 8-wide nodes while closest-hit
     // rays use the 4-wide ones: the C3 shadow traversal took 16.6 instead of 13.6 ms.)
     const bool w8 = s->dev.width == 8, wt = s->dev.watertight != 0;
-    if (w8 && wt) launch_width<8, true>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
-    else if (w8) launch_width<8, false>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
-    else if (wt) launch_width<4, true>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
-    else launch_width<4, false>(s, render, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    if (w8 && wt) launch_width<8, true>(s, most, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else if (w8) launch_width<8, false>(s, most, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else if (wt) launch_width<4, true>(s, most, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
+    else launch_width<4, false>(s, most, any_hit, rays, n_static, n_dev, hits, occ, st, counters, stride, w, roots, res);
 }
 
 // Whether a launch of at most n rays goes to groups of lanes (k_trace_coop): up to so many
@@ -540,7 +549,7 @@ int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static
             continue;
         }
         if (at > 0) BG_CUDA(cudaMemsetAsync(w, 0, sizeof(unsigned long long), st));
-        launch_layout(s, n_dev != nullptr, any_hit, rays + 2 * at, std::min(n_static - at, piece), n_dev, hits ? hits + at / stride : nullptr,
+        launch_layout(s, most > 0 ? most : INT64_MAX / 4, any_hit, rays + 2 * at, std::min(n_static - at, piece), n_dev, hits ? hits + at / stride : nullptr,
                       occ ? occ + at / stride : nullptr, st, counters, stride, w, roots, res);
     }
     BG_CUDA(cudaGetLastError());
@@ -1274,7 +1283,7 @@ extern "C" int bg_traversal_counts_noalloc(bg_scene* s, const bg_ray* rays, int6
     cudaError_t e = cudaMemsetAsync(base, 0, kNoAllocHeader, st);   // counters and work counter start at zero
     if (e == cudaSuccess && n > 0) {
         const float4* r4 = reinterpret_cast<const float4*>(rays);
-        launch_layout(s, false, any_hit != 0, r4, n, nullptr, any_hit ? nullptr : hits, any_hit ? occ : nullptr, st, cnt, 1,
+        launch_layout(s, n, any_hit != 0, r4, n, nullptr, any_hit ? nullptr : hits, any_hit ? occ : nullptr, st, cnt, 1,
                       work, nullptr, ShadowResolve{nullptr, nullptr, nullptr, 0});
         e = cudaGetLastError();
     }
