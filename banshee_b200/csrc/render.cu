@@ -932,17 +932,39 @@ static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L, bool ba
     return BG_OK;
 }
 
+// Training rows that wait for their cache's next frame, and their counts.
+static void move_training(RenderState& from, RenderState& to) {
+    for (DevBuf RenderState::* b : {&RenderState::tr_feat, &RenderState::tr_target, &RenderState::counts}) std::swap(to.*b, from.*b);
+    to.tr_cap = from.tr_cap;
+    to.tr_set = from.tr_set;
+    to.pending_cache = from.pending_cache;
+    to.pending_ptr = from.pending_ptr;
+    to.pending_frame = from.pending_frame;
+}
+
 // Path state and queues for passes of `cap` paths with up to maxL lights per
-// job; a failed allocation leaves no state behind (the next call starts over).
+// job; a failed allocation leaves no state behind but rows still to be trained
+// (the next call starts over).
 static int ensure_state(bg_scene* s, int64_t cap, int maxL, bool batched) {
     const int L = std::max(1, maxL);
     if (s->render && s->render->cap >= cap && s->render->nlights == L) return BG_OK;
-    if (s->render) render_state_free(s->render);
-    s->render = new RenderState();
-    const int rc = alloc_state(s, s->render, cap, L, batched);
-    if (rc) {
+    RenderState* rs = new RenderState();
+    if (s->render) {
+        if (s->render->pending_cache != 0) {
+            BG_CUDA(cudaDeviceSynchronize());   // the rows are written
+            move_training(*s->render, *rs);
+        }
         render_state_free(s->render);
+    }
+    s->render = rs;
+    const int rc = alloc_state(s, rs, cap, L, batched);
+    if (rc) {
         s->render = nullptr;
+        if (rs->pending_cache != 0) {
+            s->render = new RenderState();
+            move_training(*rs, *s->render);
+        }
+        render_state_free(rs);
     }
     return rc;
 }

@@ -1,0 +1,47 @@
+"""What a scene keeps between renders survives a larger render."""
+import numpy as np
+import pytest
+
+from banshee_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from banshee_b200 import capi
+    return capi.Context(0)
+
+
+def _accum(w, h):
+    import torch
+    return torch.zeros((h, w, 4), device="cuda")
+
+
+@pytest.mark.parametrize("between", ["nothing", "a larger render", "a render without room"])
+def test_pending_training_rows_are_trained(ctx, between):
+    """A cached frame's rows are trained at the start of the cache's next frame, whatever
+    plain renders come between."""
+    import torch
+    from banshee_b200 import capi
+    gs = capi.GpuScene(ctx, scenes.cornell(64, 64))
+    cache = capi.RadianceCache(gs, log2_table_size=14, train_paths=1024, train_batch=2048, train_steps=4)
+    frame, big = _accum(64, 64), _accum(1920, 1088)
+    cache.render(frame.data_ptr(), 64, 64, 1, seed=1, maxdepth=5)
+    torch.cuda.synchronize()
+    before = cache.params()
+    if between == "a larger render":
+        gs.render(big.data_ptr(), 1920, 1088, 2, seed=2, maxdepth=2, stats=False)
+    elif between == "a render without room":
+        capi.alloc_limit(1 << 20)
+        try:
+            with pytest.raises(capi.BansheeError):
+                gs.render(big.data_ptr(), 1920, 1088, 2, seed=2, maxdepth=2, stats=False)
+        finally:
+            capi.alloc_limit(None)
+    cache.render(frame.data_ptr(), 64, 64, 1, seed=3, maxdepth=5)
+    torch.cuda.synchronize()
+    after = cache.params()
+    assert (before[0] != after[0]).mean() > 0.5                      # the network has been trained
+    assert 0 < (before[1] != after[1]).sum()
+    assert np.isfinite(after[0]).all() and np.isfinite(after[1]).all()
