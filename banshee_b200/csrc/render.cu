@@ -85,6 +85,8 @@ constexpr int kMaxSegs = 1024;
 
 struct RenderState {
     int64_t cap = 0;   // paths per pass
+    int64_t asked = 0; // the largest pass that a render without autotuning has asked for (default_pass)
+    bool captured = false;   // a caller's stream capture holds its pointers
     int kmax = 0;      // DI slots per path
     int nlights = 0;
     DevBuf ext_rays[2], ext_path[2], ext_hits;
@@ -1377,7 +1379,9 @@ static int64_t default_pass(bg_scene* s, int maxL, bool batched, bool capturing,
     if (most <= kPassDefault) return kPassDefault;
     if (s->render && s->render->nlights == L) {
         if (s->render->cap >= most) return kPassMost;                            // it is there already
-        if (capturing) return std::max<int64_t>(kPassDefault, s->render->cap);   // no new one while a stream is captured
+        // no new state for the size alone while a stream is captured or when one has been, nor
+        // for a call that has had its answer, even if there is more memory by now
+        if (capturing || s->render->captured || most <= s->render->asked) return std::max<int64_t>(kPassDefault, s->render->cap);
     }
     size_t free_b = 0, all_b = 0, held = 0;
     if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess) { cudaGetLastError(); return kPassDefault; }
@@ -1441,6 +1445,8 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
     }
     if (rc) return rc;
     RenderState* rs = s->render;   // buffers may be larger than this call's pass size
+    if (cap_st != cudaStreamCaptureStatusNone) rs->captured = true;
+    if (s->tune_paths == 0 && !cache) rs->asked = std::max(rs->asked, pass_of(kPassMost));
     const int maxdepth = tr->kind == BG_TRACER_GI ? tr->maxdepth : 1;
     unsigned long long* totals = reinterpret_cast<unsigned long long*>(rs->counts.as<char>() + 64);
 

@@ -45,3 +45,31 @@ def test_pending_training_rows_are_trained(ctx, between):
     assert (before[0] != after[0]).mean() > 0.5                      # the network has been trained
     assert 0 < (before[1] != after[1]).sum()
     assert np.isfinite(after[0]).all() and np.isfinite(after[1]).all()
+
+
+def test_an_unchanged_render_allocates_nothing(ctx):
+    """The pass size that a budget allowed stays when the budget has gone: a caller may hold
+    the state's memory in a graph, and the call has not changed.  A larger call may grow it."""
+    import torch
+    from banshee_b200 import capi
+    w, h = 1920, 1088
+    used = []
+    for limit in (None, 0):
+        gs = capi.GpuScene(ctx, scenes.cornell(64, 64))
+        acc = _accum(w, h)
+        before = capi.alloc_stats()["bytes"]
+        capi.alloc_limit(limit if limit is None else int(1.2 * used[0] * (1 << 21) / (w * h * 3)))
+        try:
+            gs.render(acc.data_ptr(), w, h, 3, seed=1, maxdepth=2, stats=False)
+        finally:
+            capi.alloc_limit(None)
+        torch.cuda.synchronize()
+        used.append(capi.alloc_stats()["bytes"] - before)
+    assert used[1] < 0.7 * used[0]                                # passes of 2^21 instead of one of all
+    had = capi.alloc_stats()["bytes"]
+    gs.render(acc.data_ptr(), w, h, 3, seed=1, maxdepth=2, stats=False)
+    torch.cuda.synchronize()
+    assert capi.alloc_stats()["bytes"] < had + (1 << 20)          # (the second staging of the segment tables)
+    gs.render(acc.data_ptr(), w, h, 4, seed=1, maxdepth=2, stats=False)
+    torch.cuda.synchronize()
+    assert capi.alloc_stats()["bytes"] > had + used[1]
