@@ -67,7 +67,7 @@ struct BounceRec {
     alignas(kCounterLine) unsigned long long work[6];
 };
 constexpr int kMaxBounces = 1024;              // maxdepth <= 1024
-constexpr int kGraphKey = 15;                    // int64 fields identifying a captured pass
+constexpr int kGraphKey = 16;                    // int64 fields identifying a captured pass
 
 
 // A pass segment: `ns` samples of pixels [p0, p0 + np) of job `job`, as paths
@@ -700,21 +700,22 @@ static int launch_shade_split(const DevScene& d, int nb, int nbc, cudaStream_t s
 // Passes of at most this many paths are shaded by one kernel: each of the four
 // launches of the class split takes 2-3 us however little it has to do.
 constexpr int64_t kOneShadePaths = 32768;
+constexpr int64_t kSmallPass = int64_t(1) << 17;   // above it no kernel is chosen by a pass's paths
 
 // The shading kernels for a tracer kind, cache mode and the scene's lights.
 // Returns the number of kernels launched (< 0: an error code).  AoTracer has no
 // BSDF: its paths are shaded by one kernel.
 template <int KIND, bool CACHE, bool AREA>
-static int launch_shade_kind(const DevScene& d, int nb, int nbc, cudaStream_t st, const ShadeArgs& A, const PathState& P,
-                             const Queues& Q) {
-    if (A.cap <= kOneShadePaths) {
+static int launch_shade_kind(const DevScene& d, int64_t paths, int nb, int nbc, cudaStream_t st, const ShadeArgs& A,
+                             const PathState& P, const Queues& Q) {
+    if (paths <= kOneShadePaths) {
         k_shade<KIND, CACHE, AREA><<<nb, kShadeThreads, 0, st>>>(d, A, P, Q);
         return 1;
     }
     const int rc = launch_shade_split<KIND, CACHE, AREA>(d, nb, nbc, st, A, P, Q);
     return rc ? rc : 4;
 }
-static int launch_shade(const DevScene& d, int kind, bool cache, int nb, int nbc, cudaStream_t st,
+static int launch_shade(const DevScene& d, int kind, bool cache, int64_t paths, int nb, int nbc, cudaStream_t st,
                         const ShadeArgs& A, const PathState& P, const Queues& Q) {
     const bool area = d.has_area != 0;
     if (kind == BG_TRACER_AO) {
@@ -722,13 +723,13 @@ static int launch_shade(const DevScene& d, int kind, bool cache, int nb, int nbc
         return 1;
     }
     if (kind == BG_TRACER_DI)
-        return area ? launch_shade_kind<BG_TRACER_DI, false, true>(d, nb, nbc, st, A, P, Q)
-                    : launch_shade_kind<BG_TRACER_DI, false, false>(d, nb, nbc, st, A, P, Q);
+        return area ? launch_shade_kind<BG_TRACER_DI, false, true>(d, paths, nb, nbc, st, A, P, Q)
+                    : launch_shade_kind<BG_TRACER_DI, false, false>(d, paths, nb, nbc, st, A, P, Q);
     if (cache)
-        return area ? launch_shade_kind<BG_TRACER_GI, true, true>(d, nb, nbc, st, A, P, Q)
-                    : launch_shade_kind<BG_TRACER_GI, true, false>(d, nb, nbc, st, A, P, Q);
-    return area ? launch_shade_kind<BG_TRACER_GI, false, true>(d, nb, nbc, st, A, P, Q)
-                : launch_shade_kind<BG_TRACER_GI, false, false>(d, nb, nbc, st, A, P, Q);
+        return area ? launch_shade_kind<BG_TRACER_GI, true, true>(d, paths, nb, nbc, st, A, P, Q)
+                    : launch_shade_kind<BG_TRACER_GI, true, false>(d, paths, nb, nbc, st, A, P, Q);
+    return area ? launch_shade_kind<BG_TRACER_GI, false, true>(d, paths, nb, nbc, st, A, P, Q)
+                : launch_shade_kind<BG_TRACER_GI, false, false>(d, paths, nb, nbc, st, A, P, Q);
 }
 
 // BSDF-sampled rays towards area lights: the closest hit must be on a bundle
@@ -992,6 +993,7 @@ struct Instr {
 struct PassCfg {
     const SegRec* segs;        // device pointer to this pass's segments
     int nseg, total, npix;
+    int64_t bound;             // paths that this and the call's other passes have at most
     int maxdepth, kind;
     bool batched;
     bg_cache* cache;           // radiance-cache mode when non-null
@@ -1059,8 +1061,8 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
     PathState P = path_state(rs);
     Queues Q;
     pass_queues(rs, 0, c.batched, Q);
-    // bounds of the queues' lengths (a captured pass serves any number of paths up to cap)
-    const int64_t most = rs->cap, most_sh = most * rs->kmax, most_mis = most * rs->nlights;
+    // bounds of the queues' lengths (a captured pass serves any number of paths up to c.bound)
+    const int64_t most = c.bound, most_sh = most * rs->kmax, most_mis = most * rs->nlights;
     int rc;
     const int depth = std::max(1, c.maxdepth);
     BG_CUDA(cudaMemsetAsync(rs->bounce.ptr, 0, size_t(depth + 1) * sizeof(BounceRec), st));
@@ -1099,7 +1101,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
                 if (ins) { ++ins->launches; ++ins->launches_extend; }
             }
             ShadeArgs A{b, c.maxdepth, c.kind, rs->kmax, c.batched ? 1 : 0, -1, -1, 0, c.ao_radius, 1, int(rs->cap)};
-            const int nsh = launch_shade(s->dev, c.kind, false, nb, rs->blocks_class, st, A, P, Q);
+            const int nsh = launch_shade(s->dev, c.kind, false, most, nb, rs->blocks_class, st, A, P, Q);
             if (nsh < 0) return nsh;
             if (ins) ins->launches += nsh - 1;
             BG_CUDA(cudaEventRecord(rs->ev_fork, st));
@@ -1148,7 +1150,7 @@ static int enqueue_pass(bg_scene* s, RenderState* rs, cudaStream_t st, const Pas
         const bool wait_here = c.cache && (c.wait_train || !ins) && b == c.cache_depth;
         if (wait_here && !fork)
             BG_CUDA(cudaStreamWaitEvent(st, rs->ev_train, ins ? 0u : unsigned(cudaEventWaitExternal)));
-        const int nsh = launch_shade(s->dev, c.kind, c.cache != nullptr, nb, rs->blocks_class, st, A, P, Q);
+        const int nsh = launch_shade(s->dev, c.kind, c.cache != nullptr, most, nb, rs->blocks_class, st, A, P, Q);
         if (nsh < 0) return nsh;
         if (ins) { ins->launches += nsh; ins->mark(1); }
         const bool forked = fork && b + 1 < depth;
@@ -1233,7 +1235,7 @@ static int pass_graph(bg_scene* s, RenderState* rs, const PassCfg& c, RenderStat
                                     c.cache ? int64_t(nrc_desc(c.cache)->mlp_kernel) + 1 : 0,
                                     c.cache ? c.cache_depth : -1, c.cache ? c.train_end : -1,
                                     c.cache ? c.train_stride : 0, c.cache ? rs->tr_set : 0,
-                                    int64_t(rs->buf_epoch)};
+                                    int64_t(rs->buf_epoch), c.bound};
     ++rs->graph_clock;
     for (auto& pg : rs->graphs)
         if (pg.exec && memcmp(key, pg.key, sizeof(key)) == 0) { pg.used = rs->graph_clock; out = &pg; return BG_OK; }
@@ -1454,6 +1456,16 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
     std::vector<int> pass_begin;
     plan_passes(jobs, cap, segs, pass_begin);
     const int npass = int(pass_begin.size()) - 1;
+    // The kernels of small passes are chosen by this call's passes, not by the largest that the
+    // state has seen: in powers of two, so that few graphs serve all sizes, up to where the
+    // choices end (a preview of 64 x 64 after a 1080p frame: 208 us by the state, 183 by the call).
+    int64_t bound = 1;
+    for (int p = 0; p < npass; ++p) {
+        int64_t paths = 0;
+        for (int q = pass_begin[size_t(p)]; q < pass_begin[size_t(p) + 1]; ++q) paths += int64_t(segs[size_t(q)].np) * segs[size_t(q)].ns;
+        while (bound < paths) bound <<= 1;
+    }
+    if (bound > kSmallPass || bound > rs->cap) bound = rs->cap;
     if ((rc = ensure_tracked(rs, rs->segs, std::max<size_t>(1, segs.size()) * sizeof(SegRec))) ||
         (rc = ensure_tracked(rs, rs->jobs, jobs.size() * sizeof(JobRec))))
         return rc;
@@ -1602,6 +1614,7 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
         c.nseg = pass_begin[size_t(p) + 1] - pass_begin[size_t(p)];
         c.total = 0;
         c.npix = 0;
+        c.bound = bound;
         for (int q = pass_begin[size_t(p)]; q < pass_begin[size_t(p) + 1]; ++q) {
             c.total += segs[size_t(q)].np * segs[size_t(q)].ns;
             c.npix += segs[size_t(q)].np;

@@ -73,3 +73,22 @@ def test_an_unchanged_render_allocates_nothing(ctx):
     gs.render(acc.data_ptr(), w, h, 4, seed=1, maxdepth=2, stats=False)
     torch.cuda.synchronize()
     assert capi.alloc_stats()["bytes"] > had + used[1]
+
+
+@pytest.mark.parametrize("size", [33, 64, 150])
+def test_a_small_render_after_a_large_one(ctx, size):
+    """The same kernels and the same image as in a scene that has rendered nothing larger."""
+    import torch
+    from banshee_b200 import capi
+    got = []
+    for large in (False, True):
+        gs = capi.GpuScene(ctx, scenes.cornell(64, 64))
+        if large:
+            gs.render(_accum(640, 480).data_ptr(), 640, 480, 4, seed=1, maxdepth=5, stats=False)
+        acc = _accum(size, size)
+        stats = gs.render(acc.data_ptr(), size, size, 1, seed=2, maxdepth=5)
+        gs.render(acc.data_ptr(), size, size, 1, seed=3, maxdepth=5, stats=False)
+        torch.cuda.synchronize()
+        got.append((stats["kernel_launches"], acc.cpu().numpy()))
+    assert got[0][0] == got[1][0]
+    assert got[0][1].max() > 0 and (got[0][1].view(np.uint32) == got[1][1].view(np.uint32)).all()
