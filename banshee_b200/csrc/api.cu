@@ -522,7 +522,9 @@ int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static
     const bool few = !counters && most > 0 && groups_walk(s, most, n_dev && !small);
     const bool flat = small && !err_out && !(n_dev && few);   // (casts: 16,384 rays of one triangle 9.2 us, 9.9 in groups)
     if (few && !flat) {
-        const int grid = int(std::min<int64_t>(s->ctx->num_sms * kCoopBlocks, (most * coop_group(most, warps) + kCoopThreads - 1) / kCoopThreads));
+        // (a render's launch may have far fewer rays than `most`, and then 32 lanes for each)
+        const int64_t lanes = std::max<int64_t>(most * 8, std::min<int64_t>(most, warps) * 32);
+        const int grid = int(std::min<int64_t>(s->ctx->num_sms * kCoopBlocks, (lanes + kCoopThreads - 1) / kCoopThreads));
         auto go = [&](auto kernel) { kernel<<<grid, kCoopThreads, 0, st>>>(s->dev, rays, int(n_static), n_dev, hits, occ, roots, res, warps, err_out); };
         const bool wt = s->dev.watertight != 0;
         if (any_hit) wt ? go(k_trace_coop<true, true>) : go(k_trace_coop<true, false>);
