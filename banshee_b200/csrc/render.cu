@@ -66,7 +66,6 @@ struct BounceRec {
     alignas(kCounterLine) int n_cls[3];
     alignas(kCounterLine) unsigned long long work[6];
 };
-constexpr int kMaxBounces = 1024;              // maxdepth <= 1024
 constexpr int kGraphKey = 16;                    // int64 fields identifying a captured pass
 
 
@@ -98,7 +97,8 @@ struct RenderState {
     DevBuf st_key, st_cnt, st_rng, st_bs, st_thr, st_rad, st_dithr, st_flags;
     DevBuf slots, sample_rad;
     DevBuf cnt_out;    // outputs of the instrumented 1/64 replays
-    DevBuf bounce;     // BounceRec[kMaxBounces + 1]: counters of the pass in flight
+    DevBuf bounce;     // BounceRec[]: counters of the pass in flight (ensure_bounces)
+    std::vector<DevBuf> retired;   // earlier ones that a stream capture holds
     // radiance-cache mode: cache queries, training-path vertex records, training samples
     DevBuf q_feat, q_path, q_thr, q_out, rec, tr_feat, tr_target;
     int64_t q_cap = 0, tr_cap = 0;       // tr_cap: rows per training set
@@ -173,6 +173,7 @@ void render_state_free(RenderState* rs) {
                       &rs->q_out, &rs->rec, &rs->tr_feat, &rs->tr_target, &rs->segs, &rs->jobs,
                       &rs->ext_root[0], &rs->ext_root[1], &rs->sh_root, &rs->mis_root, &rs->cls})
         b->release();
+    for (DevBuf& b : rs->retired) b.release();
     delete rs;
 }
 
@@ -896,7 +897,7 @@ static int state_buffers(RenderState* rs, int64_t cap, int L, bool area, bool ba
         {&R.end_path, 2 * C * 4}, {&R.cls, 3 * C * 4}, {&R.counts, 256}, {&R.st_key, C * 8}, {&R.st_cnt, C * 4},
         {&R.st_rng, C * 16}, {&R.st_bs, C * 8}, {&R.st_thr, C * 16}, {&R.st_rad, C * 16}, {&R.st_dithr, 2 * C * 16},
         {&R.st_flags, C * 4}, {&R.slots, 2 * C * 2 * L * 16}, {&R.sample_rad, C * 16},
-        {&R.cnt_out, (C * 2 * L / 64 + 64) * 16}, {&R.bounce, size_t(kMaxBounces + 1) * sizeof(BounceRec)}};
+        {&R.cnt_out, (C * 2 * L / 64 + 64) * 16}};
     size_t sum = 0;
     for (const auto& x : all) {
         sum += x.bytes;
@@ -933,6 +934,18 @@ static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L, bool ba
     BG_CUDA(cudaStreamCreateWithFlags(&rs->mstream, cudaStreamNonBlocking));
     BG_CUDA(cudaEventCreateWithFlags(&rs->ev_mjoin, cudaEventDisableTiming));
     return BG_OK;
+}
+
+// Counters for passes of `depth` bounces, in steps of 32 (66 KB; for 1,024 bounces they are
+// 2 MB, and their allocation a tenth of a new scene's first small render).
+static int ensure_bounces(RenderState* rs, int depth) {
+    const size_t need = size_t((depth + 32) / 32 * 32 + 1) * sizeof(BounceRec);
+    if (rs->bounce.ptr && rs->bounce.bytes >= need) return BG_OK;
+    if (rs->captured && rs->bounce.ptr) {
+        rs->retired.push_back(rs->bounce);
+        rs->bounce = DevBuf{};
+    }
+    return ensure_tracked(rs, rs->bounce, need);
 }
 
 // Training rows that wait for their cache's next frame, and their counts.
@@ -1466,7 +1479,8 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
         while (bound < paths) bound <<= 1;
     }
     if (bound > kSmallPass || bound > rs->cap) bound = rs->cap;
-    if ((rc = ensure_tracked(rs, rs->segs, std::max<size_t>(1, segs.size()) * sizeof(SegRec))) ||
+    if ((rc = ensure_bounces(rs, std::max(1, maxdepth))) ||
+        (rc = ensure_tracked(rs, rs->segs, std::max<size_t>(1, segs.size()) * sizeof(SegRec))) ||
         (rc = ensure_tracked(rs, rs->jobs, jobs.size() * sizeof(JobRec))))
         return rc;
     std::vector<JobRec> jrec(jobs.size());

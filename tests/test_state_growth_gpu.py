@@ -92,3 +92,23 @@ def test_a_small_render_after_a_large_one(ctx, size):
         got.append((stats["kernel_launches"], acc.cpu().numpy()))
     assert got[0][0] == got[1][0]
     assert got[0][1].max() > 0 and (got[0][1].view(np.uint32) == got[1][1].view(np.uint32)).all()
+
+
+def test_deeper_renders_after_a_shallow_one(ctx):
+    """The counters of a pass grow with its bounces: a new scene's first small render allocates
+    less than a megabyte."""
+    import torch
+    from banshee_b200 import capi
+    images = []
+    for depths in ((3, 31, 32, 33, 200, 5), (200, 3, 31, 32, 33, 5)):
+        gs = capi.GpuScene(ctx, scenes.cornell(64, 64))
+        acc = _accum(8, 8)
+        before = capi.alloc_stats()["bytes"]
+        for k, depth in enumerate(depths):
+            gs.render(acc.data_ptr(), 8, 8, 16, seed=depth, maxdepth=depth, stats=False)
+            torch.cuda.synchronize()
+            if k == 0 and depth == 3:
+                assert capi.alloc_stats()["bytes"] - before < 1024 * 1300 + (1 << 20)   # (beside the state of 1,024 paths)
+        images.append(acc.cpu().numpy())
+    assert np.allclose(images[0], images[1], rtol=1e-5, atol=0)      # the same frames, summed in another order
+    assert images[0].max() > 0 and gs.error_flags() == 0
