@@ -263,6 +263,7 @@ int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* pack
     unsigned h = 0;
     BG_CUDA(cudaMemcpy(&h, bad.ptr, sizeof(h), cudaMemcpyDeviceToHost));
     *packed = h == 0;
+    if (!*packed) out.release();         // nothing reads them
     return BG_OK;
 }
 

@@ -112,3 +112,23 @@ def test_deeper_renders_after_a_shallow_one(ctx):
         images.append(acc.cpu().numpy())
     assert np.allclose(images[0], images[1], rtol=1e-5, atol=0)      # the same frames, summed in another order
     assert images[0].max() > 0 and gs.error_flags() == 0
+
+
+def test_nodes_that_cannot_be_packed_hold_no_memory(ctx):
+    """A triangle beyond the packed range leaves the scene to the plain walk; its packed nodes go."""
+    import torch
+    from banshee_b200 import capi
+    held = []
+    capi.GpuScene(ctx, scenes.soup(1 << 20, seed=5), builder=3, node_width=4).close()   # the build's scratch stays
+    for far in (False, True):
+        sc = scenes.soup(1 << 20, seed=5)
+        if far:
+            sc.meshes[0].vertices.reshape(-1, 3, 3)[0] = np.float32(4e15)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        gs = capi.GpuScene(ctx, sc, builder=3, node_width=4)
+        torch.cuda.synchronize()
+        held.append(free - torch.cuda.mem_get_info()[0])
+        packed = gs.info()["nnodes"] * 64
+        gs.close()
+    assert held[1] < held[0] - 0.8 * packed, (held, packed)
