@@ -386,12 +386,12 @@ constexpr int64_t kPackTriangles = 1000, kPackTriangles8 = 64;
 template <int WIDTH>
 static int choose_walk(const bg_scene* s, bool render, int64_t most) {
     const DevScene& d = s->dev;
+    if (WIDTH == 4 && render) return fused_walk(d) ? kWalkFused : kWalkPlain;
     if (!packed_walk<WIDTH>(d)) return kWalkPlain;
     if (WIDTH == 8) {
         const int64_t lanes = int64_t(s->trace_blocks[kWalkPacked][1][0][0][0]) * 128;
         return d.ntris < kPackTriangles8 || most * 3 < lanes * 2 ? kWalkPlain : kWalkPacked;
     }
-    if (render) return kWalkFused;
     return d.ntris < kPackTriangles ? kWalkPlain : kWalkPacked;
 }
 
@@ -518,7 +518,7 @@ int launch_trace(bg_scene* s, bool any_hit, const float4* rays, int64_t n_static
     // at most `n_most` rays, few enough for groups of lanes
     const int64_t most = n_dev ? n_most : n_static;
     const int warps = s->ctx->num_sms * kCoopBlocks * (kCoopThreads / 32);
-    const bool small = !counters && !roots && s->dev.width == 4 && packed_walk<4>(s->dev) && s->nnodes4 <= (n_dev ? kFlatNodes : kFlatNodesCast);
+    const bool small = !counters && !roots && s->dev.width == 4 && fused_walk(s->dev) && s->nnodes4 <= (n_dev ? kFlatNodes : kFlatNodesCast);
     const bool few = !counters && most > 0 && groups_walk(s, most, n_dev && !small);
     const bool flat = small && !err_out && !(n_dev && few);   // (casts: 16,384 rays of one triangle 9.2 us, 9.9 in groups)
     if (few && !flat) {
@@ -743,8 +743,8 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
         (rc = s->err.ensure(sizeof(unsigned))) ||
         (rc = s->work.ensure(kWorkSlots * sizeof(unsigned long long))))
         return rc;
-    bool packed = false;
-    if (nn4 && (rc = device_pack_nodes(s->nodes.as<WideNode4>(), nn4, s->qnodes, &packed))) return rc;
+    bool ranged = false;
+    if (nn4 && (rc = device_pack_nodes(s->nodes.as<WideNode4>(), nn4, s->qnodes, &ranged))) return rc;
     BG_CUDA(cudaMemcpy(s->mats_d.ptr, mats.data(), mats.size() * sizeof(MatRec), cudaMemcpyHostToDevice));
     if (!lights.empty())
         BG_CUDA(cudaMemcpy(s->lights_d.ptr, lights.data(), lights.size() * sizeof(LightRec), cudaMemcpyHostToDevice));
@@ -752,7 +752,8 @@ static int commit_scene(bg_scene* s, const bg_build_opts* opts) {
     BG_CUDA(cudaMemset(s->work.ptr, 0, kWorkSlots * sizeof(unsigned long long)));
     DevScene& d = s->dev;
     d.nodes = nn4 ? s->nodes.as<WideNode4>() : nullptr;
-    d.qnodes = packed ? s->qnodes.as<QNode4>() : nullptr;
+    d.qnodes = s->qnodes.as<QNode4>();
+    d.ranged = ranged ? 1 : 0;
     d.nodes8 = nn8 ? s->nodes8.as<QNode8>() : nullptr;
     s->nnodes4 = nn4;
     s->nnodes8 = nn8;

@@ -190,9 +190,10 @@ int bg_batch_commit(bg_batch* b) {
     BG_CUDA(cudaDeviceSynchronize());
     DevScene& d = M.dev;
     d.nodes = all4 ? M.nodes.as<WideNode4>() : nullptr;
-    bool packed = false;
-    if (all4 && (rc = device_pack_nodes(M.nodes.as<WideNode4>(), nn, M.qnodes, &packed))) return rc;
-    d.qnodes = packed ? M.qnodes.as<QNode4>() : nullptr;
+    bool ranged = false;
+    if (all4 && (rc = device_pack_nodes(M.nodes.as<WideNode4>(), nn, M.qnodes, &ranged))) return rc;
+    d.qnodes = M.qnodes.as<QNode4>();
+    d.ranged = ranged ? 1 : 0;
     d.nodes8 = all8 ? M.nodes8.as<QNode8>() : nullptr;
     d.width = all4 ? (all8 ? kDefaultNodeWidth : 4) : 8;
     M.nnodes4 = nn; M.nnodes8 = nn8;

@@ -168,10 +168,10 @@ int device_world_boxes(MeshArrays& A, const BundleRec* bundles, int64_t ntris, f
 // mat_class: class per material index (0 other, 1 Lambert, 2 GGX), stored in TriRec e2.w
 int device_records(const MeshArrays& A, const BundleRec* bundles, const int32_t* order, int64_t ntris,
                    TriRec* tris, ShadeRec* shade, bool vertices, const int32_t* mat_class, int nmat);
-// nodes packed for traversal (QNode4) into `out`; *packed = false when some
-// node's planes are outside the packed range or there is no memory for them (the
+// nodes packed for traversal (QNode4) into `out`, left empty when some node's planes
+// are outside the packed range (*ranged = false) or there is no memory for them (the
 // traversal then walks `nodes`)
-int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* packed);
+int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* ranged);
 constexpr int kWorkSlots = 256;
 unsigned long long* next_work_counter(bg_scene* s);
 void scene_launch_setup(bg_scene* s);

@@ -203,7 +203,7 @@ int device_world_boxes(MeshArrays& A, const BundleRec* bundles, int64_t ntris, f
     return BG_OK;
 }
 
-// WideNode4 -> QNode4, in double precision: the step of an axis is 1/250 of the
+// WideNode4 -> QNode4 (out null: only whether they fit), in double precision: the step of an axis is 1/250 of the
 // children's extent, but at least 2^-22 of the largest coordinate, so that the
 // float rounding of the grid origin stays below half a step.
 __global__ void k_pack_nodes(const WideNode4* __restrict__ nodes, int64_t n, QNode4* __restrict__ out,
@@ -244,26 +244,28 @@ __global__ void k_pack_nodes(const WideNode4* __restrict__ nodes, int64_t n, QNo
         q.ox = org[0]; q.oy = org[1]; q.oz = org[2];
         q.sx = step[0]; q.sy = step[1]; q.sz = step[2];
         q.lox = lo[0]; q.hix = hi[0]; q.loy = lo[1]; q.hiy = hi[1]; q.loz = lo[2]; q.hiz = hi[2];
-        out[i] = q;
+        if (out) out[i] = q;
         if (!ok) atomicOr(bad, 1u);
     }
 }
 
-int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* packed) {
-    *packed = false;
+int device_pack_nodes(const WideNode4* nodes, int64_t n, DevBuf& out, bool* ranged) {
+    *ranged = false;
     ScratchBuf bad;
-    int rc;
-    if ((rc = out.ensure(size_t(n) * sizeof(QNode4))) || (rc = bad.ensure(sizeof(unsigned)))) {
+    int rc = bad.ensure(sizeof(unsigned));
+    if (rc) return rc == BG_ERR_OOM ? BG_OK : rc;   // no room: the plain walk needs none
+    rc = out.ensure(size_t(n) * sizeof(QNode4));
+    if (rc) {
         out.release();
-        return rc == BG_ERR_OOM ? BG_OK : rc;   // no room: the plain walk needs none
+        if (rc != BG_ERR_OOM) return rc;
     }
     BG_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned), 0));
     k_pack_nodes<<<grid_for(n), kRT>>>(nodes, n, out.as<QNode4>(), bad.as<unsigned>());
     BG_CUDA(cudaGetLastError());
     unsigned h = 0;
     BG_CUDA(cudaMemcpy(&h, bad.ptr, sizeof(h), cudaMemcpyDeviceToHost));
-    *packed = h == 0;
-    if (!*packed) out.release();         // nothing reads them
+    *ranged = h == 0;
+    if (!*ranged) out.release();         // nothing reads them
     return BG_OK;
 }
 

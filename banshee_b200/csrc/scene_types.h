@@ -77,7 +77,7 @@ constexpr int kClassShift = 28;
 
 struct DevScene {
     const WideNode4* nodes;
-    const QNode4* qnodes;   // nodes packed for traversal (null: planes out of the packed range)
+    const QNode4* qnodes;   // nodes packed for traversal (null: planes out of the packed range, or no room)
     const QNode8* nodes8;
     const TriRec* tris;
     const ShadeRec* shade;
@@ -92,6 +92,7 @@ struct DevScene {
     int32_t has_area;       // some light is an AreaLight (selects the shading variant)
     int32_t watertight;     // tris hold (p1, p2, p3) for the watertight test, not (p1, e1, e2)
     float extent;           // largest |coordinate| of the world bounds
+    int32_t ranged;         // all planes of `nodes` are in the packed range
 };
 
 }  // namespace bg

@@ -124,11 +124,13 @@ struct TraceScene : DevScene {
     int ownstep;
 };
 
-// Whether the packed arithmetic covers the scene.
+// Whether the packed arithmetic covers the scene, on its packed or 8-wide nodes and on
+// the 128-byte ones (which need no room for packed nodes).
 template <int WIDTH>
 __host__ __device__ __forceinline__ bool packed_walk(const DevScene& S) {
     return S.extent <= 1e15f && (WIDTH == 8 || S.qnodes != nullptr);
 }
+__host__ __device__ __forceinline__ bool fused_walk(const DevScene& S) { return S.extent <= 1e15f && S.ranged; }
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;

@@ -240,3 +240,23 @@ def test_renders_on_every_walk(ctx, name, width):
             torch.cuda.synchronize()
             assert want[..., :3].max() > 0
             assert (got.view(torch.int32) == want.view(torch.int32)).all(), (w, tracer)
+
+
+@pytest.mark.parametrize("name", ["cornell", "production"])
+def test_renders_without_room_for_the_packed_nodes(ctx, name):
+    """The fused and the boxes-first walk need none: the same image, in about the same time."""
+    import torch
+    full, tight = _plain_twin(ctx, RENDERS[name](), {})
+    acc = [torch.zeros((512, 640, 4), device="cuda") for _ in range(2)]
+    times = [[], []]
+    for k in range(12):
+        for i, gs in enumerate((full, tight)):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            gs.render(acc[i].data_ptr(), 640, 512, 8, seed=k, maxdepth=5, stats=False)
+            b.record()
+            torch.cuda.synchronize()
+            times[i].append(a.elapsed_time(b))
+    assert (acc[0].view(torch.int32) == acc[1].view(torch.int32)).all()
+    fast, slow = (min(t) for t in times)
+    assert slow < 1.03 * fast, (fast, slow)
