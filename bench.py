@@ -151,11 +151,15 @@ def run_reference_arm(args, rank):
     if rank != 0:
         return 0
     from banshee_b200 import scenes
-    from oracle.oracle import Reference
+    from oracle import oracle
+    if not oracle.available("ref"):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU tracer is not built here "
+                          "(oracle/_ref/libbanshee_ref.so is made from the reference tree)"}), flush=True)
+        return 0
     sc = scenes.production(WIDTH, HEIGHT)
     ncores = os.cpu_count() or 1
     rows = max(1, min(64, args.ref_rows))
-    ref = Reference(sc)
+    ref = oracle.Reference(sc)
     acc = np.zeros((HEIGHT, WIDTH, 4), dtype=np.float32)
 
     def step(i):

@@ -26,3 +26,16 @@ def test_reference_arm_json_line():
     assert d["cpu_baseline"]["kind"] == "reference" and d["cpu_baseline"]["cores"] >= 1
     assert d["e2e"] == {"value": d["value"], "unit": "Msamples/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}
     assert d["config"]["workload"].startswith("C3")
+
+
+def test_reference_arm_without_the_reference(monkeypatch, capsys):
+    """Where the reference is not built the arm says so in one line and exits with 0."""
+    import argparse
+    import bench
+    from oracle import oracle
+    monkeypatch.setattr(oracle, "REF_SO", os.path.join(ROOT, "oracle", "no_such_library.so"))
+    rc = bench.run_reference_arm(argparse.Namespace(gpus=1, steps=2, warmup=3, ref_rows=2), 0)
+    lines = capsys.readouterr().out.splitlines()
+    assert rc == 0 and len(lines) == 1
+    d = json.loads(lines[0])
+    assert d["impl"] == "reference" and d["unavailable"] and set(d) == {"impl", "unavailable"}
