@@ -278,8 +278,11 @@ k_trace_coop(DevScene scene, const float4* __restrict__ rays, int n_static, cons
 // each turn costs both: 10 of 32 lanes are active in a Cornell box's secondary rays.
 // The boxes are the fused walk's, so at least the leaves of the plain walk are tested;
 // ties and rays outside the fused arithmetic go to the plain walk.
-//   renders  16 nodes (a bit per child): a Cornell box, where a ray enters most of the
-//            few boxes, 5.06 -> 4.78 ms (64 samples, 256 x 256)
+//   renders  16 nodes (a bit per child).  256 x 256, 16 samples, GiTracer, tree walk -> boxes
+//            first, us: closed box of 9 / 10 / 15 / 16 nodes 1381 -> 1298 / 1476 -> 1378 /
+//            1479 -> 1424 / 1497 -> 1468, boxes in the open of 1 / 6 / 9 / 15 nodes 211 -> 163 /
+//            324 -> 297 / 360 -> 328 / 358 -> 345; AoTracer between 137 -> 116 (1 node) and 289
+//            -> 295 (16)
 //   casts    4 nodes (closest / any hits in Grays/s, tree walk -> boxes first, rays from
 //            all over a soup: 1 node 38 / 40 -> 86 / 95, 3 nodes 38 / 40 -> 64 / 65, 4
 //            38 / 40 -> 48 / 48, 6 38 / 40 -> 37 / 38; Cornell box, 9 nodes, 9.2 / 13.6 ->
@@ -1089,7 +1092,11 @@ struct CastStage {
     ~CastStage() { release(); }
 };
 constexpr int kStages = 4;
-constexpr int64_t kHostInPlace = 1024;   // rays of a call that the kernel reads from and answers into pinned host memory
+// Rays of a call that the kernel reads from and answers into pinned host memory, with one
+// launch and no copies: closest hits of 1 / 64 / 1,024 rays into 20,000 triangles 22 / 28 / 32
+// us, staged 38 / 38 / 40.  (In place was the faster one up to 65,536 rays too, 306 against 385
+// us; the line keeps a long read of host memory out of a kernel that others may wait for.)
+constexpr int64_t kHostInPlace = 1024;
 thread_local CastStage t_stage[kStages];
 thread_local uint64_t t_stage_clock = 0;
 }  // namespace
@@ -1200,7 +1207,7 @@ int bg_traversal_counts(bg_scene* s, const bg_ray* rays, int64_t n, int32_t any_
         rc = launch_trace(s, any_hit != 0, reinterpret_cast<const float4*>(rays), n, nullptr, hits, occ, st, cnt, 1);
         if (rc) { tmp.release(); return rc; }
     }
-    unsigned long long h[3] = {0, 0};
+    unsigned long long h[3] = {0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     tmp.release();
@@ -1290,7 +1297,7 @@ extern "C" int bg_traversal_counts_noalloc(bg_scene* s, const bg_ray* rays, int6
                       work, nullptr, ShadowResolve{nullptr, nullptr, nullptr, 0});
         e = cudaGetLastError();
     }
-    unsigned long long h[3] = {0, 0};
+    unsigned long long h[3] = {0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return set_error(BG_ERR_CUDA, "bg_traversal_counts_noalloc: %s", cudaGetErrorString(e));

@@ -472,13 +472,11 @@ static int64_t grid_params(const bg_cache* c) { return int64_t(kNrcLevels) * (in
 
 static std::atomic<uint64_t> g_cache_ids{1};
 
-// Scratch for up to `train_rows` rows of one Adam step (encoded rows, hidden
-// activations and layer gradients of the fused training kernels) and for
-// `query_rows` queries at a time.  The tcgen05 inference kernel encodes its
-// queries in shared memory and needs none; the mma.sync path encodes them
-// into X first.  (Sizing everything by the pass, 2^24 paths, took 28.6 GB.)
-// Scratch: encoded rows, and for the mma.sync kernels a training set's activations and
-// gradients (the tcgen05 one keeps those of a tile on the chip).
+// Scratch for up to `train_rows` rows of one Adam step and `query_rows` queries at a time:
+// encoded rows, and for the mma.sync kernels a training set's activations and gradients (the
+// tcgen05 one keeps those of a tile on the chip).  The tcgen05 inference kernel encodes its
+// queries in shared memory and needs none; the mma.sync path encodes them into X first.
+// (Sizing everything by the pass, 2^24 paths, took 28.6 GB.)
 static int cache_scratch(bg_cache* c, int64_t train_rows, int64_t query_rows) {
     const int64_t xr = std::max(train_rows, c->desc.mlp_kernel == 0 ? int64_t(0) : query_rows);
     if (train_rows <= c->train_cap && xr <= c->x_cap) return BG_OK;

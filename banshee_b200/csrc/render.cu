@@ -699,7 +699,11 @@ static int launch_shade_split(const DevScene& d, int nb, int nbc, cudaStream_t s
 }
 
 // Passes of at most this many paths are shaded by one kernel: each of the four
-// launches of the class split takes 2-3 us however little it has to do.
+// launches of the class split takes 2-3 us however little it has to do.  A frame of
+// 4,096 / 32,400 / 65,536 / 262,144 / 524,176 paths, split and in one, us: Cornell box 210 and
+// 176 / 259 and 222 / 331 and 295 / 425 and 420 / 699 and 771, production scene 253 and 191 /
+// 310 and 255 / 357 and 304 / 524 and 465 / 679 and 646.  The line lies well below the
+// crossing: a pass's bound is a power of two, and the split keeps gaining with its paths.
 constexpr int64_t kOneShadePaths = 32768;
 constexpr int64_t kSmallPass = int64_t(1) << 17;   // above it no kernel is chosen by a pass's paths
 
@@ -938,14 +942,18 @@ static int alloc_state(bg_scene* s, RenderState* rs, int64_t cap, int L, bool ba
 
 // Counters for passes of `depth` bounces, in steps of 32 (66 KB; for 1,024 bounces they are
 // 2 MB, and their allocation a tenth of a new scene's first small render).
-static int ensure_bounces(RenderState* rs, int depth) {
+static int ensure_bounces(RenderState* rs, int depth, bool capturing) {
     const size_t need = size_t((depth + 32) / 32 * 32 + 1) * sizeof(BounceRec);
     if (rs->bounce.ptr && rs->bounce.bytes >= need) return BG_OK;
-    if (rs->captured && rs->bounce.ptr) {
+    if ((rs->captured || capturing) && rs->bounce.ptr) {
         rs->retired.push_back(rs->bounce);
         rs->bounce = DevBuf{};
     }
-    return ensure_tracked(rs, rs->bounce, need);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (an allocation ends a capture in the other modes)
+    if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+    const int rc = ensure_tracked(rs, rs->bounce, need);
+    if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+    return rc;
 }
 
 // Training rows that wait for their cache's next frame, and their counts.
@@ -1479,7 +1487,7 @@ int render_jobs(bg_scene* s, bg_cache* cache, const std::vector<JobSpec>& jobs, 
         while (bound < paths) bound <<= 1;
     }
     if (bound > kSmallPass || bound > rs->cap) bound = rs->cap;
-    if ((rc = ensure_bounces(rs, std::max(1, maxdepth))) ||
+    if ((rc = ensure_bounces(rs, std::max(1, maxdepth), cap_st != cudaStreamCaptureStatusNone)) ||
         (rc = ensure_tracked(rs, rs->segs, std::max<size_t>(1, segs.size()) * sizeof(SegRec))) ||
         (rc = ensure_tracked(rs, rs->jobs, jobs.size() * sizeof(JobRec))))
         return rc;

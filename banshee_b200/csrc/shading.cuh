@@ -414,7 +414,7 @@ __device__ __forceinline__ v3 light_getsample(const DevScene& S, const LightRec&
 }
 template <bool AREA, bool INL = false>
 __device__ __forceinline__ float light_getpdf(const DevScene& S, const LightRec& L, const SHit& h, v3 w) {
-    if (AREA && L.type == BG_LIGHT_AREA) 
+    if (AREA && L.type == BG_LIGHT_AREA)
         return INL ? area_getpdf_body(S, L.prim, L.mesh, L.area_world, h.p, w)
                    : area_getpdf(S, L.prim, L.mesh, L.area_world, h.p, w);
     if (L.type == BG_LIGHT_DIRECTIONAL) return 0.f;

@@ -653,7 +653,6 @@ __device__ __forceinline__ void trav_init(TS& s, const TraceScene& S, uint32_t w
     if ((s.r.flags & kPlainWalk) && (isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(b.x) || isnan(b.y) || isnan(b.z))) s.item = kNone;
 }
 
-// Runs at most `steps` node / leaf visits.  Returns true when the ray is done.
 // Pops the next stack entry, skipping entries that start beyond the closest
 // hit; false when the stack is empty.
 template <bool ANY, class STACK, bool WT, int WALK>

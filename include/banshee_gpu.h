@@ -169,7 +169,7 @@ typedef struct bg_build_opts {
 typedef struct bg_scene_info {
     int64_t ntriangles;
     int64_t nnodes;
-    int64_t node_bytes;     /* device bytes of the node array            */
+    int64_t node_bytes;     /* device bytes of the node array (4-wide trees that casts read packed hold 64 bytes per node besides) */
     int64_t tri_bytes;      /* device bytes of the traversal triangles   */
     int64_t shade_bytes;    /* device bytes of the shading records       */
     int32_t node_stride;    /* bytes per node                             */
