@@ -313,41 +313,40 @@ __device__ __forceinline__ bool wt_test(const ObjRayWT& c, v3 p1, v3 p2, v3 p3, 
 // distance over edge length and with incidence, and takes the true hit out of the box.)
 // Moller-Trumbore's record holds p2 - p1, rounded, not p2.  A little less of it, added to p1,
 // comes out between p1 and p2, as the rounding of a sum is monotone and p2 a float.
-// Once per ray, at its end: casts are 0-4 % slower with it (1M-triangle soup, closest /
-// any incoherent 1400 / 1797 -> 1409 / 1800 Mrays/s, any coherent 3845 -> 3680), a 6M-triangle
-// frame 29.0 -> 29.8 ms.  Also measured: bounds of the test's rounding instead, at every hit
-// casts 4-12 % slower, at the ray's end (the plain walk for what they leave open) C3 44.6 ms;
-// a call out of line C3 31.6 ms.
+// Once per ray, at its end (1M-triangle soup, closest / any incoherent 1400 / 1797 Mrays/s
+// without it, 1440 / 1820 with it, any coherent 3845 and 3700; a 6M-triangle frame 29.0 and
+// 29.4 ms, 29.8 with the record read by words).  Also measured: bounds of the test's rounding
+// instead, at every hit casts 4-12 % slower, at the ray's end (the plain walk for what they
+// leave open) the frame 44.6 ms; a call out of line 31.6 ms.
 template <bool WT>
 __device__ __forceinline__ bool plain_reaches(const DevScene& S, int tri, int prim, float t, const float* o, v3 inv, float tmin) {
-    const float* f = reinterpret_cast<const float*>(S.tris + tri);
-    const int bundle = __float_as_int(__ldg(f + 3));
+    const float4* f = reinterpret_cast<const float4*>(S.tris + tri);
+    float4 a = __ldg(f), b = __ldg(f + 1), c = __ldg(f + 2);
+    const int bundle = __float_as_int(a.w);
+    if (bundle >= 0) {                       // the corners themselves
+        f = reinterpret_cast<const float4*>(S.shade + (prim & kPrimMask));
+        a = __ldg(f); b = __ldg(f + 1); c = __ldg(f + 2);
+        const float4* m = reinterpret_cast<const float4*>(S.bundles[bundle].m);
+        auto row = [&](float4 r, float4 v) { return r.x * v.x + r.y * v.y + r.z * v.z + r.w; };
+        const float4 m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2);
+        a = make_float4(row(m0, a), row(m1, a), row(m2, a), 0.f);
+        b = make_float4(row(m0, b), row(m1, b), row(m2, b), 0.f);
+        c = make_float4(row(m0, c), row(m1, c), row(m2, c), 0.f);
+    } else if (!WT) {
+        const float k = 1.f - 0x1p-20f;
+        b = make_float4(fmaf(b.x, k, a.x), fmaf(b.y, k, a.y), fmaf(b.z, k, a.z), 0.f);
+        c = make_float4(fmaf(c.x, k, a.x), fmaf(c.y, k, a.y), fmaf(c.z, k, a.z), 0.f);
+    }
     float t0 = tmin, t1 = t;
-    auto axis = [&](int k, float i) {
-        float x, y, z;
-        if (bundle >= 0) {
-            const float* m = S.bundles[bundle].m + 4 * k;
-            const float* c = reinterpret_cast<const float*>(S.shade + (prim & kPrimMask));   // the corners themselves
-            x = __ldg(m) * __ldg(c) + __ldg(m + 1) * __ldg(c + 1) + __ldg(m + 2) * __ldg(c + 2) + __ldg(m + 3);
-            y = __ldg(m) * __ldg(c + 4) + __ldg(m + 1) * __ldg(c + 5) + __ldg(m + 2) * __ldg(c + 6) + __ldg(m + 3);
-            z = __ldg(m) * __ldg(c + 8) + __ldg(m + 1) * __ldg(c + 9) + __ldg(m + 2) * __ldg(c + 10) + __ldg(m + 3);
-        } else {
-            x = __ldg(f + k);
-            y = __ldg(f + 4 + k);
-            z = __ldg(f + 8 + k);
-            if (!WT) {
-                y = fmaf(y, 1.f - 0x1p-20f, x);
-                z = fmaf(z, 1.f - 0x1p-20f, x);
-            }
-        }
+    auto axis = [&](float x, float y, float z, float from, float i) {
         if (fabsf(i) == kZeroInv) i = copysignf(__int_as_float(0x7f800000), i);   // the plain walk's 1 / 0
-        const float s0 = (min3(x, y, z) - o[k]) * i, s1 = (max3(x, y, z) - o[k]) * i;
+        const float s0 = (min3(x, y, z) - from) * i, s1 = (max3(x, y, z) - from) * i;
         t0 = fmaxf(t0, fminf(s0, s1));
         t1 = fminf(t1, fmaxf(s0, s1));
     };
-    axis(0, inv.x);
-    axis(1, inv.y);
-    axis(2, inv.z);
+    axis(a.x, b.x, c.x, o[0], inv.x);
+    axis(a.y, b.y, c.y, o[1], inv.y);
+    axis(a.z, b.z, c.z, o[2], inv.z);
     return t0 <= fmaf(fabsf(t1), kBoxSlack, t1);
 }
 
