@@ -206,6 +206,9 @@ def raycast_c2(ctx, nrays=1 << 24, reps=5):
     out["coherent_any_note"] = ("degenerate by construction: rays start 1.5 units in front of the cube and end "
                                 "within 1 unit, so every ray is culled at the root (1 node, 0 triangles); "
                                 "coherent_shadow_any uses tmax U[1.5,2.5], ending inside the soup")
+    out["bytes_note"] = ("nodes, triangles and bytes per ray are the plain walk's (128- or 96-byte nodes), whose order "
+                         "defines the hits; 4-wide casts read 64-byte packed nodes, or the 128-byte ones in warps of "
+                         "one octant")
     for width, (kind, anyhit, trange) in [(w, st) for w in (4, 8) for st in sets]:
         gs.set_node_width(width)
         info = gs.info()

@@ -410,7 +410,9 @@ int bg_batch_destroy(bg_batch* batch);
  * with 2 lights 1.2 KB per path where the scene has area lights, else 0.8 KB
  * (20 or 14 GB at 2^24 paths).  Without it, passes have up to 2^23 paths where
  * the device's free memory and the allocation cap hold eight times what those
- * need, else 2^22 or 2^21; cached renders' passes 2^21.  No counterpart
+ * need, else 2^22 or 2^21, decided by the largest call so far (a smaller or
+ * an unchanged one never replaces the state); cached renders' passes 2^21, and
+ * rows that wait to be trained outlive the state.  No counterpart
  * in the reference.  Synchronises. */
 int bg_scene_autotune(bg_scene* scene, const bg_camera_desc* camera, const bg_tracer_desc* tracer,
                       int32_t probe_spp, int32_t width, int32_t height, float* accum_rgbw_dev,
